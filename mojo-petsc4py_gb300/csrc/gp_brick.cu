@@ -1,101 +1,144 @@
-// Brick form of the triangular sweeps (ILU, IC and SOR applies,
-// src/ported.mojo:633-748, 864-952) for sweeps whose dependencies are the
-// unit steps of a Cartesian grid in natural order -- the 5- and 7-point
-// stencils, upwind convection-diffusion, any operator with that pattern.
+// Brick form of the triangular sweeps (ILU, IC and SOR applies and the
+// transposed ILU apply, src/ported.mojo:633-748, 864-952) for sweeps whose
+// dependencies are the unit steps of a Cartesian grid in natural order -- the
+// 5- and 7-point stencils, upwind convection-diffusion, any operator with
+// that pattern.
 //
 // On such a grid (nx, ny, nz) a forward sweep's row r = i + nx (j + ny k)
 // depends on r - 1 (i - 1), r - nx (j - 1) and r - nx ny (k - 1), each present
 // exactly when that coordinate is >= 1; a backward sweep on r + 1, r + nx,
 // r + nx ny (mirrored coordinates make both "coordinate minus one").  The
-// dependency chain is nx + ny + nz - 2 levels long whatever the schedule, so
-// what decides the speed is the cost of a level.  On GB300 a hand-off between
-// two SMs through L2 takes ~0.45 us (store, poll and return) while a
-// dependent FP64 operation takes 64 cycles, so a level whose inputs are on
-// the SM costs a fraction of one that waits on another SM:
+// dependency chain is nx + ny + nz - 2 rows long whatever the schedule, so
+// what decides the speed is the cost of one link of it.  On GB300 a hand-off
+// between two SMs through L2 costs ~0.5 us (store, poll and return) and a
+// dependent FP64 operation 64 cycles (31 ns), during which it also holds its
+// sub-partition's FP64 unit.  So the links stay in registers where they can:
 //
-//   * a brick is BJ consecutive lines along i of one plane k (all of i).
-//     One CTA takes a brick and each compute thread walks one line, line t
-//     reaching row i at step s = i + t: the i - 1 value is the thread's own
-//     previous one, the j - 1 value the previous step's value of thread t - 1
-//     (shared memory, double buffered by step parity, one barrier of the
-//     compute warps a step);
-//   * rows are stored by position, step-major within a brick: position
-//     base + s BJ + t (positions with no row are holes), so a warp's loads of
-//     coefficients and diagonals and its stores of values are contiguous;
-//   * the k - 1 values (the same step and line of the brick one plane below)
-//     and the j - 1 values of line 0 (the brick below in j) come from other
-//     CTAs.  Fetch warps poll them in global memory (the value-as-flag array;
-//     a signalling NaN marks "not yet") -- a warp 32 lines at a time, one
-//     coalesced load a step, several steps in flight -- and drop each step's
-//     values into a shared-memory ring slot once all of them are in.  A
-//     compute thread takes its value from the slot (normally already there)
-//     and frees it; a fetch warp fills a slot only once it is free, so it runs
-//     at most a ring's length ahead.  The compute warps never wait on a global
-//     poll, and a brick that runs a hand-off behind its neighbour pays only
-//     the on-SM chain per step;
-//   * each row's coefficients, right-hand side and diagonal are loaded
-//     kBrickAhead steps before use into a register ring indexed by the step
-//     (uniform across the CTA, so the ring stays in registers);
-//   * bricks are handed out by a ticket in wavefront order (J + K); a brick
-//     depends only on the bricks at J - 1 and K - 1, which CTAs that are
+//   * a warp takes a tile of grid lines (8 x 4 in 3-D, 32 in 2-D) and walks
+//     them together, lane (tp, tq) reaching row w of its line at step
+//     w + tp + tq: the value one row back is the lane's own last one, the ones
+//     a line back the last ones of lanes (tp - 1, tq) and (tp, tq - 1), a
+//     shuffle away.  No barrier and no memory is on that chain;
+//   * the lines run along the direction whose term a row's fold takes first --
+//     k forward (ascending columns k, j, i), i backward -- so the fold starts
+//     from the lane's own value and the shuffles (51 cycles from one FP64
+//     result to the next operation) pass behind its first operation;
+//   * a CTA takes a brick of up to four such tiles, one warp (and one
+//     sub-partition's FP64 unit) each.  A value on the face of a tile goes to
+//     the neighbouring tile through a shared-memory ring, value-as-flag (a
+//     signalling NaN marks "not yet"), indexed by the step;
+//   * a value on the face of a brick goes out to global memory, and the fetch
+//     warps of the neighbouring CTA poll it there, eight lanes a face line, a
+//     row each, and drop each into the reader's ring the moment it is in.  A brick that runs a hand-off behind its neighbour never waits on
+//     memory; on 128^3 the chain crosses 22 brick faces instead of 381 levels;
+//   * the faces have two copies, used in turn: a sweep reads and writes one
+//     and marks the other "not yet" for the next sweep, so nothing is cleared
+//     in between and the values of the rows themselves need no flags;
+//   * coefficients and diagonals are stored by step, [tile][step][column]
+//     [lane], so a group of kGroup steps is one contiguous piece, brought into
+//     shared memory by cp.async.bulk two groups ahead; starting values come
+//     by cp.async.  Loads into registers would not stay in flight over that
+//     many steps: a warp has six scoreboards, and a wait on one is a wait for
+//     every load that was put on it (a register ring measured 0.4 us a step);
+//   * bricks are handed out by a ticket in wavefront order (P + Q); a brick
+//     depends only on the bricks at P - 1 and Q - 1, which CTAs that are
 //     already running hold, so the sweep cannot deadlock whatever the number
-//     of resident CTAs.  Within a CTA the fetch warps wait only on other
-//     bricks and on slots the compute threads free in step order, and every
-//     wait has an iteration budget.
+//     of resident CTAs.  Within a CTA a warp waits on lower steps only (for a
+//     value, or for a reader a whole ring behind), and every wait has a budget.
+//
+// What it measures (one sweep, GB300): 163-168 us on 128^3 (382 rows of chain;
+// 370 forward and 466 backward in the level-ordered form), 98 us on 256^2 (511
+// rows; 250 in the chunked form).  A step of a tile costs 0.15 us in 3-D forward
+// (three dependent FP64 operations are 0.093) and 0.2 with faces to read and
+// write; a brick face 1.3 us alone and up to 3 us with 128 CTAs at work, where
+// the latest of its 24 lines decides.
 //
 // Every row is the reference's fold of its terms in ascending-column order,
 // with the same operations as k_ell_sweep: results are bit-identical to the
 // reference's sequential sweeps and to the other forms.
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gp_pc.h"
 
 namespace gp {
 
-constexpr int kBrickMaxLines = 128;                  // compute threads (lines) per CTA
-constexpr int kBrickMaxFace = kBrickMaxLines + 1;    // ring columns: BJ k-face lines, the j face
-constexpr int kBrickKWarps = kBrickMaxLines / 32;    // fetch warps of the k face
-constexpr int kBrickThreads = kBrickMaxLines + 32 * (kBrickKWarps + 1);
-constexpr int kBrickAhead = 4;       // steps between a row's loads and its use
-constexpr int kBrickIdxAhead = 8;    // steps between a row's input index load and its use
-constexpr int kBrickRing = 9;        // register ring slots (kBrickIdxAhead + 1)
-constexpr int kBrickSlots = 16;      // shared-memory ring slots per column (power of 2)
-constexpr int kBrickPoll = 4;        // steps a fetch warp keeps in flight
+constexpr int kBrickMaxLines = 128;  // forced lines of a brick
+constexpr int kBrickWarps = 4;       // tiles (compute warps) of a brick
+constexpr int kBrickRing = 32;       // steps a tile's ring holds (a power of two)
+constexpr int kGroup = 16;           // steps staged together
+constexpr int kHalf = 8;             // steps between two looks at the neighbours' progress
+constexpr int kStages = 2;           // groups in shared memory
+constexpr int kBrickPoll = 8;        // lanes that poll a face line, a row each (fewer for many lines)
+// threads: the tiles' warps and those that fetch
+constexpr int kBrickFetchMax = 8;
+constexpr int kBrickMaxThreads = 32 * (kBrickWarps + kBrickFetchMax);
+// Doubles of a ring step: Wq p-face lines, Wp q-face lines, a column that is
+// never empty and one that is never read (for lanes with no face)
+__host__ __device__ constexpr int brick_pitch(bool full, bool d3) {
+  return full ? (d3 ? 16 : 4) : 32;
+}
+__host__ __device__ constexpr int brick_ring(bool full, bool d3) {
+  return kBrickRing * brick_pitch(full, d3);
+}
+constexpr int kBrickSmemMax = 226 * 1024;
 constexpr int kBrickSpin = 1 << 22;  // polls before a wait gives up
 
+// Shape of one sweep's layout, in the sweep's own (mirrored, if backward)
+// coordinates: row (w, p, q) is f = w sw + p sp + q sq, row f of the grid or
+// n - 1 - f.  Lines along w; tile (P, Q) of ntP x ntQ, lane tp + Wp tq.
+struct BrickShape {
+  int n, nw, np, nq;
+  int sw, sp, sq;
+  int Wp, Wq, LW;    // lines of a tile; LW = Wp Wq of them stored, rounded up to even
+  int CP, CQ;        // tiles of a brick
+  int ntP, ntQ, nbP, nbQ;
+  int NS;            // steps stored a tile: nw + Wp + Wq - 2 and its phase, in whole groups
+  int nwp;           // rows of a face line in memory
+  int bwd, d3;
+};
+
 struct BrickArgs {
-  int nrows, npos;         // rows of the sweep; positions (holes included)
-  int nx, ny, nz, BJ, nbJ, nbricks;
-  int in_ident, out_ident;  // in_idx / out_idx are the row itself
-  const int* border;       // [2 * nbricks]: (J, K) in hand-out order
-  const int* bbase;        // [nbJ * nz]: first position of brick (J, K) at J + nbJ K
-  const double* coef;      // [3][npos] by direction i, j, k; 0 where the row has no such term
-  const int* in_idx;       // [npos]
-  const int* out_idx;      // [npos]
-  const double* dval;      // [npos]
-  double* val;             // this sweep's value-as-flag array (by position)
-  const double* fval;      // the forward sweep's values (backward sweeps)
-  double* aux;             // by position
-  const double* auxin;
-  const double* idiag;     // by row (SOR)
+  BrickShape g;
+  int nbricks;
+  const int* border;      // [2 * nbricks]: (P, Q) of each brick in hand-out order
+  const double* coef;     // [tile][step][columns by lane]: brick_store
+  double* faces;          // [2][fsize]: the p faces, then the q faces
+  long long fsize, qface;  // doubles of one copy; where its q faces start
+  int* parity;            // which copy this sweep uses
+  const double* tin;      // the first sweep's values, by row
+  const double* tin2;     // SOR backward: its checkpoint
+  double* tout;           // first sweeps: where they go
+  double* tout2;          // SOR forward: the checkpoint
   double om1;
-  int use_t, write_out;
-  int fetch_sleep_ns;      // back-off of a fetch warp that saw nothing new
+  int write_out;
+  int poll;               // fetching lanes a face line
   unsigned* tickets;
   DevErr* err;
 };
 
-// A row's fold is three terms in a fixed direction order -- (k, j, i) or
-// (i, j, k), the reference's ascending-column slot order -- for every row: a
-// term the row does not have (at the grid boundary) has coefficient 0 and
-// value `absent`, and c * absent = -0 for ILU / SOR (sum - c v) and IC
-// (sum + c v) alike, which leaves every sum, -0 included, unchanged: the same
-// bits as skipping the term.
+// Modes with a stored column of diagonal factors.
+__host__ __device__ constexpr bool brick_has_diag(int mode) {
+  return mode == ELL_ILU_B || mode == ELL_ILUT_F || mode == ELL_ICC_F || mode == ELL_SOR_F ||
+         mode == ELL_SOR_B || mode == ELL_SOR_B0;
+}
+__host__ __device__ constexpr bool brick_bwd(int mode) {
+  return mode == ELL_ILU_B || mode == ELL_ILUT_B || mode == ELL_ICC_B || mode == ELL_SOR_B ||
+         mode == ELL_SOR_B0;
+}
+
+// A row's fold is one term a direction in a fixed order -- k, j, i forward,
+// i, j, k backward: the ascending columns -- for every row: a term the row
+// does not have (at the grid boundary) has coefficient 0 and value `absent`,
+// and c * absent = -0 for ILU / SOR (sum - c v) and IC (sum + c v) alike,
+// which leaves every sum, -0 included, unchanged: the same bits as skipping
+// the term.
 template <int MODE>
 __device__ __forceinline__ double brick_absent() {
   return (MODE == ELL_ICC_F || MODE == ELL_ICC_B) ? -0.0 : 0.0;
@@ -109,299 +152,529 @@ __device__ __forceinline__ double brick_term(double sum, double c, double v) {
     return FMA ? __fma_rn(-c, v, sum) : sub(sum, mul(c, v));
 }
 
-template <int MODE>
-__host__ __device__ constexpr bool brick_bwd() {
-  return MODE == ELL_ILU_B || MODE == ELL_ICC_B || MODE == ELL_SOR_B;
+// Columns of a step: the coefficients (of the line's own direction, then of
+// the two across in fold order) and the diagonal factor, in pairs of a lane's
+// neighbours in memory; then, staged beside them, the starting value and (SOR's
+// backward half) the forward value.
+__host__ __device__ constexpr int brick_coefs(int mode, bool d3) {
+  return (d3 ? 3 : 2) + (brick_has_diag(mode) ? 1 : 0);
+}
+__host__ __device__ constexpr int brick_cols(int mode, bool d3) {
+  return brick_coefs(mode, d3) + 1 + (mode == ELL_SOR_B ? 1 : 0);
 }
 
-// What a row needs, loaded kBrickAhead steps before it is computed.
+// What a row needs.
 struct BrickRow {
-  double ci, cj, ck;          // coefficients by direction
-  double sum0;                // the row's starting value
-  double dv;                  // diagonal factor (ILU_B, ICC_F, SOR)
-  double yf;                  // SOR_B: the forward value
-  int out;                    // output index (ILU_B, ICC_B, SOR)
+  double c0, c1, c2;  // coefficients in fold order
+  double sum0;        // the row's starting value
+  double dv;          // diagonal factor
+  double yf;          // SOR_B: the forward value
 };
+
+// ---- shared-memory staging: bulk copies counted on an mbarrier, and 8-byte
+// asynchronous copies by line
+__device__ __forceinline__ unsigned bk_smem(const void* p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void bk_mbar_init(unsigned long long* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bk_smem(bar)) : "memory");
+}
+__device__ __forceinline__ void bk_expect(unsigned long long* bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bk_smem(bar)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bk_bulk(void* dst, const void* src, unsigned bytes,
+                                        unsigned long long* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+          "r"(bk_smem(dst)),
+      "l"(src), "r"(bytes), "r"(bk_smem(bar))
+      : "memory");
+}
+__device__ __forceinline__ bool bk_wait(unsigned long long* bar, unsigned parity) {
+  for (int i = 0; i < kBrickSpin; i++) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bk_smem(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+// 8 bytes, or zeros (reading nothing) unless `ok`.
+__device__ __forceinline__ void bk_async8(unsigned dst, const double* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src),
+               "r"(ok ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void bk_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
 
 __device__ __forceinline__ bool brick_failed(DevErr* err) {
   return *reinterpret_cast<volatile int*>(&err->code) != 0;
 }
 
-// Take a value from its shared-memory ring slot and free the slot.
-__device__ __forceinline__ double brick_take(double* slot, DevErr* err) {
-  volatile unsigned long long* q = reinterpret_cast<volatile unsigned long long*>(slot);
-  unsigned long long b = *q;
-  for (int spins = 0; b == kPending; spins++) {
-    // give up at the budget, or early once another wait has given up
-    if (spins >= kBrickSpin || ((spins & 4095) == 4095 && brick_failed(err))) {
-      if (atomicCAS(&err->code, 0, GP_ERR_TIMEOUT) == 0) err->where = 41;
-      b = 0x7FF8000000000000ULL;
-      break;
-    }
-    b = *q;
-  }
-  *q = kPending;
-  return __longlong_as_double((long long)b);
+// Ring slots, by shared-memory address.  Not clobbering memory: their order
+// among each other is kept, and nothing else reads or writes a ring.  The
+// predicated forms are predicated instructions, not branches.
+__device__ __forceinline__ double ring_get(unsigned a) {
+  double v;
+  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void ring_put(unsigned a, double v) {
+  asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(a), "d"(v));
+}
+__device__ __forceinline__ void ring_put_if(bool p, unsigned a, double v) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+      "@p st.volatile.shared.f64 [%0], %1;\n\t}" ::"r"(a),
+      "d"(v), "r"((unsigned)p));
+}
+// Whether a slot is still empty.  The high word decides: no double with the
+// flag's high word is ever computed (every one is a signalling NaN).
+__device__ __forceinline__ bool empty_slot(double v) {
+  return (unsigned)__double2hiint(v) == (unsigned)(kPending >> 32);
+}
+__device__ __forceinline__ double pending_value() {
+  return __longlong_as_double((long long)kPending);
+}
+__device__ __forceinline__ double quiet_nan() {
+  return __longlong_as_double(0x7FF8000000000000LL);
+}
+// A step's operands from its stage: kept where they stand in the program (a
+// step before their use), past the waits that come between.
+__device__ __forceinline__ double stage_get(unsigned a) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void stage_get2(unsigned a, double& x, double& y) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(a));
+}
+// A tile's next step, to the writers of its ring: after the slots it emptied.
+__device__ __forceinline__ void publish(int* p, int step) {
+  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(bk_smem(p)), "r"(step) : "memory");
+}
+// A face value to the other bricks.
+__device__ __forceinline__ void face_put_if(bool p, double* a, double v) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+      "@p st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(a),
+      "d"(v), "r"((unsigned)p));
 }
 
-// Bulk prefetch of [p, p + bytes) into L2 (the 16-byte aligned interior of
-// the range; a hint that occupies no registers).
-__device__ __forceinline__ void l2_prefetch(const void* p, size_t bytes) {
-  const uintptr_t a = ((uintptr_t)p + 15) & ~(uintptr_t)15;
-  const uintptr_t e = ((uintptr_t)p + bytes) & ~(uintptr_t)15;
-  if (e > a)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a))
-                 : "memory");
-}
-
-__device__ __forceinline__ void compute_barrier(int nc) {
-  asm volatile("bar.sync 1, %0;" ::"r"(nc) : "memory");
-}
-
-// One fetch warp: each active lane has a ring column `col` and values for
-// steps [qlo, qhi) at val[src + q * stride].  The warp walks the steps in
-// order and hands a step's values to the ring once every lane that has one
-// sees it, each into its slot once the slot is free; kBrickPoll steps are
-// polled together.
-__device__ void brick_fetch(const BrickArgs& a, double* ring, bool act, int col, int qlo,
-                            int qhi, long long src, int stride) {
-  const unsigned full = 0xffffffffu;
-  volatile unsigned long long* cv = reinterpret_cast<volatile unsigned long long*>(ring) + col;
-  const int wq0 = __reduce_min_sync(full, act ? qlo : INT_MAX);
-  const int wq1 = __reduce_max_sync(full, act ? qhi : INT_MIN);
-  int q0 = wq0, spins = 0, held = 0;
-  while (q0 < wq1) {
-    bool ok[kBrickPoll];
-    unsigned long long bits[kBrickPoll];
-    bool run = true;
-#pragma unroll
-    for (int d = 0; d < kBrickPoll; d++) {
-      const int q = q0 + d;
-      const bool need = act && q >= qlo && q < qhi;
-      const bool fr = !need || cv[(size_t)(q & (kBrickSlots - 1)) * kBrickMaxFace] == kPending;
-      run = run && q < wq1 && __all_sync(full, fr);
-      ok[d] = run;
-      bits[d] = run && need ? ld_relaxed_bits(&a.val[src + (long long)q * stride]) : 0ull;
-    }
-    int got = 0;
-    run = true;
-#pragma unroll
-    for (int d = 0; d < kBrickPoll; d++) {
-      const int q = q0 + d;
-      const bool need = act && q >= qlo && q < qhi;
-      run = run && ok[d] && __all_sync(full, !need || bits[d] != kPending);
-      if (run) {
-        if (need) cv[(size_t)(q & (kBrickSlots - 1)) * kBrickMaxFace] = bits[d];
-        got++;
+// One lane of a fetch warp: rows i, i + poll, ... of one face line into
+// the reader's ring, row i at slot i + t0.  A row goes in once the reader is
+// less than a ring behind it (`prog`: its next step), and its place in the
+// line's other copy is emptied for the next sweep.
+template <int PITCH>
+__device__ void brick_fetch(const double* line, double* next, int i, int poll, int nw, unsigned ring,
+                            int t0, volatile const int* prog, bool act, DevErr* err) {
+  int spins = 0;
+  if (!act) i = nw;
+  while (__any_sync(0xffffffffu, i < nw)) {
+    if (i < nw) {
+      unsigned long long v = kPending;
+      const bool room = i + t0 < *prog + kBrickRing - 1;
+      if (room) v = ld_relaxed_bits(line + i);
+      if (++spins > kBrickSpin || ((spins & 1023) == 1023 && brick_failed(err))) {
+        // never arrived (or the reader never moved): record it and hand on a
+        // quiet NaN where there is room for one
+        if (atomicCAS(&err->code, 0, GP_ERR_TIMEOUT) == 0) err->where = 43;
+        if (!room) i = nw;
+        if (room && v == kPending) v = 0x7FF8000000000000ULL;
+      }
+      if (v != kPending) {
+        ring_put(ring + 8 * (((i + t0) & (kBrickRing - 1)) * PITCH),
+                 __longlong_as_double((long long)v));
+        next[i] = pending_value();
+        i += poll;
+        spins = 0;
       }
     }
-    if (got) {
-      q0 += got;
-      spins = held = 0;
-      continue;
-    }
-    // nothing handed on: the ring is full (the compute threads are a ring
-    // behind) or a value is not in yet
-    const bool failed = ((spins + held) & 1023) == 1023 && brick_failed(a.err);
-    if (!ok[0]) {
-      if (++held > kBrickSpin || failed) {
-        if (atomicCAS(&a.err->code, 0, GP_ERR_TIMEOUT) == 0) a.err->where = 42;
-        return;
-      }
-    } else if (++spins > kBrickSpin || failed) {
-      // a value never arrived: record it and hand on quiet NaNs for the step
-      if (atomicCAS(&a.err->code, 0, GP_ERR_TIMEOUT) == 0) a.err->where = 43;
-      const bool need = act && q0 >= qlo && q0 < qhi;
-      if (need) cv[(size_t)(q0 & (kBrickSlots - 1)) * kBrickMaxFace] = 0x7FF8000000000000ULL;
-      q0++;
-      spins = 0;
-      continue;
-    }
-    if (a.fetch_sleep_ns > 0) __nanosleep(a.fetch_sleep_ns);
   }
 }
 
-// ORD 0 folds k, j, i; ORD 1 folds i, j, k.  Launched with nc + nf threads:
-// nc = BJ rounded up to warps compute, nf = 32 (ceil(BJ / 32) + 1) fetch.
-template <int MODE, bool FMA, int ORD>
-__global__ void __launch_bounds__(kBrickThreads, 1) k_brick_sweep(const int* gate, int want,
-                                                                  BrickArgs a, DRef inr,
-                                                                  DRef outr) {
+// Steps are counted over the whole brick: line (pb, qb) of a brick is at row w
+// at step w + pb + qb, and a tile at (cp, cq) of its brick starts at the
+// multiple of kHalf below step cp Wp + cq Wq, `phase` steps before its first row.
+__host__ __device__ __forceinline__ int brick_phase(const BrickShape& g, int P, int Q) {
+  return ((P % g.CP) * g.Wp + (Q % g.CQ) * g.Wq) % kHalf;
+}
+
+// Launched with 32 (CP CQ + NF) threads: a warp a tile, then the fetch warps.
+// Dynamic shared memory: the tiles' rings, then their stages.  FULL: 32 lines
+// a tile (every address within a group is then an immediate offset).  D3: a
+// third direction (without it, two terms a row).
+//
+// A ring slot holds what was computed at the brick's step of that number, for
+// the step after it; writer and reader thus use the same slot at the same
+// place of a group, and no address within a group is computed.  The step's
+// instructions are what is left on the chain besides its FP64 operations, so
+// the loop is kept to about forty, nearly all without a branch.
+template <int MODE, bool FMA, bool FULL, bool D3>
+__global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* gate, int want,
+                                                                     BrickArgs a, DRef inr,
+                                                                     DRef outr) {
   if (gated_off(gate, want)) return;
-  constexpr bool BWD = brick_bwd<MODE>();
-  const double* __restrict__ in = inr.get();
+  constexpr bool BWD = brick_bwd(MODE);
+  constexpr bool DIAG = brick_has_diag(MODE);
+  constexpr int NC = brick_coefs(MODE, D3), NV = brick_cols(MODE, D3);
+  constexpr unsigned full = 0xffffffffu;
+  const BrickShape& g = a.g;
+  // second sweeps start from the first one's values; SOR's backward half
+  // without a forward one starts from the input
+  const double* __restrict__ in = MODE == ELL_SOR_B            ? a.tin2
+                                  : BWD && MODE != ELL_SOR_B0 ? a.tin
+                                                              : inr.get();
   double* __restrict__ out = outr.get();
-  __shared__ double sh[2][kBrickMaxLines];
-  // value rings: [slot][column]; columns 0..BJ-1 the k face (line t of the
-  // brick one plane below), column BJ the j face (the last line of the brick
-  // below in j)
-  __shared__ double ring[kBrickSlots * kBrickMaxFace];
+  extern __shared__ __align__(16) double brick_smem[];
+  __shared__ unsigned long long bars[kBrickWarps][kStages];
+  __shared__ int prog[kBrickWarps];  // each tile's next step
   __shared__ int s_brick;
-  const int t = threadIdx.x;
-  const int BJ = a.BJ;
-  const int nc = (BJ + 31) / 32 * 32;
-  const int nx = a.nx, ny = a.ny, npos = a.npos;
+  const int nw = g.nw, Wp = g.Wp, Wq = g.Wq, LW = FULL ? 32 : g.LW, NS = g.NS;
+  const int nt = g.CP * g.CQ, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int PITCH = brick_pitch(FULL, D3), RING = brick_ring(FULL, D3);
+  const int stage_n = kGroup * NV * LW;
+  double* const stages = brick_smem + nt * RING;
+  const unsigned ring0 = bk_smem(brick_smem);
+  const int par = *a.parity;
+  double* const f_now = a.faces + (par ? a.fsize : 0);
+  double* const f_next = a.faces + (par ? 0 : a.fsize);
   const double absent = brick_absent<MODE>();
-  const double pend = __longlong_as_double((long long)kPending);
-  for (int q = t; q < kBrickSlots * kBrickMaxFace; q += blockDim.x) ring[q] = pend;
+  for (int q = threadIdx.x; q < nt * RING; q += blockDim.x)
+    ring_put(ring0 + 8 * q, q % PITCH == PITCH - 2 ? absent : pending_value());
+  if (threadIdx.x < kBrickWarps * kStages) bk_mbar_init(&bars[0][0] + threadIdx.x);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  const int tq = lane / Wp, tp = lane - tq * Wp;
+  unsigned phases = 0;  // parity of each stage's next wait
   for (;;) {
-    if (t == 0) s_brick = (int)atomicAdd(&a.tickets[0], 1u);
+    if (threadIdx.x == 0) s_brick = (int)atomicAdd(&a.tickets[0], 1u);
+    if (threadIdx.x < nt)
+      prog[threadIdx.x] = (threadIdx.x % g.CP * Wp + threadIdx.x / g.CP * Wq) / kHalf * kHalf;
     __syncthreads();
     const int b = s_brick;
-    __syncthreads();  // every thread has read s_brick before it changes
     if (b >= a.nbricks) break;
-    const int J = a.border[2 * b], K = a.border[2 * b + 1];
-    const int bj = min(BJ, ny - J * BJ);
-    const int base = a.bbase[J + a.nbJ * K];
-    const int nsteps = nx + bj - 1;
-    if (t >= nc) {
-      // ---- fetch warps: the k face (lines 32 w .. 32 w + 31), then the j face
-      const int w = (t - nc) >> 5, lane = (t - nc) & 31;
-      if (w < (BJ + 31) / 32) {
-        if (K > 0) {
-          const int lt = 32 * w + lane;
-          brick_fetch(a, ring, lt < bj, lt, lt, lt + nx,
-                      (long long)a.bbase[J + a.nbJ * (K - 1)] + lt, BJ);
-        }
-      } else if (J > 0) {
-        // line 0 at step q = i takes row i of line BJ - 1 of brick (J - 1, K),
-        // which that brick reached at its step i + BJ - 1
-        brick_fetch(a, ring, lane == 0, BJ, 0, nx,
-                    (long long)a.bbase[J - 1 + a.nbJ * K] + (long long)(BJ - 1) * BJ + BJ - 1,
-                    BJ);
+    const int bP = a.border[2 * b], bQ = a.border[2 * b + 1];
+    if (warp >= nt) {
+      // ---- fetch: the brick's p faces (CQ Wq lines), then its q faces,
+      // a.poll lanes a line
+      const int np = g.CQ * Wq, lines = np + (D3 ? g.CP * Wp : 0);
+      const int t = threadIdx.x - 32 * nt, c = t / a.poll;
+      bool act = false;
+      long long line = 0;
+      int w = 0, col = 0, t0 = 0;
+      if (c < np) {
+        const int cq = c / Wq;
+        col = c - cq * Wq;
+        w = cq * g.CP;
+        t0 = c - 1;  // the step before row 0 of line (0, c)
+        const int Q = bQ * g.CQ + cq, ql = Q * Wq + col;
+        act = bP > 0 && ql < g.nq;
+        line = ((long long)bP * (g.ntQ * Wq) + ql) * g.nwp;
+      } else if (c < lines) {
+        const int cp = (c - np) / Wp, tl = c - np - cp * Wp;
+        w = cp;
+        t0 = c - np - 1;
+        col = Wq + tl;
+        const int P = bP * g.CP + cp, pl = P * Wp + tl;
+        act = bQ > 0 && pl < g.np;
+        line = a.qface + ((long long)bQ * (g.ntP * Wp) + pl) * g.nwp;
       }
+      brick_fetch<PITCH>(f_now + line, f_next + line, t % a.poll, a.poll,
+                         nw, ring0 + 8 * (w * RING + col), t0, &prog[w], act, a.err);
     } else {
-      // ---- compute: one line a thread
-      const bool line = t < bj;
-      const long long f_lo = (long long)nx * (J * BJ + (long long)ny * K);  // brick's first row
-      if (t == 0) {
-        // the brick's positions, and (forward sweeps) its rows of the input
-        const size_t pb = (size_t)nsteps * BJ * 8;
-        for (int d = 0; d < 3; d++) l2_prefetch(a.coef + (size_t)d * npos + base, pb);
-        if constexpr (MODE == ELL_ILU_B || MODE == ELL_ICC_F) l2_prefetch(a.dval + base, pb);
-        if (!a.in_ident) l2_prefetch(a.in_idx + base, pb / 2);
-        if (!a.out_ident) l2_prefetch(a.out_idx + base, pb / 2);
-        const long long r_lo = BWD ? a.nrows - f_lo - (long long)nx * bj : f_lo;
-        if constexpr (MODE == ELL_ILU_F || MODE == ELL_ICC_F || MODE == ELL_SOR_F ||
-                      MODE == ELL_SOR_B)
-          l2_prefetch(in + r_lo, (size_t)nx * bj * 8);
-        if constexpr (MODE == ELL_SOR_F || MODE == ELL_SOR_B)
-          l2_prefetch(a.idiag + r_lo, (size_t)nx * bj * 8);
-      }
-      // Every load of the ring is unconditional: a row outside the line's
-      // range (before its first step, after its last, or a line past the
-      // brick's edge) loads the nearest row of the brick instead, so no load
-      // result feeds a select and each stays in flight until its step.  The
-      // input index (a gather through in_idx) is loaded kBrickIdxAhead steps
-      // ahead, the row data kBrickAhead steps ahead.
-      const int tl = min(t, bj - 1);
-      const long long fl = (long long)nx * (J * BJ + tl + (long long)ny * K);
-      auto clamp_li = [&](int s) { return min(max(s - tl, 0), nx - 1); };
-      auto row_at = [&](int li) {
-        return BWD ? (int)(a.nrows - 1 - (fl + li)) : (int)(fl + li);
-      };
-      int ixr[kBrickRing];
-      auto load_idx = [&](int s, int& ix) {
-        if (!a.in_ident) ix = a.in_idx[base + (clamp_li(s) + tl) * BJ + tl];
-      };
-      auto load = [&](int s, int ix, BrickRow& w) {
-        const int li = clamp_li(s);
-        const int p = base + (li + tl) * BJ + tl;
-        const int r = row_at(li);
-        w.ci = a.coef[p];
-        w.cj = a.coef[(size_t)npos + p];
-        w.ck = a.coef[2 * (size_t)npos + p];
-        const int ii = a.in_ident ? r : ix;
-        if constexpr (MODE == ELL_ILU_F || MODE == ELL_ICC_F) w.sum0 = in[ii];
-        if constexpr (MODE == ELL_ILU_B) w.sum0 = a.fval[ii];
-        if constexpr (MODE == ELL_ICC_B) w.sum0 = a.auxin[ii];
-        if constexpr (MODE == ELL_SOR_F) w.sum0 = in[r];
-        if constexpr (MODE == ELL_SOR_B) {
-          if (a.use_t) {
-            w.sum0 = a.auxin[ii];
-            w.yf = a.fval[ii];
-          } else {
-            w.sum0 = in[r];
-            w.yf = 0.0;
-          }
-        }
-        if constexpr (MODE == ELL_ILU_B || MODE == ELL_ICC_F) w.dv = a.dval[p];
-        if constexpr (MODE == ELL_SOR_F || MODE == ELL_SOR_B) w.dv = a.idiag[r];
-        if constexpr (MODE == ELL_ILU_B || MODE == ELL_ICC_B)
-          w.out = a.out_ident ? r : a.out_idx[p];
-        if constexpr (MODE == ELL_SOR_F || MODE == ELL_SOR_B) w.out = r;
-      };
-      BrickRow rr[kBrickRing];
-#pragma unroll
-      for (int q = 0; q < kBrickIdxAhead; q++) load_idx(q, ixr[q]);
-#pragma unroll
-      for (int q = 0; q < kBrickAhead; q++) load(q, ixr[q], rr[q]);
-      double prev = absent;  // the line's previous value (none before its first row)
-      double* const col_k = ring + t;
-      double* const col_j = ring + BJ;
-      for (int L0 = 0; L0 < nsteps; L0 += kBrickRing) {
-#pragma unroll
-        for (int q = 0; q < kBrickRing; q++) {
-          const int L = L0 + q;
-          if (L + kBrickIdxAhead < nsteps)
-            load_idx(L + kBrickIdxAhead, ixr[(q + kBrickIdxAhead) % kBrickRing]);
-          if (L + kBrickAhead < nsteps)
-            load(L + kBrickAhead, ixr[(q + kBrickAhead) % kBrickRing],
-                 rr[(q + kBrickAhead) % kBrickRing]);
-          const BrickRow& w = rr[q];
-          const int par = L & 1;
-          const int li = L - t;
-          const size_t so = (size_t)(L & (kBrickSlots - 1)) * kBrickMaxFace;
-          if (line && li >= 0 && li < nx) {
-            double sum = w.sum0;
-            if constexpr (ORD == 0) {
-              const double vk = K > 0 ? brick_take(col_k + so, a.err) : absent;
-              sum = brick_term<MODE, FMA>(sum, w.ck, vk);
-              const double vj =
-                  t > 0 ? sh[par ^ 1][t - 1] : J > 0 ? brick_take(col_j + so, a.err) : absent;
-              sum = brick_term<MODE, FMA>(sum, w.cj, vj);
-              sum = brick_term<MODE, FMA>(sum, w.ci, prev);
-            } else {
-              sum = brick_term<MODE, FMA>(sum, w.ci, prev);
-              const double vj =
-                  t > 0 ? sh[par ^ 1][t - 1] : J > 0 ? brick_take(col_j + so, a.err) : absent;
-              sum = brick_term<MODE, FMA>(sum, w.cj, vj);
-              const double vk = K > 0 ? brick_take(col_k + so, a.err) : absent;
-              sum = brick_term<MODE, FMA>(sum, w.ck, vk);
+      // ---- compute: one tile
+      const int cq = warp / g.CP, cp = warp - cq * g.CP;
+      const int P = bP * g.CP + cp, Q = bQ * g.CQ + cq;
+      if (P < g.ntP && Q < g.ntQ) {
+        const int pl = P * Wp + tp, ql = Q * Wq + tq;
+        const bool line = lane < Wp * Wq && pl < g.np && ql < g.nq;
+        const int phase = (cp * Wp + cq * Wq) % kHalf;
+        const int sb = cp * Wp + cq * Wq - phase;  // the tile's first step
+        // the tile's step s (counted from sb) is row s - off of the lane's line
+        const int off = line ? phase + tp + tq : INT_MAX / 2;  // an idle lane never starts
+        const int ll = line ? lane : 0;
+        // the line's row w is at row0 + rs w
+        const long long rs = BWD ? -(long long)g.sw : g.sw;
+        const long long f0 = line ? pl * (long long)g.sp + ql * (long long)g.sq : 0;
+        const long long row0 = BWD ? g.n - 1 - f0 : f0;
+        const double* const cf = a.coef + (long long)(P + g.ntP * Q) * NS * NC * LW;
+        double* const stage = stages + warp * (kStages * stage_n);
+        const int ngroups = NS / kGroup;
+        const long long roff = row0 - rs * (line ? off : 0);  // step 0's row
+        const double* src = in + roff;
+        const double* src2 = MODE == ELL_SOR_B ? a.tin + roff : nullptr;
+        // stage group q (steps kGroup q ..): one commit group a call, empty
+        // where the sweep has no more steps
+        auto fill = [&](int q, int si) {
+          double* const st = stage + si * stage_n;
+          if (q < ngroups) {
+            if (lane == 0) {
+              unsigned long long* bar = &bars[warp][si];
+              constexpr unsigned cb1 = kGroup * NC * 8;
+              // the stage's last readers are behind a __syncwarp
+              bk_expect(bar, cb1 * LW);
+              bk_bulk(st, cf + (long long)q * (kGroup * NC * LW), cb1 * LW, bar);
             }
-            // the value other bricks wait on goes out first
-            double y;
-            if constexpr (MODE == ELL_ILU_B || MODE == ELL_SOR_F)
-              y = mul(sum, w.dv);
-            else if constexpr (MODE == ELL_SOR_B)
-              y = a.use_t ? add(mul(a.om1, w.yf), mul(sum, w.dv)) : mul(sum, w.dv);
-            else
-              y = sum;
-            const int p = base + L * BJ + t;
-            st_relaxed(&a.val[p], y);
-            sh[par][t] = y;
-            prev = y;
-            if constexpr (MODE == ELL_ILU_B || MODE == ELL_ICC_B) {
-              out[w.out] = y;
-            } else if constexpr (MODE == ELL_ICC_F) {
-              a.aux[p] = mul(sum, w.dv);
-            } else if constexpr (MODE == ELL_SOR_F) {
-              a.aux[p] = sum;
-              if (a.write_out) out[w.out] = y;
-            } else if constexpr (MODE == ELL_SOR_B) {
-              out[w.out] = y;
+            const int w0 = q * kGroup - off;
+            const unsigned dst = bk_smem(st + kGroup * NC * LW + lane);
+            if (lane < LW) {
+#pragma unroll
+              for (int u = 0; u < kGroup; u++) {
+                const bool ok = (unsigned)(w0 + u) < (unsigned)nw;
+                bk_async8(dst + u * 8 * LW, src + rs * u, ok);
+                if constexpr (MODE == ELL_SOR_B)
+                  bk_async8(dst + (kGroup + u) * 8 * LW, src2 + rs * u, ok);
+              }
             }
+            src += rs * kGroup;
+            if constexpr (MODE == ELL_SOR_B) src2 += rs * kGroup;
           }
-          compute_barrier(nc);
+          bk_commit();
+        };
+        // where this tile's face values come from and go to
+        const unsigned ring = ring0 + 8 * warp * RING;
+        const bool fromp = line && tp == 0 && P > 0, fromq = D3 && line && tq == 0 && Q > 0;
+        const bool faces = __any_sync(full, fromp || fromq);
+        const bool lastp = line && tp == Wp - 1 && P + 1 < g.ntP;
+        const bool lastq = D3 && line && tq == Wq - 1 && Q + 1 < g.ntQ;
+        const bool outs = __any_sync(full, lastp || lastq);
+        const bool ringp = cp + 1 < g.CP && P + 1 < g.ntP, ringq = cq + 1 < g.CQ && Q + 1 < g.ntQ;
+        const bool rings = ringp || ringq;
+        // this lane's columns: read from, emptied, and the neighbouring tiles'
+        const unsigned colp = ring + 8 * tq, colq = ring + 8 * (Wq + tp);
+        const unsigned full_col = ring + 8 * (PITCH - 2), no_col = ring + 8 * (PITCH - 1);
+        const unsigned rp = fromp ? colp : full_col, rq = fromq ? colq : full_col;
+        const unsigned ep = fromp ? colp : no_col, eq = fromq ? colq : no_col;
+        const unsigned np = lastp && ringp ? colp + 8 * RING : no_col;
+        const unsigned nq = lastq && ringq ? colq + 8 * g.CP * RING : no_col;
+        const bool outp = lastp && !ringp, outq = lastq && !ringq;
+        const int nwop = outp ? nw : 0, nwoq = outq ? nw : 0;
+        // face lines this lane writes (row -off at the pointer)
+        double* fop = f_now + ((long long)(bP + 1) * (g.ntQ * Wq) + ql) * g.nwp - (outp ? off : 0);
+        double* foq = f_now + a.qface + ((long long)(bQ + 1) * (g.ntP * Wp) + pl) * g.nwp -
+                      (outq ? off : 0);
+        double* po = (BWD ? out : a.tout) + roff;  // step 0's row
+        double* pt2 = MODE == ELL_SOR_F ? a.tout2 + roff : nullptr;
+        double* pw = MODE == ELL_SOR_F && a.write_out ? out + roff : nullptr;
+        for (int q = 0; q < kStages; q++) fill(q, q);
+        // a face lane's value for the step at hand, `absent` where it has none
+        unsigned before = 8 * ((sb - 1) & (kBrickRing - 1)) * PITCH;  // the last step's slot
+        double fp = ring_get(rp + before), fq = ring_get(rq + before);
+        double prev = absent;  // the lane's last value (none before its first row)
+        int si = 0;
+        for (int s0 = 0; s0 < NS; s0 += kGroup) {
+          // the group's stage: this lane's copies (all lanes' behind the
+          // __syncwarp), then the bulk copy
+          asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+          if (!bk_wait(&bars[warp][si], phases >> si & 1u)) {
+            if (atomicCAS(&a.err->code, 0, GP_ERR_TIMEOUT) == 0) a.err->where = 44;
+          }
+          phases ^= 1u << si;
+          __syncwarp();
+          const unsigned st = bk_smem(stage + si * stage_n);
+          unsigned c0 = st + 16 * ll, v0 = st + 8 * (kGroup * NC * LW + ll);
+          unsigned c1 = st + 16 * LW + (D3 && DIAG ? 16 : 8) * ll;
+          auto take = [&](int u) {
+            BrickRow r;
+            r.sum0 = stage_get(v0 + 8 * u * LW);
+            stage_get2(c0 + 8 * u * NC * LW, r.c0, r.c1);
+            if constexpr (D3 && DIAG)
+              stage_get2(c1 + 8 * u * NC * LW, r.c2, r.dv);
+            else if constexpr (D3)
+              r.c2 = stage_get(c1 + 8 * u * NC * LW);
+            else if constexpr (DIAG)
+              r.dv = stage_get(c1 + 8 * u * NC * LW);
+            if constexpr (MODE == ELL_SOR_B) r.yf = stage_get(v0 + 8 * (kGroup + u) * LW);
+            return r;
+          };
+          BrickRow r = take(0);
+          // with_faces: some lane reads face values; with_out: some lane's are read
+          auto steps = [&](auto with_faces, auto with_out) {
+            constexpr bool FACES = decltype(with_faces)::value, OUTS = decltype(with_out)::value;
+            // unrolled over half a group: the code has to stay in the
+            // instruction cache of the sub-partition that runs it
+#pragma unroll 1
+            for (int u0 = 0; u0 < kGroup; u0 += kHalf) {
+              if constexpr (FACES) {
+                if (u0) {  // the slots of the steps so far are free
+                  __syncwarp();
+                  if (lane == 0) publish(&prog[warp], sb + s0 + u0);
+                }
+              }
+              if constexpr (OUTS) {
+                // room in the rings of the neighbouring tiles for the next values
+                if (rings) {
+                  for (int spins = 0;; spins++) {
+                    const int at_p = ringp ? *(volatile int*)&prog[warp + 1] : INT_MAX / 2;
+                    const int at_q = ringq ? *(volatile int*)&prog[warp + g.CP] : INT_MAX / 2;
+                    if (sb + s0 + u0 + kHalf < min(at_p, at_q) + kBrickRing) break;
+                    if (spins > kBrickSpin || ((spins & 4095) == 4095 && brick_failed(a.err))) {
+                      if (lane == 0 && atomicCAS(&a.err->code, 0, GP_ERR_TIMEOUT) == 0)
+                        a.err->where = 42;
+                      break;
+                    }
+                  }
+                }
+              }
+              const unsigned slot = 8 * (((sb + s0 + u0) & (kBrickRing - 1)) * PITCH);
+#pragma unroll
+              for (int h = 0; h < kHalf; h++) {
+              const int u = u0 + h, w = s0 - off + u;
+              const bool act = (unsigned)w < (unsigned)nw;
+              double vp = __shfl_up_sync(full, prev, 1);
+              double vq = absent;
+              if constexpr (D3) vq = __shfl_up_sync(full, prev, Wp);
+              double sum = brick_term<MODE, FMA>(r.sum0, r.c0, prev);
+              // the next row's operands, behind the shuffles in the queue
+              BrickRow ahead;
+              if (h + 1 < kHalf || u0 == 0) ahead = take(h + 1);
+              if constexpr (FACES) {
+                // inactive lanes have no value to wait for, and any will do
+                if (__any_sync(full, act && (empty_slot(fp) || (D3 && empty_slot(fq))))) {
+                  int spins = 0;
+                  do {
+                    if (empty_slot(fp)) fp = ring_get(rp + before);
+                    if (D3 && empty_slot(fq)) fq = ring_get(rq + before);
+                    if (++spins > kBrickSpin || ((spins & 4095) == 4095 && brick_failed(a.err))) {
+                      if (atomicCAS(&a.err->code, 0, GP_ERR_TIMEOUT) == 0) a.err->where = 41;
+                      if (empty_slot(fp)) fp = quiet_nan();
+                      if (empty_slot(fq)) fq = quiet_nan();
+                    }
+                  } while (__any_sync(full, act && (empty_slot(fp) || (D3 && empty_slot(fq)))));
+                }
+                if (tp == 0) vp = fp;
+                if (D3 && tq == 0) vq = fq;
+                ring_put(ep + before, pending_value());
+                if constexpr (D3) ring_put(eq + before, pending_value());
+                // a first look at the next step's values
+                before = slot + h * (8 * PITCH);
+                fp = ring_get(rp + before);
+                if constexpr (D3) fq = ring_get(rq + before);
+              } else {
+                if (tp == 0) vp = absent;
+                if (D3 && tq == 0) vq = absent;
+              }
+              // forward: k, j, i = own, q, p; backward: i, j, k = own, p, q
+              if constexpr (!D3) {
+                sum = brick_term<MODE, FMA>(sum, r.c1, vp);
+              } else if constexpr (!BWD) {
+                sum = brick_term<MODE, FMA>(sum, r.c1, vq);
+                sum = brick_term<MODE, FMA>(sum, r.c2, vp);
+              } else {
+                sum = brick_term<MODE, FMA>(sum, r.c1, vp);
+                sum = brick_term<MODE, FMA>(sum, r.c2, vq);
+              }
+              double y;
+              if constexpr (MODE == ELL_ILU_B || MODE == ELL_ILUT_F || MODE == ELL_SOR_F ||
+                            MODE == ELL_SOR_B0)
+                y = mul(sum, r.dv);
+              else if constexpr (MODE == ELL_SOR_B)
+                y = add(mul(a.om1, r.yf), mul(sum, r.dv));
+              else
+                y = sum;
+              prev = act ? y : prev;
+              // the values other tiles wait on go out first
+              if constexpr (OUTS) {
+                ring_put_if(act, np + slot + h * (8 * PITCH), y);
+                if constexpr (D3) ring_put_if(act, nq + slot + h * (8 * PITCH), y);
+                face_put_if((unsigned)w < (unsigned)nwop, fop + h, y);
+                if constexpr (D3) face_put_if((unsigned)w < (unsigned)nwoq, foq + h, y);
+              }
+              const double t = MODE == ELL_ICC_F ? mul(sum, r.dv) : y;
+              if (act) po[rs * h] = t;
+              if constexpr (MODE == ELL_SOR_F) {
+                if (act) pt2[rs * h] = sum;
+                if (act && pw) pw[rs * h] = y;
+              }
+              r = ahead;
+              }
+              c0 += 8 * kHalf * NC * LW;
+              c1 += 8 * kHalf * NC * LW;
+              v0 += 8 * kHalf * LW;
+              fop += kHalf;
+              foq += kHalf;
+              po += rs * kHalf;
+              if constexpr (MODE == ELL_SOR_F) {
+                pt2 += rs * kHalf;
+                if (pw) pw += rs * kHalf;
+              }
+            }
+          };
+          if (faces)
+            steps(std::true_type{}, std::true_type{});
+          else if (outs)
+            steps(std::false_type{}, std::true_type{});
+          else
+            steps(std::false_type{}, std::false_type{});
+          __syncwarp();  // the stage is read, the ring's slots are free
+          fill(s0 / kGroup + kStages, si);
+          si = si + 1 == kStages ? 0 : si + 1;
+          if (faces && lane == 0) publish(&prog[warp], sb + s0 + kGroup);
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
       }
     }
     __syncthreads();
   }
-  if (t == 0 && atomic_add_acq_rel(&a.tickets[1], 1u) == gridDim.x - 1) {
+  if (threadIdx.x == 0 && atomic_add_acq_rel(&a.tickets[1], 1u) == gridDim.x - 1) {
     a.tickets[0] = 0u;
     a.tickets[1] = 0u;
+    *a.parity = par ^ 1;
   }
+}
+
+// Stored coefficients from the factor (or operator) values: one thread a
+// position of [tile][step][lane], its coefficients in fold order (0 where the
+// row has no such term or there is no row) and the diagonal: src[dslot[row]],
+// or diag[row] for SOR.  With `stale`, only while that word is set.
+__global__ void k_brick_refresh(const int* gate, int want, BrickShape g, int nc, int npos,
+                                const int* __restrict__ slot, const int* __restrict__ dslot,
+                                const double* __restrict__ src, const double* __restrict__ diag,
+                                double* __restrict__ coef, const int* stale) {
+  if (gated_off(gate, want)) return;
+  if (stale && !*stale) return;
+  const int nd = g.d3 ? 3 : 2;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < npos; e += gridDim.x * blockDim.x) {
+    const int lane = e % g.LW, ts = e / g.LW, s = ts % g.NS, T = ts / g.NS;
+    const int P = T % g.ntP, Q = T / g.ntP, tq = lane / g.Wp, tp = lane - tq * g.Wp;
+    const int w = s - tp - tq - brick_phase(g, P, Q), p = P * g.Wp + tp, q = Q * g.Wq + tq;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (lane < g.Wp * g.Wq && w >= 0 && w < g.nw && p < g.np && q < g.nq) {
+      const int f = w * g.sw + p * g.sp + q * g.sq, row = g.bwd ? g.n - 1 - f : f;
+      for (int d = 0; d < nd; d++) {
+        // fold order: k, j, i forward and i, j, k backward
+        const int c = slot[(size_t)(g.bwd ? d : nd - 1 - d) * g.n + row];
+        if (c >= 0) v[d] = src[c];
+      }
+      if (nc > nd) v[nd] = diag ? diag[row] : src[dslot[row]];
+    }
+    // columns 0 and 1 as pairs by lane, then the rest: a pair or a column
+    double* const c = coef + (size_t)ts * nc * g.LW;
+    c[2 * lane] = v[0];
+    c[2 * lane + 1] = v[1];
+    if (nc == 4) {
+      c[2 * g.LW + 2 * lane] = v[2];
+      c[2 * g.LW + 2 * lane + 1] = v[3];
+    } else if (nc == 3) {
+      c[2 * g.LW + lane] = v[2];
+    }
+  }
+}
+
+__global__ void k_brick_clear(long long n, double* __restrict__ faces) {
+  const double p = __longlong_as_double((long long)kPending);
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
+       q += (long long)gridDim.x * blockDim.x)
+    faces[q] = p;
 }
 
 // ------------------------------------------------------------------ host
@@ -412,15 +685,12 @@ static int bup(T** d, const std::vector<T>& h) {
   return GP_OK;
 }
 
-// Settings of later set-ups (gp_set_sweep_bricks; GPETSC_SWEEP_BRICKS,
-// GPETSC_BRICK_LINES, GPETSC_BRICK_CTAS_PER_SM and GPETSC_BRICK_FETCH_SLEEP_NS
-// set the defaults).
+// Settings of later set-ups (gp_set_sweep_bricks; GPETSC_SWEEP_BRICKS and
+// GPETSC_BRICK_LINES set the defaults).
 struct BrickTuning {
-  int mode = 0;        // 0 never, 1 where the model says it is faster, 2 wherever it applies
-  int BJ = 0;          // lines of a brick; 0: chosen by the model
-  int ctas_per_sm = 1;
-  int max_ctas = 0;    // cap on the persistent grid (0: none)
-  int fetch_sleep_ns = 0;
+  int mode = 1;      // 0 never, 1 where the model says it is faster, 2 wherever it applies
+  int BJ = 0;        // lines of a brick (of one plane); 0: chosen
+  int max_ctas = 0;  // cap on the persistent grid (0: none)
 };
 static BrickTuning& brick_tuning() {
   static BrickTuning t = [] {
@@ -429,10 +699,6 @@ static BrickTuning& brick_tuning() {
       v.mode = std::max(0, std::min(2, std::atoi(e)));
     if (const char* e = std::getenv("GPETSC_BRICK_LINES"))
       v.BJ = std::max(0, std::min(kBrickMaxLines, std::atoi(e)));
-    if (const char* e = std::getenv("GPETSC_BRICK_CTAS_PER_SM"))
-      v.ctas_per_sm = std::max(1, std::min(4, std::atoi(e)));
-    if (const char* e = std::getenv("GPETSC_BRICK_FETCH_SLEEP_NS"))
-      v.fetch_sleep_ns = std::max(0, std::min(1000, std::atoi(e)));
     return v;
   }();
   return t;
@@ -447,252 +713,311 @@ void set_sweep_bricks(int mode, int lines, int max_ctas) {
 // Grid detection: every row r (in sweep coordinates f = r forward, n-1-r
 // backward; i = f % nx, j = f / nx % ny, k = f / (nx ny)) depends on exactly
 // its grid neighbours r -/+ 1 (when i >= 1), nx (j >= 1) and nx ny (k >= 1),
-// listed in one direction order for every row -- k, j, i (ord 0) or i, j, k
-// (ord 1) -- so that each row's fold is the three-term fold with absent
-// terms at the grid boundary.  On success slot[d][r] is the coefficient slot
-// of row r's term in direction d (-1 where it has none).
+// listed with ascending columns.  The sweep's last row has every coordinate at
+// its end, so its dependencies give the grid's sizes.  On success slot[d][r]
+// is the coefficient slot of row r's term in direction d (-1 where it has
+// none).
 static bool brick_detect(int n, bool forward, const std::vector<int>& dptr,
-                         const std::vector<int>& dcol, const std::vector<int>& dsl,
-                         int* nx_out, int* ny_out, int* nz_out, int* ord_out,
+                         const std::vector<int>& dcol, const std::vector<int>& dsl, int* dims,
                          std::vector<int>& slot) {
-  std::vector<long long> offs;
-  for (int r = 0; r < n; r++) {
-    if (dptr[r + 1] - dptr[r] > 3) return false;
-    for (int q = dptr[r]; q < dptr[r + 1]; q++) {
-      const long long o = forward ? (long long)r - dcol[q] : (long long)dcol[q] - r;
-      if (o <= 0) return false;
-      if (std::find(offs.begin(), offs.end(), o) == offs.end()) {
-        offs.push_back(o);
-        if (offs.size() > 3) return false;
-      }
-    }
-  }
-  std::sort(offs.begin(), offs.end());
-  if (offs.empty() || offs[0] != 1) return false;
-  const long long nx = offs.size() >= 2 ? offs[1] : n;
-  const long long nxny = offs.size() >= 3 ? offs[2] : n;
-  if (nx <= 1 || nxny % nx || n % nxny) return false;
+  if (n < 2) return false;
+  const int last = forward ? n - 1 : 0, nd = dptr[last + 1] - dptr[last];
+  if (nd < 1 || nd > 3) return false;
+  long long offs[3];
+  for (int q = 0; q < nd; q++)
+    offs[q] = std::llabs((long long)dcol[dptr[last] + q] - last);
+  std::sort(offs, offs + nd);
+  if (offs[0] != 1) return false;
+  const long long nx = nd >= 2 ? offs[1] : n, nxny = nd >= 3 ? offs[2] : n;
+  if (nx <= 1 || nxny % nx || n % nxny || nxny < nx) return false;
   const long long ny = nxny / nx;
-  int ord = -1;
-  slot.assign((size_t)3 * n, -1);
-  for (int r = 0; r < n; r++) {
-    const long long f = forward ? r : (long long)n - 1 - r;
-    const long long i = f % nx, j = (f / nx) % ny, k = f / nxny;
-    const int want = (i >= 1 ? 1 : 0) | (j >= 1 ? 2 : 0) | (k >= 1 ? 4 : 0);
-    int seen = 0, last = -1, up_all = -1;
-    for (int q = dptr[r]; q < dptr[r + 1]; q++) {
-      const long long o = forward ? (long long)r - dcol[q] : (long long)dcol[q] - r;
-      const int d = o == 1 ? 0 : o == nx ? 1 : o == nxny ? 2 : -1;
-      if (d < 0 || !(want >> d & 1) || (seen >> d & 1)) return false;
-      if (last >= 0) {
-        const int up = d > last ? 1 : 0;  // ord 1 ascends i, j, k; ord 0 descends
-        if (up_all >= 0 && up != up_all) return false;
-        up_all = up;
+  slot.resize((size_t)3 * n);
+  std::atomic<bool> ok{true};
+  host_parallel_for(n, [&](int64_t r0, int64_t r1) {
+    for (int64_t r = r0; r < r1; r++) {
+      const long long f = forward ? r : (long long)n - 1 - r;
+      const long long c[3] = {f % nx, (f / nx) % ny, f / nxny}, o[3] = {1, nx, nxny};
+      int q = dptr[r];
+      // ascending columns: k, j, i forward, i, j, k backward
+      for (int e = 0; e < 3; e++) {
+        const int d = forward ? 2 - e : e;
+        int sl = -1;
+        if (c[d] >= 1) {
+          if (q >= dptr[r + 1] || dcol[q] != (forward ? r - o[d] : r + o[d])) {
+            ok = false;
+            return;
+          }
+          sl = dsl[q++];
+        }
+        slot[(size_t)d * n + r] = sl;
       }
-      seen |= 1 << d;
-      last = d;
-      slot[(size_t)d * n + r] = dsl[q];
+      if (q != dptr[r + 1]) {
+        ok = false;
+        return;
+      }
     }
-    if (seen != want) return false;  // the full stencil, nothing missing
-    if (up_all >= 0) {
-      if (ord >= 0 && ord != up_all) return false;
-      ord = up_all;
-    }
+  });
+  dims[0] = (int)nx;
+  dims[1] = (int)ny;
+  dims[2] = (int)(n / nxny);
+  return ok;
+}
+
+// Modelled duration of one brick sweep (us): the chain of nx + ny + nz - 2
+// rows at a step each plus a hand-off a brick face, or the bricks' steps over
+// the SMs, whichever is longer.  The other forms take at least 1.25 us a
+// dependency level in level order, or 0.4 us a level and the staging of a
+// chunk (their own model, gp_sweep.cu).
+constexpr double kBrickStep = 0.22, kBrickHandoff = 2.0, kBrickStart = 4.0;
+static double other_model_us(int nlevels) { return std::min(1.25 * nlevels, 20.0 + 0.4 * nlevels); }
+static double brick_model_us(const BrickShape& g) {
+  const double chain = (g.nw + g.np + g.nq - 2) * kBrickStep + (g.nbP + g.nbQ - 2) * kBrickHandoff;
+  const double rounds = std::ceil((double)g.nbP * g.nbQ / std::max(1, num_sms()));
+  return kBrickStart + std::max(chain, rounds * (g.NS * kBrickStep + kBrickStart));
+}
+
+static BrickShape brick_shape(const int* dims, bool bwd, int lines) {
+  BrickShape g{};
+  const int nx = dims[0], ny = dims[1], nz = dims[2];
+  g.n = nx * ny * nz;
+  g.bwd = bwd ? 1 : 0;
+  g.d3 = nz > 1 ? 1 : 0;
+  if (bwd) {  // along i, across j and k
+    g.nw = nx, g.np = ny, g.nq = nz;
+    g.sw = 1, g.sp = nx, g.sq = nx * ny;
+  } else if (nz > 1) {  // along k, across i and j
+    g.nw = nz, g.np = nx, g.nq = ny;
+    g.sw = nx * ny, g.sp = 1, g.sq = nx;
+  } else {  // along j, across i
+    g.nw = ny, g.np = nx, g.nq = 1;
+    g.sw = nx, g.sp = 1, g.sq = 0;
   }
-  *nx_out = (int)nx;
-  *ny_out = (int)ny;
-  *nz_out = (int)(n / nxny);
-  *ord_out = ord < 0 ? 0 : ord;
-  return true;
+  if (lines > 0) {
+    // forced: `lines` neighbouring lines (more than a warp's in equal parts)
+    const int bp = std::min({lines, nx, ny}), most = g.d3 ? 29 : 32;
+    g.CP = std::min(kBrickWarps, (bp + most - 1) / most);
+    g.CQ = 1;
+    g.Wp = std::min(most, (bp + g.CP - 1) / g.CP);
+    g.Wq = 1;
+  } else {
+    // 3-D: 8 x 4 lines a warp and 2 x 2 warps, the least surface of the
+    // shapes that fill a warp; 2-D: 32 lines a warp and 4 warps in a row
+    g.Wp = std::min(g.np, g.d3 ? 8 : 32);
+    g.Wq = std::max(1, std::min(g.nq, 32 / g.Wp));
+    if (g.d3) g.Wq = std::min(g.Wq, 30 - g.Wp);  // a ring step's columns
+    const int tp = (g.np + g.Wp - 1) / g.Wp, tq = (g.nq + g.Wq - 1) / g.Wq;
+    g.CQ = tp == 1 ? std::min(tq, kBrickWarps) : tq == 1 ? 1 : 2;
+    g.CP = std::min(tp, kBrickWarps / g.CQ);
+  }
+  g.LW = (g.Wp * g.Wq + 1) & ~1;  // bulk copies of whole 16 bytes
+  g.ntP = (g.np + g.Wp - 1) / g.Wp;
+  g.ntQ = (g.nq + g.Wq - 1) / g.Wq;
+  g.nbP = (g.ntP + g.CP - 1) / g.CP;
+  g.nbQ = (g.ntQ + g.CQ - 1) / g.CQ;
+  int phase = 0;  // the largest of any tile of a brick
+  for (int cp = 0; cp < g.CP; cp++)
+    for (int cq = 0; cq < g.CQ; cq++)
+      phase = std::max(phase, (cp * g.Wp + cq * g.Wq) % kHalf);
+  g.NS = (g.nw + g.Wp + g.Wq - 2 + phase + kGroup - 1) / kGroup * kGroup;
+  g.nwp = (g.nw + 3) & ~3;  // whole sectors
+  return g;
 }
 
-// Modelled duration of one brick sweep (us), from GB300 measurements: a
-// step is the on-SM chain (three dependent FP64 operations of 64 cycles,
-// shared memory, the compute barrier) or the SM's FP64 rate (~4 warp
-// instructions a row, one a sub-partition every 64 cycles), whichever is
-// longer; each brick boundary on the critical path costs a hand-off through
-// L2 and the fetch ring, plus, along j, the BJ - 1 steps line BJ - 1 runs
-// behind line 0.
-static double brick_model_us(int nx, int ny, int nz, int BJ) {
-  const double lat_step_us = 0.15, handoff_us = 0.8;
-  const int nbJ = (ny + BJ - 1) / BJ;
-  const int warps = (BJ + 31) / 32;
-  const double step_us = std::max(lat_step_us, (warps + 3) / 4 * 4.0 * 64.0 / 2.07e3);
-  return (nbJ - 1) * ((BJ - 1) * step_us + handoff_us) + (nz - 1) * handoff_us +
-         (nx + BJ - 1) * step_us;
+static BrickShape shape_of(const EllSweep& e) {
+  const int dims[3] = {e.gx, e.gy, e.gz};
+  return brick_shape(dims, e.bwd, e.blines);
 }
 
-int brick_build(EllSweep& e, int mode, int n, bool forward, const std::vector<int>& dptr,
-                const std::vector<int>& dcol, const std::vector<int>& dsl,
-                const std::vector<int>& in_row, const std::vector<int>& out_row,
-                const std::vector<int>& dslot_row, double other_us, bool* built,
-                std::vector<int>* pos_of_row) {
-  (void)mode;
+template <int MODE>
+static void brick_launch(int grid, int threads, const int* gate, int want, const BrickArgs& a,
+                         DRef in, DRef out, cudaStream_t s) {
+  const BrickShape& g = a.g;
+  // the other arithmetics, and tiles of other shapes, take the general addresses
+  const bool f = arith_mode() == kFma;
+  const bool full = g.LW == 32 && g.Wp + g.Wq <= (g.d3 ? 14 : 33);
+  const size_t smem = (size_t)g.CP * g.CQ * 8 *
+                      (brick_ring(full && f, g.d3) + kStages * kGroup * brick_cols(MODE, g.d3) * g.LW);
+  auto k = g.d3 ? (!f     ? k_brick_sweep<MODE, false, false, true>
+                   : full ? k_brick_sweep<MODE, true, true, true>
+                          : k_brick_sweep<MODE, true, false, true>)
+                : (!f     ? k_brick_sweep<MODE, false, false, false>
+                   : full ? k_brick_sweep<MODE, true, true, false>
+                          : k_brick_sweep<MODE, true, false, false>);
+  k<<<grid, threads, smem, s>>>(gate, want, a, in, out);
+}
+
+template <int MODE>
+static void brick_attrs() {
+  for (auto k : {k_brick_sweep<MODE, true, true, true>, k_brick_sweep<MODE, true, false, true>,
+                 k_brick_sweep<MODE, false, false, true>, k_brick_sweep<MODE, true, true, false>,
+                 k_brick_sweep<MODE, true, false, false>, k_brick_sweep<MODE, false, false, false>})
+    cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kBrickSmemMax);
+}
+
+// The kernels' shared-memory limit, once a device (at set-up: not capturable).
+static void brick_set_attrs() {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 64 && (done.load() >> dev & 1ull)) return;
+  brick_attrs<ELL_ILU_F>();
+  brick_attrs<ELL_ILU_B>();
+  brick_attrs<ELL_ILUT_F>();
+  brick_attrs<ELL_ILUT_B>();
+  brick_attrs<ELL_ICC_F>();
+  brick_attrs<ELL_ICC_B>();
+  brick_attrs<ELL_SOR_F>();
+  brick_attrs<ELL_SOR_B>();
+  brick_attrs<ELL_SOR_B0>();
+  if (dev < 64) done |= 1ull << dev;
+}
+
+static int brick_layout(EllSweep& e, int mode, const int* dims, int lines,
+                        const std::vector<int>& slot, const std::vector<int>& dslot) {
+  ell_free(e);
+  brick_set_attrs();
+  const BrickShape g = brick_shape(dims, brick_bwd(mode), lines);
+  e.brick = true;
+  e.bwd = brick_bwd(mode);
+  e.blines = lines;
+  e.gx = dims[0];
+  e.gy = dims[1];
+  e.gz = dims[2];
+  e.BJ = g.CP * g.Wp;
+  e.BK = g.CQ * g.Wq;
+  e.n = g.n;
+  e.npos = g.ntP * g.ntQ * g.NS * g.LW;
+  e.W = 3;
+  e.bcols = brick_coefs(mode, g.d3);
+  e.nbricks = g.nbP * g.nbQ;
+  // hand-out order: wavefronts P + Q, then Q
+  std::vector<int> border;
+  border.reserve(2 * (size_t)e.nbricks);
+  for (int w = 0; w <= g.nbP + g.nbQ - 2; w++)
+    for (int Q = std::max(0, w - (g.nbP - 1)); Q <= std::min(w, g.nbQ - 1); Q++) {
+      border.push_back(w - Q);
+      border.push_back(Q);
+    }
+  GP_TRY(bup(&e.border, border));
+  GP_TRY(bup(&e.cslot, slot));
+  if (brick_has_diag(mode) && !dslot.empty()) GP_TRY(bup(&e.dslot, dslot));
+  GP_CUDA(cudaMalloc(&e.coef, (size_t)e.bcols * e.npos * sizeof(double)));
+  e.qface = (long long)(g.nbP + 1) * g.ntQ * g.Wq * g.nwp;
+  e.fsize = e.qface + (g.d3 ? (long long)(g.nbQ + 1) * g.ntP * g.Wp * g.nwp : 0);
+  GP_CUDA(cudaMalloc(&e.faces, (size_t)(2 * e.fsize) * sizeof(double) + sizeof(int)));
+  e.parity = reinterpret_cast<int*>(e.faces + 2 * e.fsize);
+  GP_TRY(brick_reset(e, 0));
+  GP_CUDA(cudaDeviceSynchronize());
+  e.ok = true;
+  return GP_OK;
+}
+
+// Both copies of the faces empty: at set-up, and after a wait ran out.
+int brick_reset(EllSweep& e, cudaStream_t s) {
+  if (!e.brick) return GP_OK;
+  GP_CUDA(cudaMemsetAsync(e.parity, 0, sizeof(int), s));
+  k_brick_clear<<<std::max(1, num_sms()), 256, 0, s>>>(2 * e.fsize, e.faces);
+  GP_CHECK_LAUNCH();
+  return GP_OK;
+}
+
+int brick_build(EllSweep& ef, EllSweep& eb, int mode_f, int mode_b, int n,
+                const std::vector<int>& fptr, const std::vector<int>& fcol,
+                const std::vector<int>& fsl, const std::vector<int>& bptr,
+                const std::vector<int>& bcol, const std::vector<int>& bsl,
+                const std::vector<int>& dslot, const std::vector<int>& perm, int nlevels,
+                bool chosen_form, bool* built) {
   *built = false;
   const BrickTuning& tu = brick_tuning();
-  if (tu.mode == 0 || n == 0) return GP_OK;
-  int nx, ny, nz, ord;
-  std::vector<int> slot;
-  if (!brick_detect(n, forward, dptr, dcol, dsl, &nx, &ny, &nz, &ord, slot)) return GP_OK;
-  // lines of a brick: at most kBrickMaxLines and the grid's ny, and at most
-  // nx (a brick's steps, nx + BJ - 1, bound the holes of its layout)
-  const int cap = std::min({kBrickMaxLines, ny, std::max(nx, 1)});
-  int BJ = std::min(tu.BJ, cap);
-  double best = 0.0;
-  if (BJ <= 0) {
-    std::vector<int> cand = {1, 2, 4, 8, 16, 32, 64, 128, ny};
-    for (int c : cand) {
-      if (c < 1 || c > cap) continue;
-      const double est = brick_model_us(nx, ny, nz, c);
-      if (!BJ || est < best) {
-        BJ = c;
-        best = est;
-      }
-    }
-    if (!BJ) return GP_OK;
-  } else {
-    best = brick_model_us(nx, ny, nz, BJ);
+  if (tu.mode == 0 || (tu.mode == 1 && chosen_form) || n < 2) return GP_OK;
+  for (int i = 0; i < (int)perm.size(); i++)
+    if (perm[i] != i) return GP_OK;  // rows and grid in natural order only
+  int df[3], db[3];
+  std::vector<int> sf, sb;
+  if (!brick_detect(n, true, fptr, fcol, fsl, df, sf) ||
+      !brick_detect(n, false, bptr, bcol, bsl, db, sb))
+    return GP_OK;
+  if (df[0] != db[0] || df[1] != db[1] || df[2] != db[2]) return GP_OK;
+  const int lines = std::max(0, tu.BJ);
+  double est = 0.0;
+  for (bool bwd : {false, true}) {
+    const BrickShape g = brick_shape(df, bwd, lines);
+    // positions (steps x lanes, idle ones included) are int32, and few lanes
+    // idle: a grid of very short lines keeps the other forms
+    const long long pos = (long long)g.ntP * g.ntQ * g.NS * g.LW;
+    const double us = brick_model_us(g);
+    if (pos > INT_MAX / 4) return GP_OK;
+    if (tu.mode == 1 &&
+        (pos > 4LL * n + 4096 || us > other_model_us(std::max(nlevels, 1))))
+      return GP_OK;
+    est += us;
   }
-  if (tu.mode == 1 && !(best < other_us)) return GP_OK;
-  const int nbJ = (ny + BJ - 1) / BJ;
-  const long long nbricks = (long long)nbJ * nz;
-  if (nbricks > INT_MAX / 2) return GP_OK;
-  // hand-out order: wavefronts J + K, then K; positions are assigned in the
-  // same order, BJ per step of each brick
-  std::vector<int> border, bbase((size_t)nbricks, 0);
-  border.reserve(2 * (size_t)nbricks);
-  long long P = 0;
-  for (long long w = 0; w <= nbJ + nz - 2; w++)
-    for (long long K = std::max(0LL, w - (nbJ - 1)); K <= std::min<long long>(w, nz - 1); K++) {
-      const int J = (int)(w - K);
-      border.push_back(J);
-      border.push_back((int)K);
-      bbase[(size_t)J + (size_t)nbJ * K] = (int)P;
-      const int bj = std::min(BJ, ny - J * BJ);
-      P += (long long)(nx + bj - 1) * BJ;
-      if (P > INT_MAX - 1) return GP_OK;  // positions are int32
-    }
-  // per-position data: coefficient slots by direction ([d][P]; -1 no term,
-  // refreshed to 0), input / output / diagonal slots; holes have no terms
-  const int W = 3;
-  std::vector<int> cnt((size_t)P, 0), cs((size_t)3 * P, -1), in((size_t)P, 0), out((size_t)P, 0),
-      ds((size_t)P, 0), pos(n);
-  bool in_ident = true, out_ident = true;
-  const long long nxny = (long long)nx * ny;
-  for (int r = 0; r < n; r++) {
-    const long long f = forward ? r : (long long)n - 1 - r;
-    const int i = (int)(f % nx), j = (int)((f / nx) % ny), k = (int)(f / nxny);
-    const int J = j / BJ, t = j % BJ;
-    const long long p = (long long)bbase[(size_t)J + (size_t)nbJ * k] + (long long)(i + t) * BJ + t;
-    pos[r] = (int)p;
-    cnt[p] = W;
-    for (int d = 0; d < 3; d++) cs[(size_t)d * P + p] = slot[(size_t)d * n + r];
-    in[p] = in_row.empty() ? r : in_row[r];
-    out[p] = out_row.empty() ? r : out_row[r];
-    in_ident = in_ident && in[p] == r;
-    out_ident = out_ident && out[p] == r;
-    if (!dslot_row.empty()) ds[p] = dslot_row[r];
-  }
-  ell_free(e);
-  e.n = (int)P;
-  e.nrows = n;
-  e.W = W;
-  GP_TRY(bup(&e.cnt, cnt));
-  GP_TRY(bup(&e.cslot, cs));
-  if (!in_ident) GP_TRY(bup(&e.in_idx, in));
-  if (!out_ident) GP_TRY(bup(&e.out_idx, out));
-  if (!dslot_row.empty()) GP_TRY(bup(&e.dslot, ds));
-  GP_TRY(bup(&e.border, border));
-  GP_TRY(bup(&e.bbase, bbase));
-  GP_CUDA(cudaMalloc(&e.coef, (size_t)W * P * sizeof(double)));
-  GP_CUDA(cudaMalloc(&e.dval, std::max<long long>(P, 1) * sizeof(double)));
-  e.brick = true;
-  e.gx = nx;
-  e.gy = ny;
-  e.gz = nz;
-  e.BJ = BJ;
-  e.BK = 1;
-  e.nbJ = nbJ;
-  e.bord = ord;
-  e.nbricks = (int)nbricks;
-  e.in_ident = in_ident;
-  e.out_ident = out_ident;
-  e.est_us = best;
-  e.bgrid = (int)std::max<long long>(1, std::min<long long>(nbricks, (long long)num_sms() * tu.ctas_per_sm));
-  if (tu.max_ctas > 0) e.bgrid = std::min(e.bgrid, tu.max_ctas);
-  e.ok = true;
-  if (pos_of_row) *pos_of_row = pos;
+  GP_TRY(brick_layout(ef, mode_f, df, lines, sf, dslot));
+  GP_TRY(brick_layout(eb, mode_b, df, lines, sb, dslot));
   if (std::getenv("GPETSC_SWEEP_VERBOSE"))
     std::fprintf(stderr,
-                 "gpetsc sweep: n=%d bricks grid %dx%dx%d lines %d bricks=%lld positions=%lld "
-                 "grid=%d est=%.0fus (other form %.0fus)\n",
-                 n, nx, ny, nz, BJ, nbricks, P, e.bgrid, best, other_us);
+                 "gpetsc sweep: n=%d grid %dx%dx%d bricks of %dx%d (forward) and %dx%d lines: "
+                 "%d and %d, est=%.0fus\n",
+                 n, df[0], df[1], df[2], ef.BJ, ef.BK, eb.BJ, eb.BK, ef.nbricks, eb.nbricks, est);
   *built = true;
   return GP_OK;
 }
 
-template <int MODE, bool FMA>
-static void brick_launch_a(const EllSweep& e, const int* gate, int want, const BrickArgs& a,
-                           DRef in, DRef out, cudaStream_t s) {
-  // compute threads (a line each), then the fetch warps: the k face 32
-  // lines a warp, and one for the j face
-  const int threads = (e.BJ + 31) / 32 * 32 + 32 * ((e.BJ + 31) / 32 + 1);
-  if (e.bord == 0)
-    k_brick_sweep<MODE, FMA, 0><<<e.bgrid, threads, 0, s>>>(gate, want, a, in, out);
-  else
-    k_brick_sweep<MODE, FMA, 1><<<e.bgrid, threads, 0, s>>>(gate, want, a, in, out);
-}
-
-template <int MODE>
-static void brick_launch(const EllSweep& e, const int* gate, int want, const BrickArgs& a,
-                         DRef in, DRef out, cudaStream_t s) {
-  if (arith_mode() == kFma)
-    brick_launch_a<MODE, true>(e, gate, want, a, in, out, s);
-  else
-    brick_launch_a<MODE, false>(e, gate, want, a, in, out, s);
+int brick_refresh(EllSweep& e, const double* src, const double* diag, const int* gate, int want,
+                  const int* stale, cudaStream_t s) {
+  if (!e.ok || !e.brick || e.n == 0) return GP_OK;
+  const int grid = std::max(1, std::min((e.npos + 255) / 256, num_sms() * 8));
+  k_brick_refresh<<<grid, 256, 0, s>>>(gate, want, shape_of(e), e.bcols, e.npos, e.cslot, e.dslot,
+                                       src, diag, e.coef, stale);
+  GP_CHECK_LAUNCH();
+  return GP_OK;
 }
 
 int brick_sweep(int mode, const EllSweep& e, const int* gate, int want, DRef in, DRef out,
-                double* val, const double* fval, double* aux, const double* auxin,
-                const double* idiag, double omega, int use_t, int write_out, unsigned* tickets,
-                DevErr* err, cudaStream_t s) {
+                const double* tin, const double* tin2, double* tout, double* tout2, double omega,
+                int write_out, unsigned* tickets, DevErr* err, cudaStream_t s) {
   if (e.n == 0) return GP_OK;
   BrickArgs a;
-  a.nrows = e.nrows;
-  a.npos = e.n;
-  a.nx = e.gx;
-  a.ny = e.gy;
-  a.nz = e.gz;
-  a.BJ = e.BJ;
-  a.nbJ = e.nbJ;
+  a.g = shape_of(e);
   a.nbricks = e.nbricks;
-  a.in_ident = e.in_ident ? 1 : 0;
-  a.out_ident = e.out_ident ? 1 : 0;
   a.border = e.border;
-  a.bbase = e.bbase;
   a.coef = e.coef;
-  a.in_idx = e.in_idx;
-  a.out_idx = e.out_idx;
-  a.dval = e.dval;
-  a.val = val;
-  a.fval = fval;
-  a.aux = aux;
-  a.auxin = auxin;
-  a.idiag = idiag;
+  a.faces = e.faces;
+  a.fsize = e.fsize;
+  a.qface = e.qface;
+  a.parity = e.parity;
+  a.tin = tin;
+  a.tin2 = tin2;
+  a.tout = tout;
+  a.tout2 = tout2;
   a.om1 = 1.0 - omega;
-  a.use_t = use_t;
   a.write_out = write_out;
-  a.fetch_sleep_ns = brick_tuning().fetch_sleep_ns;
   a.tickets = tickets;
   a.err = err;
+  // kBrickPoll lanes for every face line of a brick; none where one brick is
+  // the grid
+  const int cols = a.g.CQ * a.g.Wq + (a.g.d3 ? a.g.CP * a.g.Wp : 0);
+  a.poll = kBrickPoll;
+  while (a.poll > 1 && cols * a.poll > 32 * kBrickFetchMax) a.poll /= 2;
+  const int nf = e.nbricks > 1 ? (cols * a.poll + 31) / 32 : 0;
+  const int threads = 32 * (a.g.CP * a.g.CQ + nf);
+  int grid = std::min(e.nbricks, num_sms() * 2);
+  if (brick_tuning().max_ctas > 0) grid = std::min(grid, brick_tuning().max_ctas);
+#define BRICK_LAUNCH(M) \
+  case M: brick_launch<M>(grid, threads, gate, want, a, in, out, s); break;
   switch (mode) {
-    case ELL_ILU_F: brick_launch<ELL_ILU_F>(e, gate, want, a, in, out, s); break;
-    case ELL_ILU_B: brick_launch<ELL_ILU_B>(e, gate, want, a, in, out, s); break;
-    case ELL_ICC_F: brick_launch<ELL_ICC_F>(e, gate, want, a, in, out, s); break;
-    case ELL_ICC_B: brick_launch<ELL_ICC_B>(e, gate, want, a, in, out, s); break;
-    case ELL_SOR_F: brick_launch<ELL_SOR_F>(e, gate, want, a, in, out, s); break;
-    case ELL_SOR_B: brick_launch<ELL_SOR_B>(e, gate, want, a, in, out, s); break;
+    BRICK_LAUNCH(ELL_ILU_F)
+    BRICK_LAUNCH(ELL_ILU_B)
+    BRICK_LAUNCH(ELL_ILUT_F)
+    BRICK_LAUNCH(ELL_ILUT_B)
+    BRICK_LAUNCH(ELL_ICC_F)
+    BRICK_LAUNCH(ELL_ICC_B)
+    BRICK_LAUNCH(ELL_SOR_F)
+    BRICK_LAUNCH(ELL_SOR_B)
+    BRICK_LAUNCH(ELL_SOR_B0)
   }
+#undef BRICK_LAUNCH
   GP_CHECK_LAUNCH();
   return GP_OK;
 }

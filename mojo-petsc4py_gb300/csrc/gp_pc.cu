@@ -177,8 +177,7 @@ __global__ void k_ell_refresh_g(const int* gate, int want, int n, const int* __r
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const int c = cnt[p];
     for (int e = 0; e < c; e++) {
-      const int cs = cslot[(size_t)e * n + p];
-      coef[(size_t)e * n + p] = cs >= 0 ? src[cs] : 0.0;  // < 0: no term (brick form)
+      coef[(size_t)e * n + p] = src[cslot[(size_t)e * n + p]];
     }
   }
 }
@@ -574,6 +573,7 @@ int pc_check(Pc* pc, cudaStream_t s) {
   GP_CUDA(cudaStreamSynchronize(s));
   if (h.code == 0) return GP_OK;
   GP_CUDA(cudaMemsetAsync(pc->err, 0, sizeof(DevErr), s));
+  for (EllSweep* e : {&pc->ef, &pc->eb, &pc->etf, &pc->etb}) GP_TRY(brick_reset(*e, s));
   GP_CUDA(cudaStreamSynchronize(s));
   set_error("preconditioner sweep wait ran out of budget (site " + std::to_string(h.where) +
             ")");
@@ -649,16 +649,21 @@ static int setup_sor(Pc* pc, cudaStream_t s) {
   GP_TRY(plan(pc->fwd, n, lp, lc, true, s, &of));
   GP_TRY(plan(pc->bwd, n, up, uc, false, s, &ob));
   setup_mark("levels");
-  GP_TRY(ell_build(pc->ef, ELL_SOR_F, n, true, of, lp, lc, ls, none, none, none, &fpos,
-                   pc->fwd.nlevels));
-  setup_mark("fwd-layout");
-  GP_TRY(ell_build(pc->eb, ELL_SOR_B, n, false, ob, up, uc, us, fpos, none, none, nullptr,
-                   pc->bwd.nlevels));
-  setup_mark("bwd-layout");
-  pc->vlen = std::max({n, pc->ef.n, pc->eb.n});
-  GP_TRY(dalloc(&pc->t, pc->vlen));
-  GP_TRY(dalloc(&pc->yf, pc->vlen));
-  GP_TRY(dalloc(&pc->yb, pc->vlen));
+  bool bricks = false;
+  GP_TRY(brick_build(pc->ef, pc->eb, ELL_SOR_F, ELL_SOR_B, n, lp, lc, ls, up, uc, us, none, none,
+                     pc->fwd.nlevels, sweep_form_chosen(), &bricks));
+  setup_mark("brick-layout");
+  if (!bricks) {
+    GP_TRY(ell_build(pc->ef, ELL_SOR_F, n, true, of, lp, lc, ls, none, none, none, &fpos,
+                     pc->fwd.nlevels));
+    setup_mark("fwd-layout");
+    GP_TRY(ell_build(pc->eb, ELL_SOR_B, n, false, ob, up, uc, us, fpos, none, none, nullptr,
+                     pc->bwd.nlevels));
+    setup_mark("bwd-layout");
+    GP_TRY(dalloc(&pc->yb, n));
+  }
+  GP_TRY(dalloc(&pc->t, n));
+  GP_TRY(dalloc(&pc->yf, n));
   GP_CUDA(cudaMalloc(&pc->sor_stale, sizeof(int)));
   GP_CUDA(cudaMemsetAsync(pc->sor_stale, 1, sizeof(int), s));  // nonzero: recompute
   pc->sor_vver = A->vver;
@@ -715,12 +720,19 @@ static int ilu_prepare(Pc* pc, const std::vector<int>& perm_c, cudaStream_t s) {
   GP_TRY(plan(pc->fwd, n, lp, lc, true, s, &of));
   GP_TRY(plan(pc->bwd, n, up, uc, false, s, &ob));
   setup_mark("levels");
-  GP_TRY(ell_build(pc->ef, ELL_ILU_F, n, true, of, lp, lc, ls, P.r, none, none, &fpos,
-                   pc->fwd.nlevels));
-  setup_mark("fwd-layout");
-  GP_TRY(ell_build(pc->eb, ELL_ILU_B, n, false, ob, up, uc, us, fpos, perm_c, dsl, nullptr,
-                   pc->bwd.nlevels));
-  setup_mark("bwd-layout");
+  bool bricks = false;
+  if (P.r == perm_c)
+    GP_TRY(brick_build(pc->ef, pc->eb, ELL_ILU_F, ELL_ILU_B, n, lp, lc, ls, up, uc, us, dsl, P.r,
+                       pc->fwd.nlevels, sweep_form_chosen(), &bricks));
+  setup_mark("brick-layout");
+  if (!bricks) {
+    GP_TRY(ell_build(pc->ef, ELL_ILU_F, n, true, of, lp, lc, ls, P.r, none, none, &fpos,
+                     pc->fwd.nlevels));
+    setup_mark("fwd-layout");
+    GP_TRY(ell_build(pc->eb, ELL_ILU_B, n, false, ob, up, uc, us, fpos, perm_c, dsl, nullptr,
+                     pc->bwd.nlevels));
+    setup_mark("bwd-layout");
+  }
   // the numeric phase's update lists (the searches of the elimination, once);
   // kept to the end of the function: the copies below are asynchronous
   std::vector<int> uptr(P.bi[n] + 1, 0), udst, usrc;
@@ -803,9 +815,8 @@ static int ilu_prepare(Pc* pc, const std::vector<int>& perm_c, cudaStream_t s) {
   GP_TRY(dalloc(&pc->ba, std::max(P.nnz, 1)));
   GP_CUDA(cudaMalloc(&pc->done, std::max(n, 1) * sizeof(int)));
   GP_CUDA(cudaMemsetAsync(pc->done, 0, std::max(n, 1) * sizeof(int), s));
-  pc->vlen = std::max({n, pc->ef.n, pc->eb.n});
-  GP_TRY(dalloc(&pc->yf, pc->vlen));
-  GP_TRY(dalloc(&pc->yb, pc->vlen));
+  GP_TRY(dalloc(&pc->yf, n));
+  if (!bricks) GP_TRY(dalloc(&pc->yb, n));
   GP_CUDA(cudaStreamSynchronize(s));  // host vectors above go out of scope
   return GP_OK;
 }
@@ -925,12 +936,18 @@ static int icc_prepare(Pc* pc, const std::vector<int>& perm_c, cudaStream_t s) {
   GP_TRY(plan(pc->fwd, n, tptr, trow_deps, true, s, &of));
   GP_TRY(plan(pc->bwd, n, up, uc, false, s, &ob));
   setup_mark("levels");
-  GP_TRY(ell_build(pc->ef, ELL_ICC_F, n, true, of, tptr, trow_deps, tsl, perm_c, none, dsl, &fpos,
-                   pc->fwd.nlevels));
-  setup_mark("fwd-layout");
-  GP_TRY(ell_build(pc->eb, ELL_ICC_B, n, false, ob, up, uc, us, fpos, perm_c, none, nullptr,
-                   pc->bwd.nlevels));
-  setup_mark("bwd-layout");
+  bool bricks = false;
+  GP_TRY(brick_build(pc->ef, pc->eb, ELL_ICC_F, ELL_ICC_B, n, tptr, trow_deps, tsl, up, uc, us, dsl,
+                     perm_c, pc->fwd.nlevels, sweep_form_chosen(), &bricks));
+  setup_mark("brick-layout");
+  if (!bricks) {
+    GP_TRY(ell_build(pc->ef, ELL_ICC_F, n, true, of, tptr, trow_deps, tsl, perm_c, none, dsl,
+                     &fpos, pc->fwd.nlevels));
+    setup_mark("fwd-layout");
+    GP_TRY(ell_build(pc->eb, ELL_ICC_B, n, false, ob, up, uc, us, fpos, perm_c, none, nullptr,
+                     pc->bwd.nlevels));
+    setup_mark("bwd-layout");
+  }
   GP_TRY(upload(&pc->bi, P.bi, s));
   GP_TRY(upload(&pc->bj, P.bj, s));
   GP_TRY(upload(&pc->bdiag, P.bdiag, s));
@@ -947,10 +964,11 @@ static int icc_prepare(Pc* pc, const std::vector<int>& perm_c, cudaStream_t s) {
   GP_TRY(dalloc(&pc->ba_orig, std::max(P.nnz, 1)));
   GP_CUDA(cudaMalloc(&pc->done, std::max(n, 1) * sizeof(int)));
   GP_CUDA(cudaMemsetAsync(pc->done, 0, std::max(n, 1) * sizeof(int), s));
-  pc->vlen = std::max({n, pc->ef.n, pc->eb.n});
-  GP_TRY(dalloc(&pc->yf, pc->vlen));
-  GP_TRY(dalloc(&pc->yb, pc->vlen));
-  GP_TRY(dalloc(&pc->ys, pc->vlen));
+  if (!bricks) {
+    GP_TRY(dalloc(&pc->yf, n));
+    GP_TRY(dalloc(&pc->yb, n));
+  }
+  GP_TRY(dalloc(&pc->ys, n));
   GP_CUDA(cudaStreamSynchronize(s));
   return GP_OK;
 }
@@ -1148,7 +1166,19 @@ int pc_apply(Pc* pc, DRef x, DRef y, cudaStream_t s, const int* gate, int want) 
       k_sor_diag<<<(n + 255) / 256, 256, 0, s>>>(n, pc->opt.omega, pc->opt.fshift, A->diagpos,
                                                   A->val, pc->idiag, pc->mdiag, gate, want,
                                                   pc->sor_stale);
-      k_fill_pending<<<grid_for(pc->vlen), 256, 0, s>>>(gate, want, pc->vlen, pc->yf, pc->yb);
+      if (pc->ef.brick) {
+        GP_TRY(brick_refresh(pc->ef, A->val, pc->idiag, gate, want, pc->sor_stale, s));
+        GP_TRY(brick_refresh(pc->eb, A->val, pc->idiag, gate, want, pc->sor_stale, s));
+        k_clear_word<<<1, 1, 0, s>>>(gate, want, pc->sor_stale);
+        if (fw)
+          GP_TRY(brick_sweep(ELL_SOR_F, pc->ef, gate, want, x, y, nullptr, nullptr, pc->yf, pc->t,
+                             pc->opt.omega, bw ? 0 : 1, tk0, pc->err, s));
+        if (bw)
+          GP_TRY(brick_sweep(fw ? ELL_SOR_B : ELL_SOR_B0, pc->eb, gate, want, x, y, pc->yf, pc->t, nullptr, nullptr,
+                             pc->opt.omega, 1, tk1, pc->err, s));
+        break;
+      }
+      k_fill_pending<<<g, 256, 0, s>>>(gate, want, n, pc->yf, pc->yb);
       if (pc->ef.ok && pc->eb.ok) {
         if (!pc->ef.tiled)
           k_ell_refresh_g<<<g, 256, 0, s>>>(gate, want, pc->ef.n, pc->ef.cnt, pc->ef.cslot,
@@ -1178,7 +1208,14 @@ int pc_apply(Pc* pc, DRef x, DRef y, cudaStream_t s, const int* gate, int want) 
       break;
     }
     case PC_ILU:
-      k_fill_pending<<<grid_for(pc->vlen), 256, 0, s>>>(gate, want, pc->vlen, pc->yf, pc->yb);
+      if (pc->ef.brick) {
+        GP_TRY(brick_sweep(ELL_ILU_F, pc->ef, gate, want, x, y, nullptr, nullptr, pc->yf, nullptr,
+                           0.0, 0, tk0, pc->err, s));
+        GP_TRY(brick_sweep(ELL_ILU_B, pc->eb, gate, want, x, y, pc->yf, nullptr, nullptr, nullptr,
+                           0.0, 0, tk1, pc->err, s));
+        break;
+      }
+      k_fill_pending<<<g, 256, 0, s>>>(gate, want, n, pc->yf, pc->yb);
       if (pc->ef.ok && pc->eb.ok) {
         GP_TRY(ell_sweep(ELL_ILU_F, pc->ef, gate, want, x, y, pc->yf, nullptr, nullptr, nullptr,
                          nullptr, 0.0, 0, 0, tk0, pc->err, pc->ba, s));
@@ -1192,7 +1229,14 @@ int pc_apply(Pc* pc, DRef x, DRef y, cudaStream_t s, const int* gate, int want) 
                                            pc->bdiag, pc->perm_c, pc->yf, pc->yb, y, pc->err);
       break;
     case PC_ICC:
-      k_fill_pending<<<grid_for(pc->vlen), 256, 0, s>>>(gate, want, pc->vlen, pc->yf, pc->yb);
+      if (pc->ef.brick) {
+        GP_TRY(brick_sweep(ELL_ICC_F, pc->ef, gate, want, x, y, nullptr, nullptr, pc->ys, nullptr,
+                           0.0, 0, tk0, pc->err, s));
+        GP_TRY(brick_sweep(ELL_ICC_B, pc->eb, gate, want, x, y, pc->ys, nullptr, nullptr, nullptr,
+                           0.0, 0, tk1, pc->err, s));
+        break;
+      }
+      k_fill_pending<<<g, 256, 0, s>>>(gate, want, n, pc->yf, pc->yb);
       if (pc->ef.ok && pc->eb.ok) {
         GP_TRY(ell_sweep(ELL_ICC_F, pc->ef, gate, want, x, y, pc->yf, nullptr, pc->ys, nullptr,
                          nullptr, 0.0, 0, 0, tk0, pc->err, pc->ba, s));
@@ -1271,8 +1315,15 @@ int pc_transpose_prepare(Pc* pc, cudaStream_t s) {
   int nlev = 0;
   level_order(n, up, uc, true, of, &nlev);
   level_order(n, lp, lc, false, ob, &nlev);
-  GP_TRY(ell_build_chunked(pc->etf, ELL_ILU_B, n, true, of, up, uc, us, perm_c, none, dsl, &fpos));
-  GP_TRY(ell_build_chunked(pc->etb, ELL_ILU_F, n, false, ob, lp, lc, ls, fpos, P.r, none, nullptr));
+  bool bricks = false;
+  if (P.r == perm_c)
+    GP_TRY(brick_build(pc->etf, pc->etb, ELL_ILUT_F, ELL_ILUT_B, n, up, uc, us, lp, lc, ls, dsl,
+                       perm_c, nlev, sweep_form_chosen(), &bricks));
+  if (!bricks) {
+    GP_TRY(ell_build(pc->etf, ELL_ILU_B, n, true, of, up, uc, us, perm_c, none, dsl, &fpos));
+    GP_TRY(ell_build(pc->etb, ELL_ILU_F, n, false, ob, lp, lc, ls, fpos, P.r, none, nullptr));
+    if (!pc->yb) GP_TRY(dalloc(&pc->yb, n));
+  }
   if (!pc->etf.ok || !pc->etb.ok) {
     ell_free(pc->etf);
     ell_free(pc->etb);
@@ -1302,6 +1353,12 @@ int pc_apply_transpose(Pc* pc, DRef x, DRef y, cudaStream_t s, const int* gate, 
   if (!pc->trans_ready) {
     set_error("transposed apply used before pc_transpose_prepare");
     return GP_ERR_NOT_SETUP;
+  }
+  if (pc->etf.brick) {
+    GP_TRY(brick_sweep(ELL_ILUT_F, pc->etf, gate, want, x, y, nullptr, nullptr, pc->yf, nullptr,
+                       0.0, 0, pc->tickets, pc->err, s));
+    return brick_sweep(ELL_ILUT_B, pc->etb, gate, want, x, y, pc->yf, nullptr, nullptr, nullptr,
+                       0.0, 0, pc->tickets + 2, pc->err, s);
   }
   k_fill_pending<<<grid_for(n), 256, 0, s>>>(gate, want, n, pc->yf, pc->yb);
   // U^T z = x[c]: input gathered from x by the sweep's in_idx, no output

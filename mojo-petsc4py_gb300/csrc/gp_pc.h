@@ -37,7 +37,13 @@ struct SweepPlan {
 // (gp_sweep.cu); `ok` is false when some row has more than kEllMaxW
 // dependencies, and the CSR sweep kernels are used instead.
 constexpr int kEllMaxW = 16;
-enum EllMode : int { ELL_ILU_F, ELL_ILU_B, ELL_ICC_F, ELL_ICC_B, ELL_SOR_F, ELL_SOR_B };
+enum EllMode : int {
+  ELL_ILU_F, ELL_ILU_B, ELL_ICC_F, ELL_ICC_B, ELL_SOR_F, ELL_SOR_B,
+  // brick form only: the two sweeps of the transposed ILU apply (U^T with the
+  // diagonal, then L^T; the other forms run them as ILU_B and ILU_F) and SOR's
+  // backward half without a forward one
+  ELL_ILUT_F, ELL_ILUT_B, ELL_SOR_B0
+};
 struct EllSweep {
   int n = 0, W = 0;
   bool ok = false;
@@ -65,31 +71,43 @@ struct EllSweep {
   double est_us = 0.0;            // simulated duration of one tiled sweep
   int rows_per_chunk = 0;         // chunk size of the tiled layout
   // Brick form (gp_brick.cu, k_brick_sweep): the sweep's dependencies are the
-  // unit steps of a grid gx x gy x gz; CTAs take bricks of BJ grid lines of
-  // one plane (BK = 1) and each thread walks one line.  `n` counts positions,
-  // step-major within each brick with holes (nrows rows); the per-position
-  // arrays are cslot / coef as [direction][n], in_idx, out_idx (absent when
-  // the identity), dslot / dval, and values are indexed by position.
-  bool brick = false;
-  int gx = 0, gy = 0, gz = 0, BJ = 0, BK = 0, nbJ = 0, nbricks = 0, bgrid = 0, nrows = 0;
-  int bord = 0;            // fold order of a row's terms: 0 k, j, i; 1 i, j, k
-  bool in_ident = false, out_ident = false;
-  int* border = nullptr;   // [2 * nbricks]: (J, K) of each brick in hand-out order
-  int* bbase = nullptr;    // [nbJ * gz]: first position of brick (J, K) at J + nbJ K
+  // unit steps of a grid gx x gy x gz; a CTA takes BJ x BK grid lines, a tile
+  // of them a warp.  cslot is [direction][row], dslot by row, coef
+  // [tile][step][bcols][lane] (npos steps x lanes, idle ones included).  The
+  // two sweeps of a PC have it together.
+  bool brick = false, bwd = false;
+  int gx = 0, gy = 0, gz = 0, BJ = 0, BK = 0, nbricks = 0, npos = 0, bcols = 0;
+  int blines = 0;             // forced lines of a brick (0: chosen)
+  int* border = nullptr;      // [2 * nbricks]: place of each brick in hand-out order
+  double* faces = nullptr;    // two copies of the bricks' face values, used in turn
+  long long fsize = 0, qface = 0;
+  int* parity = nullptr;      // which copy the next sweep uses (in faces' block)
 };
 void ell_free(EllSweep& e);
-// Brick layout of a sweep when its dependencies have the grid structure and
-// (unless forced) the model puts it below `other_us`; *built says whether.
-// pos_of_row: each row's position in the brick layout.
-int brick_build(EllSweep& e, int mode, int n, bool forward, const std::vector<int>& dptr,
-                const std::vector<int>& dcol, const std::vector<int>& dsl,
-                const std::vector<int>& in_row, const std::vector<int>& out_row,
-                const std::vector<int>& dslot_row, double other_us, bool* built,
-                std::vector<int>* pos_of_row);
+// Brick layout of a PC's two sweeps (mode_f, mode_b their EllModes) when the
+// dependencies of both have the grid structure in natural order (`perm` the
+// identity, or empty) and the model puts it below the other forms; *built says
+// whether.  chosen_form: the caller asked for a level-ordered or chunked form,
+// which only a forced brick form (mode 2) overrides.  dslot: each row's
+// diagonal slot, for the modes that take it from the factor.
+int brick_build(EllSweep& ef, EllSweep& eb, int mode_f, int mode_b, int n,
+                const std::vector<int>& fptr, const std::vector<int>& fcol,
+                const std::vector<int>& fsl, const std::vector<int>& bptr,
+                const std::vector<int>& bcol, const std::vector<int>& bsl,
+                const std::vector<int>& dslot, const std::vector<int>& perm, int nlevels,
+                bool chosen_form, bool* built);
+// Coefficients (and diagonal: from src, or diag by row) of a brick sweep from
+// the current values; with `stale`, only while that word is set.
+int brick_refresh(EllSweep& e, const double* src, const double* diag, const int* gate, int want,
+                  const int* stale, cudaStream_t s);
+int brick_reset(EllSweep& e, cudaStream_t s);
+// One brick sweep.  First sweeps read `in` and leave their values (tout) and
+// SOR's checkpoint (tout2) by row, where second sweeps read them (tin, tin2).
 int brick_sweep(int mode, const EllSweep& e, const int* gate, int want, DRef in, DRef out,
-                double* val, const double* fval, double* aux, const double* auxin,
-                const double* idiag, double omega, int use_t, int write_out, unsigned* tickets,
-                DevErr* err, cudaStream_t s);
+                const double* tin, const double* tin2, double* tout, double* tout2, double omega,
+                int write_out, unsigned* tickets, DevErr* err, cudaStream_t s);
+// Whether the level-ordered or a chunked form was asked for (gp_set_sweep_form).
+bool sweep_form_chosen();
 // Brick form of later set-ups: mode 0 never, 1 where modelled faster, 2
 // wherever the structure allows; lines > 0 forces the lines of a brick;
 // max_ctas > 0 caps the persistent grid.
@@ -104,19 +122,6 @@ int ell_build(EllSweep& e, int mode, int n, bool forward, const std::vector<int>
               const std::vector<int>& out_row, const std::vector<int>& dslot_row,
               std::vector<int>* pos_of_row, int nlevels = 0);
 int ell_refresh(EllSweep& e, const double* src, cudaStream_t s);
-// ell_build choosing between the level-ordered and the chunked form only (no
-// brick layout: its kernel reads the reference's inputs of each mode only).
-int ell_build_chunked(EllSweep& e, int mode, int n, bool forward, const std::vector<int>& order,
-                      const std::vector<int>& dptr, const std::vector<int>& dcol,
-                      const std::vector<int>& dsl, const std::vector<int>& in_row,
-                      const std::vector<int>& out_row, const std::vector<int>& dslot_row,
-                      std::vector<int>* pos_of_row);
-// ell_build in the level-ordered form only (no chunked or brick layout).
-int ell_build_levels(EllSweep& e, int mode, int n, bool forward, const std::vector<int>& order,
-                     const std::vector<int>& dptr, const std::vector<int>& dcol,
-                     const std::vector<int>& dsl, const std::vector<int>& in_row,
-                     const std::vector<int>& out_row, const std::vector<int>& dslot_row,
-                     std::vector<int>* pos_of_row);
 int sweep_wait_probe(int budget, int set, cudaStream_t s);
 // Sweep form of later set-ups (gp_set_sweep_form).
 void set_sweep_form(int tiles, int tile_rows);
@@ -141,9 +146,6 @@ struct Pc {
   PcOptions opt;
   Csr* A = nullptr;  // operator the PC was set up from (not owned)
   int n = 0;
-  // entries of the sweeps' value arrays yf, yb, ys, t: the rows, or more
-  // where a sweep's layout has holes (the brick form)
-  int vlen = 0;
   int device = -1;
   bool ready = false;
   int epoch = 0;

@@ -121,6 +121,8 @@ void set_sweep_form(int tiles, int tile_rows) {
   sweep_tuning_mut().tile_rows = std::max(0, std::min(8192, tile_rows));
 }
 
+bool sweep_form_chosen() { return !sweep_tuning().tiles || sweep_tuning().tile_rows > 0; }
+
 template <int MODE, int WMAX, bool FMA>
 __global__ void __launch_bounds__(kEllBlock) k_ell_sweep(const int* gate, int want, EllArgs a,
                                                          DRef inr, DRef outr) {
@@ -574,7 +576,7 @@ __global__ void k_ell_refresh(int n, int W, const int* __restrict__ cnt,
     const int c = cnt[p];
     for (int e = 0; e < c; e++) {
       const int cs = cslot[(size_t)e * n + p];
-      coef[(size_t)e * n + p] = cs >= 0 ? src[cs] : 0.0;  // < 0: no term (brick form)
+      coef[(size_t)e * n + p] = src[cs];
     }
     if (dslot) dval[p] = src[dslot[p]];
   }
@@ -590,7 +592,7 @@ static int up(T** d, const std::vector<T>& h) {
 
 void ell_free(EllSweep& e) {
   void* ptrs[] = {e.cnt,  e.dep,   e.cslot, e.coef,     e.in_idx, e.out_idx, e.dslot,
-                  e.dval, e.rowof, e.blob,  e.blob_off, e.cstart, e.border, e.bbase};
+                  e.dval, e.rowof, e.blob,  e.blob_off, e.cstart, e.border, e.faces};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   e = EllSweep();
@@ -923,7 +925,7 @@ static int ell_build_impl(EllSweep& e, int mode, int n, bool forward,
                           const std::vector<int>& dsl, const std::vector<int>& in_row,
                           const std::vector<int>& out_row, const std::vector<int>& dslot_row,
                           std::vector<int>* pos_of_row, bool allow_tiles,
-                          bool allow_bricks = true, int nlevels = 0) {
+                          int nlevels = 0) {
   ell_free(e);
   int W = 0;
   for (int i = 0; i < n; i++) W = std::max(W, dptr[i + 1] - dptr[i]);
@@ -938,18 +940,6 @@ static int ell_build_impl(EllSweep& e, int mode, int n, bool forward,
     if (!nlev) nlev = sweep_levels(n, dptr, dcol, forward);
     tiled = tile_choose(mode, n, W, dptr, dcol, forward, nlev, tu, tp, &considered);
     setup_mark("chunk-model");
-  }
-  if (allow_tiles && allow_bricks && n > 0) {
-    // the brick form, where the sweep is a grid in natural order and the
-    // model puts it below the better of the other two forms
-    if (!nlev) nlev = sweep_levels(n, dptr, dcol, forward);
-    double other = TileModel().ell_level * nlev;
-    if (tiled) other = std::min(other, tp.est_us);
-    bool built = false;
-    GP_TRY(brick_build(e, mode, n, forward, dptr, dcol, dsl, in_row, out_row, dslot_row, other,
-                       &built, pos_of_row));
-    setup_mark("brick-check");
-    if (built) return GP_OK;
   }
   const std::vector<int>& order = tiled ? tp.order : order_in;
   std::vector<int> pos(n);
@@ -1021,25 +1011,7 @@ int ell_build(EllSweep& e, int mode, int n, bool forward, const std::vector<int>
               const std::vector<int>& out_row, const std::vector<int>& dslot_row,
               std::vector<int>* pos_of_row, int nlevels) {
   return ell_build_impl(e, mode, n, forward, order, dptr, dcol, dsl, in_row, out_row,
-                        dslot_row, pos_of_row, true, true, nlevels);
-}
-
-int ell_build_chunked(EllSweep& e, int mode, int n, bool forward, const std::vector<int>& order,
-                      const std::vector<int>& dptr, const std::vector<int>& dcol,
-                      const std::vector<int>& dsl, const std::vector<int>& in_row,
-                      const std::vector<int>& out_row, const std::vector<int>& dslot_row,
-                      std::vector<int>* pos_of_row) {
-  return ell_build_impl(e, mode, n, forward, order, dptr, dcol, dsl, in_row, out_row,
-                        dslot_row, pos_of_row, true, false);
-}
-
-int ell_build_levels(EllSweep& e, int mode, int n, bool forward, const std::vector<int>& order,
-                     const std::vector<int>& dptr, const std::vector<int>& dcol,
-                     const std::vector<int>& dsl, const std::vector<int>& in_row,
-                     const std::vector<int>& out_row, const std::vector<int>& dslot_row,
-                     std::vector<int>* pos_of_row) {
-  return ell_build_impl(e, mode, n, forward, order, dptr, dcol, dsl, in_row, out_row,
-                        dslot_row, pos_of_row, false);
+                        dslot_row, pos_of_row, true, nlevels);
 }
 
 // Run the wait once on a pending flag (set = 0) or a ready one (set = 1) and
@@ -1083,6 +1055,7 @@ int sweep_wait_probe(int budget, int set, cudaStream_t s) {
 
 int ell_refresh(EllSweep& e, const double* src, cudaStream_t s) {
   if (!e.ok || e.tiled || e.n == 0) return GP_OK;  // the tiled form gathers at each sweep
+  if (e.brick) return brick_refresh(e, src, nullptr, nullptr, 0, nullptr, s);
   k_ell_refresh<<<std::max(1, std::min((e.n + 255) / 256, num_sms() * 8)), 256, 0, s>>>(
       e.n, e.W, e.cnt, e.cslot, src, e.coef, e.dslot, e.dval);
   GP_CHECK_LAUNCH();
@@ -1176,9 +1149,6 @@ int ell_sweep(int mode, const EllSweep& e, const int* gate, int want, DRef in, D
               const double* idiag, double omega, int use_t, int write_out, unsigned* tickets,
               DevErr* err, const double* coefsrc, cudaStream_t s) {
   if (e.n == 0) return GP_OK;
-  if (e.brick)
-    return brick_sweep(mode, e, gate, want, in, out, val, fval, aux, auxin, idiag, omega, use_t,
-                       write_out, tickets, err, s);
   EllArgs a;
   a.n = e.n;
   a.cnt = e.cnt;
