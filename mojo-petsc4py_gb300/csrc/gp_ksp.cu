@@ -171,6 +171,25 @@ __global__ void k_waxpy_d(const int* gate, int want, int n, DRef wr, const doubl
         xr.get(), yr.get());
 }
 
+// x / d, correctly rounded, for many x and one d > 0: `r` is 1 / d rounded to
+// nearest.  Two corrections of the quotient x r by its exact remainder: the
+// first leaves it within an ulp of x / d, and from there the second rounds
+// correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Five FP64 instructions; a division by itself
+// costs about twice that, and FP64 instructions are what a normalisation is
+// bound by.  Outside the range where no step can round off or overflow
+// (plain_range) the division itself.
+__device__ __forceinline__ bool plain_range(double v) {
+  const unsigned e = (unsigned)__double2hiint(v) >> 20 & 0x7ffu;
+  return e - 523u < 1000u;  // 2^-500 <= |v| < 2^500
+}
+__device__ __forceinline__ double div_by(double x, double d, double r, bool d_plain) {
+  if (!d_plain || !plain_range(x)) return div_(x, d);
+  double q = mul(x, r);
+  q = __fma_rn(__fma_rn(-q, d, x), r, q);
+  return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
 // x = x * (*a)   (VecScale)  or  x = x / (*a) when *a > 0 (VecNormalize)
 template <bool DIVIDE>
 __global__ void k_scale_d(const int* gate, int want, int n, DRef xr, const double* a) {
@@ -179,7 +198,9 @@ __global__ void k_scale_d(const int* gate, int want, int n, DRef xr, const doubl
   const double al = *a;
   if (DIVIDE) {
     if (!(al > 0.0)) return;
-    ew<1>(n, x, [=](double xv, double, double) { return div_(xv, al); }, x);
+    const double r = div_(1.0, al);
+    const bool plain = plain_range(al);
+    ew<1>(n, x, [=](double xv, double, double) { return div_by(xv, al, r, plain); }, x);
   } else {
     ew<1>(n, x, [=](double xv, double, double) { return mul(xv, al); }, x);
   }
@@ -246,29 +267,59 @@ __global__ void __launch_bounds__(kRedBlock) k_dred(const int* gate, int want, i
 }
 
 // One batch of the multi-dot: v[q] += sum_i x_i basis_q,i for q < JN, over
-// the grid-stride elements of this thread.
+// the grid-stride elements of this thread in ascending order, the loads of two
+// elements in flight together.
 template <bool FMA, int JN>
 __device__ __forceinline__ void mdot_batch(int n, const double* __restrict__ x,
                                            const double* __restrict__ basis, double (&v)[8]) {
-  GRID_LOOP(i, n) {
-    const double a = x[i];
+  constexpr int U = 2;
+  double a[U], bv[U][JN];
+  grid_batched<U>(
+      n,
+      [&](int u, unsigned i) {
+        a[u] = x[i];
 #pragma unroll
-    for (int q = 0; q < JN; q++) v[q] = madd<FMA>(a, basis[(size_t)q * n + i], v[q]);
-  }
+        for (int q = 0; q < JN; q++) bv[u][q] = basis[(size_t)q * n + i];
+      },
+      [&](int u, unsigned) {
+#pragma unroll
+        for (int q = 0; q < JN; q++) v[q] = madd<FMA>(a[u], bv[u][q], v[q]);
+      });
+}
+
+constexpr int kMaxBasis = 64;
+
+// ||h||, for the refinement test of KSP_GMRES_CGS_REFINE_IFNEEDED.
+__device__ __forceinline__ void cgs_norm(KspState* st, const double* lhh, int k) {
+  double hnrm = 0.0;
+  for (int j = 0; j < k; j++) hnrm = add(hnrm, mul(lhh[j], lhh[j]));
+  st->red[1] = __dsqrt_rn(hnrm);
+}
+
+// The Hessenberg column after a Gram-Schmidt pass: projection j, negated in
+// lhh, and added to the column (from zero in the first pass).
+__device__ __forceinline__ void cgs_store(const KspState* st, double* hs, double* lhh, int j,
+                                          double d, bool first) {
+  const int it = st->it, m = st->m;
+  double* hh = hs + it * (m + 2) + j;
+  double* hes = hs + (m + 2) * (m + 1) + it * (m + 1) + j;
+  const double l = -d;
+  lhh[j] = l;
+  *hh = sub(first ? 0.0 : *hh, l);
+  *hes = sub(first ? 0.0 : *hes, l);
 }
 
 // VecMDot of x against `*count` contiguous basis vectors (ld = n): one pass
-// over x and the basis, per-block partial sums for every vector, last block
-// folds the partials.  Used by classical Gram-Schmidt.
-constexpr int kMaxBasis = 64;
+// over x and the basis, per-block partial sums for every vector; the last block
+// folds the partials and keeps the Hessenberg column (gate_idx 1: the first
+// pass).  Used by classical Gram-Schmidt.
 template <bool FMA>
-__global__ void __launch_bounds__(kRedBlock) k_mdot(const int* gate, int want, int n, DRef xr,
-                                                    const double* __restrict__ basis,
-                                                    const int* count, RedSlot slot,
-                                                    double* __restrict__ out) {
-  if (gated_off(gate, want)) return;
-  const double* __restrict__ x = xr.get();
-  const int k = *count;
+__global__ void __launch_bounds__(kRedBlock) k_mdot(KspState* st, int gate_idx, int n,
+                                                    const double* __restrict__ basis, RedSlot slot,
+                                                    double* hs, double* lhh) {
+  if (gated_off(&st->g[gate_idx], 1)) return;
+  const double* __restrict__ x = st->vv_it1;
+  const int k = st->kcount;
   __shared__ double sh[kRedBlock / 32][kMaxBasis];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -341,11 +392,14 @@ __global__ void __launch_bounds__(kRedBlock) k_mdot(const int* gate, int want, i
         t = add(t, __ldcg(&slot.partials[(size_t)j * slot.stride + b]));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t = add(t, __shfl_down_sync(0xffffffffu, t, o));
-      if (lane == 0) out[j] = t;
+      if (lane == 0) cgs_store(st, hs, lhh, j, t, gate_idx == 1);
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) *slot.ticket = 0u;
+  if (threadIdx.x == 0) {
+    *slot.ticket = 0u;
+    if (gate_idx == 1 && st->cgstype == 1) cgs_norm(st, lhh, k);
+  }
 }
 
 // y = (from_zero ? 0 : y) + sum_{j < *count} coef_j basis_j, ascending j per
@@ -858,38 +912,68 @@ struct Hs {
 // is set or cleared by a control kernel that precedes its kernels in the body.
 __device__ void gm_set_phase(KspState* st, int ph) {
   st->phase = ph;
+  // the Gram-Schmidt of a step that follows: it + 1 vectors, and a second pass
+  // from the start where that is always made
+  if (ph == PH_STEP) {
+    st->kcount = st->it + 1;
+    st->g[7] = st->cgstype == 2 ? 1 : 0;
+  }
   st->g[0] = ph == PH_RESTART;
   st->g[1] = ph == PH_STEP;
   st->g[2] = ph == PH_BUILD;
 }
 
-// KSPGMRESUpdateHessenberg, src/ksp.mojo:589-629
-__device__ int gm_update_hessenberg(Hs& H, int it, int m, int hapend, double* res) {
-  double* hh = H.hh;
-  for (int j = 1; j <= it; j++) {
-    const int idx = it * (m + 2) + (j - 1);
-    const double tt = hh[idx];
-    const double h1 = hh[idx + 1];
-    hh[idx] = add(mul(H.cc[j - 1], tt), mul(H.ss[j - 1], h1));
-    hh[idx + 1] = sub(mul(H.cc[j - 1], h1), mul(H.ss[j - 1], tt));
+// KSPGMRESUpdateHessenberg, src/ksp.mojo:589-629, by one warp.  Applying the
+// earlier rotations to the new column is a chain, t_{j+1} = c_j h_{j+1} - s_j t_j;
+// only that (two dependent FP64 operations a rotation) is left to one lane, the
+// products with h before it and the rows c_j t_j + s_j h_{j+1} after it go a
+// rotation a lane, and the new rotation's two divisions a lane each.  The same
+// operations as one after another.  `sh`: 5 kMaxBasis doubles of shared memory.
+__device__ int gm_update_hessenberg(Hs& H, int it, int m, int hapend, double* res, double* sh) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  double* hh = H.hh + it * (m + 2);
+  double *c = sh, *sn = sh + kMaxBasis, *ch = sh + 2 * kMaxBasis, *snh = sh + 3 * kMaxBasis,
+         *t = sh + 4 * kMaxBasis;
+  for (int j = lane; j < it; j += 32) {
+    const double h1 = hh[j + 1];
+    c[j] = H.cc[j];
+    sn[j] = H.ss[j];
+    ch[j] = mul(c[j], h1);
+    snh[j] = mul(sn[j], h1);
   }
-  if (!hapend) {
-    const int base = it * (m + 2) + it;
-    const double a = hh[base], b = hh[base + 1];
-    const double tt = __dsqrt_rn(add(mul(a, a), mul(b, b)));
-    if (tt == 0.0) {
-      *res = 0.0;
-      return R_NULL;
-    }
-    H.cc[it] = div_(a, tt);
-    H.ss[it] = div_(b, tt);
-    H.rs[it + 1] = mul(-H.ss[it], H.rs[it]);
-    H.rs[it] = mul(H.cc[it], H.rs[it]);
-    hh[base] = add(mul(H.cc[it], a), mul(H.ss[it], b));
-    *res = fabs(H.rs[it + 1]);
+  double tt = hh[0];
+  __syncwarp();
+  for (int j = 0; j < it; j++) {
+    if (lane == 0) t[j] = tt;
+    tt = sub(ch[j], mul(sn[j], tt));
+  }
+  __syncwarp();
+  for (int j = lane; j < it; j += 32) hh[j] = add(mul(c[j], t[j]), snh[j]);
+  const double a = tt, b = hh[it + 1];
+  __syncwarp();
+  *res = 0.0;
+  if (hapend) {
+    if (lane == 0 && it > 0) hh[it] = a;
     return 0;
   }
-  *res = 0.0;
+  const double r = __dsqrt_rn(add(mul(a, a), mul(b, b)));
+  if (r == 0.0) {
+    if (lane == 0 && it > 0) hh[it] = a;
+    return R_NULL;
+  }
+  const double q = div_(lane == 0 ? a : b, r);
+  const double cn = __shfl_sync(full, q, 0), ss = __shfl_sync(full, q, 1);
+  const double rs = H.rs[it], rs1 = mul(-ss, rs);
+  __syncwarp();
+  if (lane == 0) {
+    H.cc[it] = cn;
+    H.ss[it] = ss;
+    H.rs[it + 1] = rs1;
+    H.rs[it] = mul(cn, rs);
+    hh[it] = add(mul(cn, a), mul(ss, b));
+  }
+  *res = fabs(rs1);
   return 0;
 }
 
@@ -937,33 +1021,13 @@ __global__ void k_gm_restart_ctrl(KspState* st, double* hs, double* hist, double
   }
 }
 
-// classical Gram-Schmidt bookkeeping around the MDot / MAXPY pair
-// (src/ksp.mojo:533-586).  pass 0: zero the column and set the count.
-__global__ void k_gm_cgs0(KspState* st, double* hs) {
-  if (!st->g[1]) return;
-  Hs H(hs, st->m);
-  const int it = st->it, m = st->m;
-  for (int j = 0; j <= it; j++) {
-    H.hh[it * (m + 2) + j] = 0.0;
-    H.hes[it * (m + 1) + j] = 0.0;
-  }
-  st->kcount = it + 1;
-  st->g[7] = st->cgstype == 2 ? 1 : 0;
-}
-
-// negate the projections and fold them into the Hessenberg column
+// the ordered multi-dot's results, as k_mdot's last block keeps its own
+// (src/ksp.mojo:533-586)
 __global__ void k_gm_cgs1(KspState* st, double* hs, double* lhh, int gate_idx) {
   if (!st->g[gate_idx]) return;
-  Hs H(hs, st->m);
-  const int it = st->it, m = st->m;
-  double hnrm = 0.0;
-  for (int j = 0; j <= it; j++) {
-    lhh[j] = -lhh[j];
-    H.hh[it * (m + 2) + j] = sub(H.hh[it * (m + 2) + j], lhh[j]);
-    H.hes[it * (m + 1) + j] = sub(H.hes[it * (m + 1) + j], lhh[j]);
-    hnrm = add(hnrm, mul(lhh[j], lhh[j]));
-  }
-  if (gate_idx == 1) st->red[1] = __dsqrt_rn(hnrm);
+  const int it = st->it;
+  for (int j = 0; j <= it; j++) cgs_store(st, hs, lhh, j, lhh[j], gate_idx == 1);
+  if (gate_idx == 1) cgs_norm(st, lhh, it + 1);
 }
 
 // REFINE_IFNEEDED: refine when ||v_{it+1}|| < ||h||
@@ -972,20 +1036,31 @@ __global__ void k_gm_cgs_ifneeded(KspState* st) {
   if (st->red[0] < st->red[1]) st->g[7] = 1;
 }
 
-__global__ void k_gm_step_ctrl(KspState* st, double* hs, double* hist, double* vv, int n) {
-  if (!st->g[1]) return;
+// End of an Arnoldi step, by one warp on `st` (the state, or a copy of it that
+// the caller writes back): the column's last entry st->tt = ||v_{it+1}||, the
+// rotations, the convergence test and the next phase.  |tt / rs| is only formed
+// where it can decide: the happy breakdown bound is at most haptol.
+__device__ void gm_step_warp(KspState* st, double* hs, double* hist, double* vv, int n,
+                             double* sh) {
   Hs H(hs, st->m);
-  const int m = st->m;
+  const int m = st->m, lane = threadIdx.x & 31;
   int it = st->it;
   const double tt = st->tt;
-  H.hh[it * (m + 2) + it + 1] = tt;
-  H.hes[it * (m + 1) + it + 1] = tt;
-  double hapbnd = fabs(div_(tt, H.rs[it]));
-  hapbnd = hapbnd > st->haptol ? st->haptol : hapbnd;
-  const int hapend = tt < hapbnd ? 1 : 0;
-  st->hapend = hapend;
+  if (lane == 0) {
+    H.hh[it * (m + 2) + it + 1] = tt;
+    H.hes[it * (m + 1) + it + 1] = tt;
+  }
+  int hapend = 0;
+  if (!(tt >= st->haptol)) {
+    double hapbnd = fabs(div_(tt, H.rs[it]));
+    hapbnd = hapbnd > st->haptol ? st->haptol : hapbnd;
+    hapend = tt < hapbnd ? 1 : 0;
+  }
+  __syncwarp();
   double res;
-  int reason = gm_update_hessenberg(H, it, m, hapend, &res);
+  int reason = gm_update_hessenberg(H, it, m, hapend, &res, sh);
+  if (lane) return;
+  st->hapend = hapend;
   st->res = res;
   it += 1;
   st->it = it;
@@ -1005,9 +1080,16 @@ __global__ void k_gm_step_ctrl(KspState* st, double* hs, double* hist, double* v
   if (reason == 0 && it < m && st->its < st->max_it) {
     st->vv_it = vv + (size_t)it * n;
     st->vv_it1 = vv + (size_t)(it + 1) * n;
+    gm_set_phase(st, PH_STEP);
   } else {
     gm_set_phase(st, PH_BUILD);
   }
+}
+
+__global__ void k_gm_step_ctrl(KspState* st, double* hs, double* hist, double* vv, int n) {
+  __shared__ double sh[5 * kMaxBasis];
+  if (!st->g[1]) return;
+  gm_step_warp(st, hs, hist, vv, n, sh);
 }
 
 // KSPGMRESBuildSoln's back substitution (src/ksp.mojo:632-664); the vector
@@ -1092,32 +1174,32 @@ __global__ void k_fg_start_ctrl(KspState* st, double* hs, double* hist, double* 
   }
 }
 
-__global__ void k_fg_step_ctrl(KspState* st, double* hs, double* hist, double* vv,
-                               double* prevec, int n) {
-  st->g[10] = 0;
-  st->g[11] = 0;
-  st->g[12] = 0;
-  if (!st->g[1]) return;
+// the same for a flexible step
+__device__ void fg_step_warp(KspState* st, double* hs, double* hist, double* vv, double* prevec,
+                             int n, double* sh) {
   Hs H(hs, st->m);
-  const int m = st->m;
+  const int m = st->m, lane = threadIdx.x & 31;
   int it = st->it;
   const double tt = st->tt;
-  H.hh[it * (m + 2) + it + 1] = tt;
-  H.hes[it * (m + 1) + it + 1] = tt;
+  if (lane == 0) {
+    H.hh[it * (m + 2) + it + 1] = tt;
+    H.hes[it * (m + 1) + it + 1] = tt;
+  }
   double hapbnd = fabs(div_(tt, H.rs[it]));
   hapbnd = hapbnd > st->haptol ? st->haptol : hapbnd;
-  int hapend = 0;
-  if (tt > hapbnd) {
+  const int hapend = tt > hapbnd ? 0 : 1;
+  __syncwarp();
+  double res;
+  int reason = gm_update_hessenberg(H, it, m, hapend, &res, sh);
+  if (lane) return;
+  if (!hapend) {
     st->inv = div_(1.0, tt);
     st->vv_scale = st->vv_it1;
     st->g[10] = 1;  // v_{it+1} *= 1/tt
   } else {
     st->g[12] = 1;  // TEMP = 0
-    hapend = 1;
   }
   st->hapend = hapend;
-  double res;
-  int reason = gm_update_hessenberg(H, it, m, hapend, &res);
   st->res = res;
   st->g[7] = 0;
   if (reason) {
@@ -1136,9 +1218,101 @@ __global__ void k_fg_step_ctrl(KspState* st, double* hs, double* hist, double* v
     st->vv_it = vv + (size_t)it * n;
     st->vv_it1 = vv + (size_t)(it + 1) * n;
     st->pv_it = prevec + (size_t)it * n;
+    gm_set_phase(st, PH_STEP);
   } else {
     gm_set_phase(st, PH_BUILD);
   }
+}
+
+__global__ void k_fg_step_ctrl(KspState* st, double* hs, double* hist, double* vv,
+                               double* prevec, int n) {
+  __shared__ double sh[5 * kMaxBasis];
+  if (threadIdx.x == 0) st->g[10] = st->g[11] = st->g[12] = 0;
+  __syncwarp();
+  if (!st->g[1]) return;
+  fg_step_warp(st, hs, hist, vv, prevec, n, sh);
+}
+
+// The rest of a step after the multi-dot, in one pass: v_{it+1} += sum lhh_j
+// v_j (VecMAXPY, ascending j per element), its norm (each thread's elements in
+// the order of k_dred, so the same sum), and in the last block the step's
+// control.  The control works on a copy of the state in shared memory: its
+// scalars are read one after another, an L2 latency each from global memory.
+template <bool FMA, bool FLEX>
+__global__ void __launch_bounds__(kRedBlock) k_gm_update(KspState* st, double* hs, double* hist,
+                                                         double* vv, double* prevec, int n,
+                                                         const double* lhh, RedSlot slot) {
+  if (gated_off(&st->g[1], 1)) {
+    if (FLEX && blockIdx.x == 0 && threadIdx.x == 0) st->g[10] = st->g[11] = st->g[12] = 0;
+    return;
+  }
+  __shared__ double coef[kMaxBasis];
+  __shared__ double sh[5 * kMaxBasis];
+  __shared__ KspState S;
+  double* __restrict__ y = st->vv_it1;
+  const double* __restrict__ basis = vv;
+  const int k = st->kcount;
+  if (threadIdx.x < k) coef[threadIdx.x] = lhh[threadIdx.x];
+  __syncthreads();
+  double v[1] = {0.0};
+  // four elements a trip, four vectors' loads of each in flight
+  constexpr int U = kVecBatch, J = 4;
+  const unsigned stride = gridDim.x * blockDim.x, un = (unsigned)n;
+  for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < un; i0 += U * stride) {
+    double yv[U];
+    unsigned ii[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      ii[u] = i0 + u * stride < un ? i0 + u * stride : i0;  // past the end: not stored
+      yv[u] = y[ii[u]];
+    }
+    int j = 0;
+    for (; j + J <= k; j += J) {
+      double bv[U][J];
+#pragma unroll
+      for (int q = 0; q < J; q++)
+#pragma unroll
+        for (int u = 0; u < U; u++) bv[u][q] = basis[(size_t)(j + q) * n + ii[u]];
+#pragma unroll
+      for (int q = 0; q < J; q++)
+#pragma unroll
+        for (int u = 0; u < U; u++) yv[u] = madd<FMA>(coef[j + q], bv[u][q], yv[u]);
+    }
+    for (; j < k; j++) {
+      double bv[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) bv[u] = basis[(size_t)j * n + ii[u]];
+#pragma unroll
+      for (int u = 0; u < U; u++) yv[u] = madd<FMA>(coef[j], bv[u], yv[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i0 + u * stride < un) {
+        y[ii[u]] = yv[u];
+        v[0] = madd<FMA>(yv[u], yv[u], v[0]);
+      }
+  }
+  double tot[1];
+  if (!grid_finish<1>(v, slot, tot)) return;
+  static_assert(sizeof(KspState) % sizeof(int) == 0, "copied by words");
+  constexpr int kWords = sizeof(KspState) / sizeof(int);
+  for (int q = threadIdx.x; q < kWords; q += blockDim.x)
+    reinterpret_cast<int*>(&S)[q] = __ldcg(reinterpret_cast<const int*>(st) + q);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) {
+      S.tt = __dsqrt_rn(fabs(tot[0]));
+      if (FLEX) S.g[10] = S.g[11] = S.g[12] = 0;
+    }
+    __syncwarp();
+    if constexpr (FLEX)
+      fg_step_warp(&S, hs, hist, vv, prevec, n, sh);
+    else
+      gm_step_warp(&S, hs, hist, vv, n, sh);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < kWords; q += blockDim.x)
+    reinterpret_cast<int*>(st)[q] = reinterpret_cast<const int*>(&S)[q];
 }
 
 // KSPFGMRESBuildSoln's back substitution (src/ksp.mojo:880-903)
@@ -1588,27 +1762,31 @@ static int bcgs_epilogue(const Run& r, double* x) {
 // ------------------------------------------------------------------ GMRES
 // classical Gram-Schmidt on v_{it+1} against v_0..v_it, with the optional
 // refinement pass (src/ksp.mojo:533-586)
-static int cgs_pass(const Run& r, int gate_idx) {
+static int cgs_dots(const Run& r, int gate_idx) {
   Ksp* k = r.k;
-  const int* g = r.G(gate_idx);
-  DRef v1 = DRef::at(&k->st->vv_it1);
   if (arith_mode() == kOrdered) {
     const int kmax = std::min(k->opt.restart + 1, kMaxBasis);
-    k_ord_mdot<<<kOrdChains * kmax, 32, 0, r.s>>>(g, 1, r.n, v1, k->vv, &k->st->kcount,
-                                                   k->slot, k->lhh);
+    k_ord_mdot<<<kOrdChains * kmax, 32, 0, r.s>>>(r.G(gate_idx), 1, r.n, DRef::at(&k->st->vv_it1),
+                                                   k->vv, &k->st->kcount, k->slot, k->lhh);
+    k_gm_cgs1<<<1, 1, 0, r.s>>>(k->st, k->hs, k->lhh, gate_idx);
   } else {
-    FL(k_mdot, red_grid(r.n), kRedBlock, r.s, g, 1, r.n, v1, k->vv, &k->st->kcount, k->slot,
-                                                k->lhh);
+    FL(k_mdot, red_grid(r.n), kRedBlock, r.s, k->st, gate_idx, r.n, k->vv, k->slot, k->hs, k->lhh);
   }
-  k_gm_cgs1<<<1, 1, 0, r.s>>>(k->st, k->hs, k->lhh, gate_idx);
-  FL(k_maxpy_dyn, r.grid(), 256, r.s, g, 1, r.n, v1, k->vv, k->lhh, &k->st->kcount, 0);
+  GP_CHECK_LAUNCH();
+  return GP_OK;
+}
+
+static int cgs_pass(const Run& r, int gate_idx) {
+  Ksp* k = r.k;
+  GP_TRY(cgs_dots(r, gate_idx));
+  FL(k_maxpy_dyn, r.grid(), 256, r.s, r.G(gate_idx), 1, r.n, DRef::at(&k->st->vv_it1), k->vv,
+     k->lhh, &k->st->kcount, 0);
   GP_CHECK_LAUNCH();
   return GP_OK;
 }
 
 static int cgs(const Run& r) {
   Ksp* k = r.k;
-  k_gm_cgs0<<<1, 1, 0, r.s>>>(k->st, k->hs);
   GP_TRY(cgs_pass(r, 1));
   if (k->opt.cgstype == 1) {
     GP_TRY(r.red<D_NRM>(r.G(1), DRef::at(&k->st->vv_it1), DRef::at(&k->st->vv_it1), nullptr,
@@ -1617,6 +1795,26 @@ static int cgs(const Run& r) {
   }
   if (k->opt.cgstype != 0) GP_TRY(cgs_pass(r, 7));
   return GP_OK;
+}
+
+// Whether an Arnoldi step's projections, norm and control go in k_mdot and
+// k_gm_update: one classical pass, sums in the parallel trees.
+static bool gm_fused(const Run& r) {
+  return arith_mode() != kOrdered && !r.k->opt.orthog && r.k->opt.cgstype == 0;
+}
+
+// Arnoldi steps per loop trip.  The trip's other kernels (a restart before the
+// steps and the solution update after them, gated off in most trips) and the
+// loop's own node cost about 30 us a trip at any size, an unused step about 10;
+// as many as divide the restart, up to 10.  The modified Gram-Schmidt's steps
+// are 3 `restart` kernels each and go one a trip.
+static int gm_steps(const Run& r) {
+  if (r.k->opt.orthog) return 1;
+  const int m = r.k->opt.restart;
+  int best = 1;
+  for (int c = 2; c <= std::min(10, m); c++)
+    if (m % c == 0) best = c;
+  return best >= 4 ? best : std::min(6, m);
 }
 
 // modified Gram-Schmidt (KSPGMRESModifiedGramSchmidtOrthogonalization,
@@ -1663,24 +1861,14 @@ static int gmres_prologue(const Run& r) {
   return GP_OK;
 }
 
+// A trip: a restart where a cycle begins, steps, and the solution update where
+// they ended the cycle (so the trip that converges is the last one).
 static int gmres_body(const Run& r, const double* b, double* x) {
   Ksp* k = r.k;
   const int n = r.n, side = k->opt.pc_side;
   KspState* st = k->st;
   DRef TEMP = DRef::of(k->work), TMATOP = DRef::of(k->work + n), VV0 = DRef::of(k->vv);
   DRef X = DRef::of(x), B = DRef::of(b);
-  // ---- build the solution at the end of a cycle (KSPGMRESBuildSoln)
-  k_gm_backsub<<<1, 1, 0, r.s>>>(st, k->hs);
-  const int m = k->opt.restart;
-  double* rs = k->hs + (size_t)(m + 2) * (m + 1) + (size_t)(m + 1) * (m + 1) + 2 * (m + 1);
-  FL(k_maxpy_dyn, r.grid(), 256, r.s, r.G(6), 1, n, TEMP, k->vv, rs, &st->kcount, 1);
-  GP_CHECK_LAUNCH();
-  if (side == 1) {  // KSPUnwindPreconditioner for right preconditioning
-    GP_TRY(r.pcapply(r.G(6), TEMP, TMATOP));
-    GP_TRY(r.copy(r.G(6), TMATOP, TEMP));
-  }
-  FL(k_axpy_d, r.grid(), 256, r.s, r.G(6), 1, n, X, r.S(&KspState::c_one), 1.0, TEMP);
-  k_gm_build_ctrl<<<1, 1, 0, r.s>>>(st);
   // ---- restart: r0 = M^-1 (b - A x) (or b), normalised
   k_gm_restart_prep<<<1, 1, 0, r.s>>>(st);
   GP_TRY(r.matmult(r.G(3), X, TEMP));
@@ -1698,13 +1886,40 @@ static int gmres_body(const Run& r, const double* b, double* x) {
   k_scale_d<true><<<r.grid(), 256, 0, r.s>>>(r.G(0), 1, n, VV0, r.S(&KspState::res));
   k_gm_restart_ctrl<<<1, 1, 0, r.s>>>(st, k->hs, k->hist, k->vv, n);
   GP_CHECK_LAUNCH();
-  // ---- one Arnoldi step
+  // ---- Arnoldi steps
   DRef vit = DRef::at(&st->vv_it), vit1 = DRef::at(&st->vv_it1);
-  GP_TRY(r.apply_ba(r.G(1), side, vit, vit1, TMATOP));
-  GP_TRY(k->opt.orthog ? mgs(r) : cgs(r));
-  GP_TRY(r.red<D_NRM>(r.G(1), vit1, vit1, nullptr, r.S(&KspState::tt)));
-  k_scale_d<true><<<r.grid(), 256, 0, r.s>>>(r.G(1), 1, n, vit1, r.S(&KspState::tt));
-  k_gm_step_ctrl<<<1, 1, 0, r.s>>>(st, k->hs, k->hist, k->vv, n);
+  for (int step = gm_steps(r); step > 0; step--) {
+    GP_TRY(r.apply_ba(r.G(1), side, vit, vit1, TMATOP));
+    if (gm_fused(r)) {
+      GP_TRY(cgs_dots(r, 1));
+      if (arith_mode() == kFma)
+        k_gm_update<true, false><<<red_grid(n), kRedBlock, 0, r.s>>>(
+            st, k->hs, k->hist, k->vv, nullptr, n, k->lhh, k->slot);
+      else
+        k_gm_update<false, false><<<red_grid(n), kRedBlock, 0, r.s>>>(
+            st, k->hs, k->hist, k->vv, nullptr, n, k->lhh, k->slot);
+      // v_{it+1}, now v_it, where another step follows
+      k_scale_d<true><<<r.grid(), 256, 0, r.s>>>(r.G(1), 1, n, vit, r.S(&KspState::tt));
+    } else {
+      GP_TRY(k->opt.orthog ? mgs(r) : cgs(r));
+      GP_TRY(r.red<D_NRM>(r.G(1), vit1, vit1, nullptr, r.S(&KspState::tt)));
+      k_scale_d<true><<<r.grid(), 256, 0, r.s>>>(r.G(1), 1, n, vit1, r.S(&KspState::tt));
+      k_gm_step_ctrl<<<1, 32, 0, r.s>>>(st, k->hs, k->hist, k->vv, n);
+    }
+    GP_CHECK_LAUNCH();
+  }
+  // ---- build the solution at the end of a cycle (KSPGMRESBuildSoln)
+  k_gm_backsub<<<1, 1, 0, r.s>>>(st, k->hs);
+  const int m = k->opt.restart;
+  double* rs = k->hs + (size_t)(m + 2) * (m + 1) + (size_t)(m + 1) * (m + 1) + 2 * (m + 1);
+  FL(k_maxpy_dyn, r.grid(), 256, r.s, r.G(6), 1, n, TEMP, k->vv, rs, &st->kcount, 1);
+  GP_CHECK_LAUNCH();
+  if (side == 1) {  // KSPUnwindPreconditioner for right preconditioning
+    GP_TRY(r.pcapply(r.G(6), TEMP, TMATOP));
+    GP_TRY(r.copy(r.G(6), TMATOP, TEMP));
+  }
+  FL(k_axpy_d, r.grid(), 256, r.s, r.G(6), 1, n, X, r.S(&KspState::c_one), 1.0, TEMP);
+  k_gm_build_ctrl<<<1, 1, 0, r.s>>>(st);
   GP_CHECK_LAUNCH();
   return GP_OK;
 }
@@ -1736,29 +1951,42 @@ static int fgmres_body(const Run& r, const double* b, double* x) {
   KspState* st = k->st;
   DRef TEMP = DRef::of(k->work), VV0 = DRef::of(k->vv), X = DRef::of(x), B = DRef::of(b);
   double* rs = k->hs + (size_t)(m + 2) * (m + 1) + (size_t)(m + 1) * (m + 1) + 2 * (m + 1);
-  // ---- build (KSPFGMRESBuildSoln) and the next residual
-  k_fg_backsub<<<1, 1, 0, r.s>>>(st, k->hs);
-  FL(k_maxpy_dyn, r.grid(), 256, r.s, r.G(8), 1, n, TEMP, k->prevec, rs, &st->kcount, 1);
-  FL(k_axpy_d, r.grid(), 256, r.s, r.G(8), 1, n, X, r.S(&KspState::c_one), 1.0, TEMP);
-  k_fg_build_ctrl<<<1, 1, 0, r.s>>>(st);
-  GP_CHECK_LAUNCH();
+  // ---- cycle start: the residual of a later cycle, ||r||, convergence test,
+  // v_0 = r / ||r|| (by reciprocal)
   GP_TRY(r.matmult(r.G(9), X, TEMP));
   FL(k_waxpy_d, r.grid(), 256, r.s, r.G(9), 1, n, VV0, r.S(&KspState::c_one), -1.0, TEMP, B);
-  // ---- cycle start: ||r||, convergence test, v_0 = r / ||r|| (by reciprocal)
   GP_TRY(r.red<D_NRM>(r.G(0), VV0, VV0, nullptr, r.S(&KspState::res)));
   k_fg_start_ctrl<<<1, 1, 0, r.s>>>(st, k->hs, k->hist, k->vv, k->prevec, n);
   k_scale_d<false><<<r.grid(), 256, 0, r.s>>>(r.G(11), 1, n, VV0, r.S(&KspState::inv));
   GP_CHECK_LAUNCH();
-  // ---- one flexible Arnoldi step
+  // ---- flexible Arnoldi steps
   DRef vit = DRef::at(&st->vv_it), vit1 = DRef::at(&st->vv_it1), pit = DRef::at(&st->pv_it);
-  GP_TRY(r.pcapply(r.G(1), vit, pit));
-  GP_TRY(r.matmult(r.G(1), pit, vit1));
-  GP_TRY(k->opt.orthog ? mgs(r) : cgs(r));
-  GP_TRY(r.red<D_NRM>(r.G(1), vit1, vit1, nullptr, r.S(&KspState::tt)));
-  k_fg_step_ctrl<<<1, 1, 0, r.s>>>(st, k->hs, k->hist, k->vv, k->prevec, n);
-  k_scale_d<false><<<r.grid(), 256, 0, r.s>>>(r.G(10), 1, n, DRef::at(&st->vv_scale),
-                                              r.S(&KspState::inv));
-  GP_TRY(r.zero(r.G(12), TEMP));
+  for (int step = gm_steps(r); step > 0; step--) {
+    GP_TRY(r.pcapply(r.G(1), vit, pit));
+    GP_TRY(r.matmult(r.G(1), pit, vit1));
+    if (gm_fused(r)) {
+      GP_TRY(cgs_dots(r, 1));
+      if (arith_mode() == kFma)
+        k_gm_update<true, true><<<red_grid(n), kRedBlock, 0, r.s>>>(
+            st, k->hs, k->hist, k->vv, k->prevec, n, k->lhh, k->slot);
+      else
+        k_gm_update<false, true><<<red_grid(n), kRedBlock, 0, r.s>>>(
+            st, k->hs, k->hist, k->vv, k->prevec, n, k->lhh, k->slot);
+    } else {
+      GP_TRY(k->opt.orthog ? mgs(r) : cgs(r));
+      GP_TRY(r.red<D_NRM>(r.G(1), vit1, vit1, nullptr, r.S(&KspState::tt)));
+      k_fg_step_ctrl<<<1, 32, 0, r.s>>>(st, k->hs, k->hist, k->vv, k->prevec, n);
+    }
+    k_scale_d<false><<<r.grid(), 256, 0, r.s>>>(r.G(10), 1, n, DRef::at(&st->vv_scale),
+                                                r.S(&KspState::inv));
+    GP_TRY(r.zero(r.G(12), TEMP));
+    GP_CHECK_LAUNCH();
+  }
+  // ---- build (KSPFGMRESBuildSoln)
+  k_fg_backsub<<<1, 1, 0, r.s>>>(st, k->hs);
+  FL(k_maxpy_dyn, r.grid(), 256, r.s, r.G(8), 1, n, TEMP, k->prevec, rs, &st->kcount, 1);
+  FL(k_axpy_d, r.grid(), 256, r.s, r.G(8), 1, n, X, r.S(&KspState::c_one), 1.0, TEMP);
+  k_fg_build_ctrl<<<1, 1, 0, r.s>>>(st);
   GP_CHECK_LAUNCH();
   return GP_OK;
 }
