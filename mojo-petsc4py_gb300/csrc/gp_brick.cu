@@ -168,7 +168,7 @@ struct BrickRow {
   double c0, c1, c2;  // coefficients in fold order
   double sum0;        // the row's starting value
   double dv;          // diagonal factor
-  double yf;          // SOR_B: the forward value
+  double yf;          // SOR_B: the forward value's share, (1 - omega) y
 };
 
 // ---- shared-memory staging: bulk copies counted on an mbarrier, and 8-byte
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
               r.c2 = stage_get(c1 + 8 * u * NC * LW);
             else if constexpr (DIAG)
               r.dv = stage_get(c1 + 8 * u * NC * LW);
-            if constexpr (MODE == ELL_SOR_B) r.yf = stage_get(v0 + 8 * (kGroup + u) * LW);
+            if constexpr (MODE == ELL_SOR_B) r.yf = mul(a.om1, stage_get(v0 + 8 * (kGroup + u) * LW));
             return r;
           };
           BrickRow r = take(0);
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
                             MODE == ELL_SOR_B0)
                 y = mul(sum, r.dv);
               else if constexpr (MODE == ELL_SOR_B)
-                y = add(mul(a.om1, r.yf), mul(sum, r.dv));
+                y = add(r.yf, mul(sum, r.dv));
               else
                 y = sum;
               prev = act ? y : prev;
@@ -635,13 +635,11 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
 // Stored coefficients from the factor (or operator) values: one thread a
 // position of [tile][step][lane], its coefficients in fold order (0 where the
 // row has no such term or there is no row) and the diagonal: src[dslot[row]],
-// or diag[row] for SOR.  With `stale`, only while that word is set.
-__global__ void k_brick_refresh(const int* gate, int want, BrickShape g, int nc, int npos,
+// or diag[row] for SOR.
+__global__ void k_brick_refresh(BrickShape g, int nc, int npos,
                                 const int* __restrict__ slot, const int* __restrict__ dslot,
                                 const double* __restrict__ src, const double* __restrict__ diag,
-                                double* __restrict__ coef, const int* stale) {
-  if (gated_off(gate, want)) return;
-  if (stale && !*stale) return;
+                                double* __restrict__ coef) {
   const int nd = g.d3 ? 3 : 2;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < npos; e += gridDim.x * blockDim.x) {
     const int lane = e % g.LW, ts = e / g.LW, s = ts % g.NS, T = ts / g.NS;
@@ -964,12 +962,11 @@ int brick_build(EllSweep& ef, EllSweep& eb, int mode_f, int mode_b, int n,
   return GP_OK;
 }
 
-int brick_refresh(EllSweep& e, const double* src, const double* diag, const int* gate, int want,
-                  const int* stale, cudaStream_t s) {
+int brick_refresh(EllSweep& e, const double* src, const double* diag, cudaStream_t s) {
   if (!e.ok || !e.brick || e.n == 0) return GP_OK;
   const int grid = std::max(1, std::min((e.npos + 255) / 256, num_sms() * 8));
-  k_brick_refresh<<<grid, 256, 0, s>>>(gate, want, shape_of(e), e.bcols, e.npos, e.cslot, e.dslot,
-                                       src, diag, e.coef, stale);
+  k_brick_refresh<<<grid, 256, 0, s>>>(shape_of(e), e.bcols, e.npos, e.cslot, e.dslot, src, diag,
+                                       e.coef);
   GP_CHECK_LAUNCH();
   return GP_OK;
 }

@@ -97,7 +97,8 @@ __device__ __forceinline__ void ew(int n, double* y, F f, const double* a,
 }
 
 constexpr int kBodyUnroll = 1;    // default loop-body copies per graph trip
-constexpr int kBodyUnrollCg = 8;  // the same for the fused CG body
+constexpr int kBodyUnrollCg = 8;  // the same for the fused CG body with Jacobi
+constexpr int kBodyUnrollPc = 4;  // and for the fused bodies with other preconditioners
 constexpr int kEagerPoll = 8;   // host-driven loop: trips between state polls
 
 __global__ void k_copy_d(const int* gate, int want, int n, DRef xr, DRef yr) {
@@ -794,12 +795,17 @@ __global__ void __launch_bounds__(kRedBlock, 4) k_cgf_update(
 }
 
 // ||z||^2 and z.r after a separate preconditioner apply (first: prologue).
+// Ends the loop trip with `loop` set, as k_cgf_update does with Jacobi.
 template <bool FMA>
 __global__ void __launch_bounds__(kRedBlock) k_cgf_red(KspState* st, double* hist, int n,
                                                        const double* __restrict__ z,
                                                        const double* __restrict__ r,
-                                                       RedSlot slot, int first) {
-  if (!first && st->active != 1) return;
+                                                       RedSlot slot, int first, int loop,
+                                                       cudaGraphConditionalHandle h) {
+  if (!first && st->active != 1) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) body_loop_ctrl(loop, h, st);
+    return;
+  }
   double v[2] = {0.0, 0.0};
   constexpr int U = kVecBatch;
   double zv[U], rv[U];
@@ -810,8 +816,10 @@ __global__ void __launch_bounds__(kRedBlock) k_cgf_red(KspState* st, double* his
         v[1] = madd<FMA>(zv[u], rv[u], v[1]);
       });
   double tot[2];
-  if (grid_finish<2>(v, slot, tot) && threadIdx.x == 0)
+  if (grid_finish<2>(v, slot, tot) && threadIdx.x == 0) {
     cg_tail(st, hist, __dsqrt_rn(tot[0]), tot[1], first != 0);
+    body_loop_ctrl(loop, h, st);
+  }
 }
 
 // ================================================================== BCGS
@@ -832,10 +840,15 @@ __global__ void k_bcgs_init(KspState* st, double* hist) {
   st->g[G_ON] = 1;
 }
 
-__global__ void k_bcgs_a(KspState* st) {
-  if (st->active != 1) return;
+// the top of an iteration, once rho is known
+__device__ __forceinline__ void bcgs_top(KspState* st) {
   st->bbeta = mul(div_(st->rho, st->rhoold), div_(st->alpha, st->omegaold));
   st->c_omb = mul(-st->omegaold, st->bbeta);
+}
+
+__global__ void k_bcgs_a(KspState* st) {
+  if (st->active != 1) return;
+  bcgs_top(st);
 }
 
 __global__ void k_bcgs_b(KspState* st) {
@@ -890,6 +903,130 @@ __global__ void k_bcgs_d(KspState* st, double* hist) {
   }
   st->i += 1;
   if (st->i >= st->max_it) stop(st, st->dp, its, R_DIVITS);
+}
+
+// ================================================================== BCGS, fused
+// The same recurrence with each dot product's scalar logic in the last block of
+// its reduction and the end of an iteration -- both updates, the norm, the next
+// iteration's rho and its coefficients -- in one pass: besides the products and
+// the preconditioner, seven launches an iteration (two of them for d2 == 0,
+// gated off) instead of nineteen.  Every element is computed with the operations
+// of the unfused kernels (a factor of one left out), and every sum adds the same
+// terms in the order of k_dred.
+
+// P = R - omegaold beta V + beta P
+template <bool FMA>
+__global__ void k_bcgs_p(const KspState* st, int n, double* __restrict__ p,
+                         const double* __restrict__ r, const double* __restrict__ v) {
+  if (gated_off(&st->g[G_ON], 1)) return;
+  const double be = st->c_omb, ga = st->bbeta;
+  ew<3>(
+      n, p, [=](double pv, double vv, double rv) { return madd<FMA>(ga, pv, madd<FMA>(be, vv, rv)); },
+      p, v, r);
+}
+
+// WHAT 0: d1 = V.RP, then alpha = rho / d1 (k_bcgs_b).  WHAT 1: d1 = T.S and
+// d2 = T.T, then omega = d1 / d2 or the d2 == 0 branch (k_bcgs_c).  WHAT 2, in
+// that branch: S.S, a breakdown unless it is zero (k_bcgs_c2).
+template <int WHAT, bool FMA>
+__global__ void __launch_bounds__(kRedBlock) k_bcgs_dots(KspState* st, int n,
+                                                         const double* __restrict__ x,
+                                                         const double* __restrict__ y,
+                                                         RedSlot slot) {
+  if (gated_off(&st->g[WHAT == 2 ? 6 : G_ON], 1)) return;
+  constexpr int NR = WHAT == 1 ? 2 : 1, U = kVecBatch;
+  double v[NR];
+#pragma unroll
+  for (int q = 0; q < NR; q++) v[q] = 0.0;
+  double xv[U], yv[U];
+  grid_batched<U>(
+      n,
+      [&](int u, unsigned i) {
+        xv[u] = x[i];
+        yv[u] = y[i];
+      },
+      [&](int u, unsigned) {
+        v[0] = madd<FMA>(xv[u], yv[u], v[0]);
+        if (WHAT == 1) v[NR - 1] = madd<FMA>(xv[u], xv[u], v[NR - 1]);
+      });
+  double tot[NR];
+  if (!grid_finish<NR>(v, slot, tot) || threadIdx.x) return;
+  st->d1 = tot[0];
+  if constexpr (WHAT == 0) {
+    if (tot[0] == 0.0)
+      stop(st, st->dp, st->its, R_BREAKDOWN);
+    else
+      st->alpha = div_(st->rho, tot[0]);
+  } else if constexpr (WHAT == 1) {
+    st->d2 = tot[NR - 1];
+    st->g[6] = tot[NR - 1] == 0.0;
+    st->g[7] = !st->g[6];
+    if (st->g[7]) st->omega = div_(tot[0], tot[NR - 1]);
+    st->g[0] = (st->g[7] && st->normtype != N_NONE && st->chknorm < st->i + 2) ? 1 : 0;
+  } else {
+    if (tot[0] != 0.0) stop(st, st->dp, st->its, R_BREAKDOWN);
+  }
+}
+
+// X += alpha P + omega S, R = S - omega T, ||R|| and the next rho = R.RP, then
+// the end of the iteration (k_bcgs_d) and the top of the next; ends the trip.
+// Where d2 was zero, X has its update and the solve ends (k_bcgs_c3).
+template <bool FMA>
+__global__ void __launch_bounds__(kRedBlock, 4) k_bcgs_xr(
+    KspState* st, double* hist, int n, double* __restrict__ x, double* __restrict__ r,
+    const double* __restrict__ p, const double* __restrict__ s, const double* __restrict__ t,
+    const double* __restrict__ rp, RedSlot slot, int loop, cudaGraphConditionalHandle h) {
+  if (gated_off(&st->g[7], 1)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (st->active == 1 && st->g[6]) stop(st, 0.0, st->its + 1, R_RTOL);
+      body_loop_ctrl(loop, h, st);
+    }
+    return;
+  }
+  const double al = st->alpha, om = st->omega, nom = -om;
+  constexpr int U = 2;
+  double v[2] = {0.0, 0.0};
+  double xv[U], pv[U], sv[U], tv[U], rv[U];
+  grid_batched<U>(
+      n,
+      [&](int u, unsigned i) {
+        xv[u] = x[i];
+        pv[u] = p[i];
+        sv[u] = s[i];
+        tv[u] = t[i];
+        rv[u] = rp[i];
+      },
+      [&](int u, unsigned i) {
+        x[i] = add(xv[u], madd<FMA>(om, sv[u], mul(al, pv[u])));
+        const double ri = madd<FMA>(nom, tv[u], sv[u]);
+        r[i] = ri;
+        v[0] = madd<FMA>(ri, ri, v[0]);
+        v[1] = madd<FMA>(ri, rv[u], v[1]);
+      });
+  double tot[2];
+  if (!grid_finish<2>(v, slot, tot) || threadIdx.x) return;
+  if (st->g[0]) st->dp = __dsqrt_rn(fabs(tot[0]));
+  const double rho = st->rho, dp = st->dp;
+  st->rhoold = rho;
+  st->omegaold = om;
+  const int its = st->its + 1;
+  st->its = its;
+  hist[its] = dp;
+  const int reason = conv_default(st, its, dp);
+  if (reason) {
+    stop(st, dp, its, reason);
+  } else if (rho == 0.0) {
+    stop(st, dp, its, R_BREAKDOWN);
+  } else {
+    st->i += 1;
+    if (st->i >= st->max_it) {
+      stop(st, dp, its, R_DIVITS);
+    } else {
+      st->rho = tot[1];
+      bcgs_top(st);
+    }
+  }
+  body_loop_ctrl(loop, h, st);
 }
 
 // ================================================================== GMRES
@@ -1627,7 +1764,7 @@ static int cg_prologue_fused(const Run& r, const double* b, double* x) {
   }
   GP_TRY(r.pcapply(nullptr, R, Z));
   FL(k_cgf_red, red_grid(n), kRedBlock, r.s, k->st, k->hist, n, k->work + n, k->work, k->slot,
-     1);
+     1, 0, 0);
   GP_CHECK_LAUNCH();
   return GP_OK;
 }
@@ -1675,13 +1812,15 @@ static int cg_body_fused(const Run& r, double* x) {
       k_cgf_update<false, false><<<g, kRedBlock, 0, r.s>>>(k->st, k->hist, n, x, R, P, W, Z,
                                                            nullptr, k->slot, 0, 0);
     GP_TRY(r.pcapply(r.G(G_ON), DRef::of(R), DRef::of(Z)));
-    FL(k_cgf_red, g, kRedBlock, r.s, k->st, k->hist, n, Z, R, k->slot, 0);
+    FL(k_cgf_red, g, kRedBlock, r.s, k->st, k->hist, n, Z, R, k->slot, 0, r.loop, r.cond);
   }
   GP_CHECK_LAUNCH();
   return GP_OK;
 }
 
 // ------------------------------------------------------------------ BCGS
+static bool bcgs_fused_ok() { return arith_mode() != kOrdered; }
+
 static int bcgs_prologue(const Run& r, const double* b, double* x) {
   Ksp* k = r.k;
   const KspOptions& o = k->opt;
@@ -1702,6 +1841,40 @@ static int bcgs_prologue(const Run& r, const double* b, double* x) {
   GP_TRY(r.copy(on, R, RP));
   GP_TRY(r.zero(on, P));
   GP_TRY(r.zero(on, V));
+  if (bcgs_fused_ok()) {  // later iterations' rho: k_bcgs_xr
+    GP_TRY(r.red<D_DOT>(on, R, RP, r.S(&KspState::rho), nullptr));
+    k_bcgs_a<<<1, 1, 0, r.s>>>(k->st);
+    GP_CHECK_LAUNCH();
+  }
+  return GP_OK;
+}
+
+static int bcgs_body_fused(const Run& r, double* x) {
+  Ksp* k = r.k;
+  const int n = r.n, side = k->opt.pc_side;
+  double* w = k->work;
+  double *R = w, *RP = w + n, *V = w + 2 * (size_t)n, *T = w + 3 * (size_t)n,
+         *S = w + 4 * (size_t)n, *P = w + 5 * (size_t)n;
+  KspState* st = k->st;
+  const int* on = r.G(G_ON);
+  const bool f = arith_mode() == kFma;
+  const int g = red_grid(n);
+  auto dots = [&](auto kf, auto ke, const double* a, const double* b) {
+    (f ? kf : ke)<<<g, kRedBlock, 0, r.s>>>(st, n, a, b, k->slot);
+  };
+  FL(k_bcgs_p, r.grid(), 256, r.s, st, n, P, R, V);
+  GP_TRY(r.apply_ba(on, side, DRef::of(P), DRef::of(V), DRef::of(T)));
+  dots(k_bcgs_dots<0, true>, k_bcgs_dots<0, false>, V, RP);
+  FL(k_waxpy_d, r.grid(), 256, r.s, on, 1, n, DRef::of(S), r.S(&KspState::alpha), -1.0,
+     DRef::of(V), DRef::of(R));
+  GP_TRY(r.apply_ba(on, side, DRef::of(S), DRef::of(T), DRef::of(R)));
+  dots(k_bcgs_dots<1, true>, k_bcgs_dots<1, false>, T, S);
+  dots(k_bcgs_dots<2, true>, k_bcgs_dots<2, false>, S, S);
+  FL(k_axpy_d, r.grid(), 256, r.s, r.G(6), 1, n, DRef::of(x), r.S(&KspState::alpha), 1.0,
+     DRef::of(P));
+  auto kx = f ? k_bcgs_xr<true> : k_bcgs_xr<false>;
+  kx<<<g, kRedBlock, 0, r.s>>>(st, k->hist, n, x, R, P, S, T, RP, k->slot, r.loop, r.cond);
+  GP_CHECK_LAUNCH();
   return GP_OK;
 }
 
@@ -2020,16 +2193,17 @@ static int run_prologue(const Run& r, const double* b, double* x) {
   return GP_OK;
 }
 
-// Whether the body's last kernel ends the loop trip itself (the fused CG with
-// Jacobi: its update kernel), so no separate loop-control kernel follows.
+// Whether the body's last kernel ends the loop trip itself (the fused CG's and
+// BiCGStab's), so no separate loop-control kernel follows.
 static bool body_ends_trip(const Run& r) {
-  return r.k->opt.type == KSP_CG && cg_fused_ok(r) && r.pc->opt.type == PC_JACOBI;
+  return (r.k->opt.type == KSP_CG && cg_fused_ok(r)) ||
+         (r.k->opt.type == KSP_BCGS && bcgs_fused_ok());
 }
 
 static int run_body(const Run& r, const double* b, double* x) {
   switch (r.k->opt.type) {
     case KSP_CG: return cg_fused_ok(r) ? cg_body_fused(r, x) : cg_body(r, x);
-    case KSP_BCGS: return bcgs_body(r, x);
+    case KSP_BCGS: return bcgs_fused_ok() ? bcgs_body_fused(r, x) : bcgs_body(r, x);
     case KSP_GMRES: return gmres_body(r, b, x);
     case KSP_FGMRES: return fgmres_body(r, b, x);
   }
@@ -2037,15 +2211,18 @@ static int run_body(const Run& r, const double* b, double* x) {
 }
 
 // Loop-body copies per conditional trip (GPETSC_KSP_UNROLL, 1..16; by default
-// kBodyUnrollCg for the three-kernel fused CG body, whose trips are short
-// enough that the conditional node's re-launch shows, else kBodyUnroll).
+// kBodyUnrollCg for the three-kernel CG body with Jacobi, whose trips are short
+// enough that the conditional node's re-launch shows most; kBodyUnrollPc for the
+// other bodies that end their own trip, where an unused copy is 6 to 14 launches;
+// else kBodyUnroll).
 static int body_unroll(const Run& r) {
   static int env = [] {
     const char* e = std::getenv("GPETSC_KSP_UNROLL");
     return e ? std::max(1, std::min(16, std::atoi(e))) : 0;
   }();
   if (env) return env;
-  return body_ends_trip(r) ? kBodyUnrollCg : kBodyUnroll;
+  if (!body_ends_trip(r)) return kBodyUnroll;
+  return r.k->opt.type == KSP_CG && r.pc->opt.type == PC_JACOBI ? kBodyUnrollCg : kBodyUnrollPc;
 }
 
 // GPETSC_KSP_GRAPH=0: drive the loop from the host (same kernels, launched on

@@ -137,12 +137,6 @@ __global__ void k_copy_g(const int* gate, int want, int n, DRef xr, DRef yr) {
     y[i] = x[i];
 }
 
-// ------------------------------------------------------------------ SOR
-__global__ void k_clear_word(const int* gate, int want, int* w) {
-  if (gated_off(gate, want)) return;
-  *w = 0;
-}
-
 static bool stream_capturing(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
@@ -152,34 +146,15 @@ static bool stream_capturing(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-// With `stale` given, runs only while *stale is nonzero (A's values changed
-// since the last run): the result depends on the values alone.
+// ------------------------------------------------------------------ SOR
 __global__ void k_sor_diag(int n, double omega, double fshift, const int* __restrict__ diagpos,
                            const double* __restrict__ val, double* __restrict__ idiag,
-                           double* __restrict__ mdiag, const int* gate = nullptr, int want = 0,
-                           const int* stale = nullptr) {
-  if (gated_off(gate, want)) return;
-  if (stale && *stale == 0) return;
+                           double* __restrict__ mdiag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double a = val[diagpos[i]];
   mdiag[i] = a;
   idiag[i] = (omega == 1.0 && fshift <= 0.0) ? div_(1.0, a) : div_(omega, add(fshift, a));
-}
-
-// SOR's ELL coefficients follow A's current values (gathered by an apply
-// while *stale is nonzero)
-__global__ void k_ell_refresh_g(const int* gate, int want, int n, const int* __restrict__ cnt,
-                                const int* __restrict__ cslot, const double* __restrict__ src,
-                                double* __restrict__ coef, const int* stale) {
-  if (gated_off(gate, want)) return;
-  if (*stale == 0) return;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-    const int c = cnt[p];
-    for (int e = 0; e < c; e++) {
-      coef[(size_t)e * n + p] = src[cslot[(size_t)e * n + p]];
-    }
-  }
 }
 
 __global__ void k_fill_pending(const int* gate, int want, int n, double* __restrict__ a,
@@ -531,7 +506,7 @@ static void free_all(Pc* pc) {
                   pc->perm_r, pc->perm_c, pc->perm_ic, pc->ba, pc->ba_orig, pc->done, pc->cptr, pc->crow,
                   pc->cslot, pc->tptr, pc->trow, pc->tslot, pc->amap, pc->fwd.order,
                   pc->bwd.order, pc->num.order, pc->yf, pc->yb, pc->ys, pc->t, pc->tickets,
-                  pc->err, pc->upd_ptr, pc->upd_dst, pc->upd_src, pc->sor_stale};
+                  pc->err, pc->upd_ptr, pc->upd_dst, pc->upd_src};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   ell_free(pc->ef);
@@ -596,6 +571,24 @@ static int check_sorted_with_diag(const Csr* A, const char* who) {
     }
   }
   return GP_OK;
+}
+
+// What SOR's applies take from A's values: the inverted diagonal and the
+// sweeps' coefficients.  The reference inverts the diagonal on every apply
+// (MatInvertDiagonalForSOR_SeqAIJ, src/ported.mojo:610-633); it depends on the
+// values alone, so it is done at set-up and, ahead of the next apply or solve,
+// when the values changed (pc_values_sync), never inside an apply: a solver
+// loop's applies have no kernels for it.
+static int sor_refresh(Pc* pc, cudaStream_t s) {
+  const Csr* A = pc->A;
+  pc->sor_vver = A->vver;
+  GP_TRY(sor_diagonals(pc, s));
+  if (pc->ef.brick) {
+    GP_TRY(brick_refresh(pc->ef, A->val, pc->idiag, s));
+    return brick_refresh(pc->eb, A->val, pc->idiag, s);
+  }
+  GP_TRY(ell_refresh(pc->ef, A->val, s));
+  return ell_refresh(pc->eb, A->val, s);
 }
 
 static int setup_sor(Pc* pc, cudaStream_t s) {
@@ -664,15 +657,7 @@ static int setup_sor(Pc* pc, cudaStream_t s) {
   }
   GP_TRY(dalloc(&pc->t, n));
   GP_TRY(dalloc(&pc->yf, n));
-  GP_CUDA(cudaMalloc(&pc->sor_stale, sizeof(int)));
-  GP_CUDA(cudaMemsetAsync(pc->sor_stale, 1, sizeof(int), s));  // nonzero: recompute
-  pc->sor_vver = A->vver;
-  if (n) {
-    k_sor_diag<<<(n + 255) / 256, 256, 0, s>>>(n, pc->opt.omega, pc->opt.fshift, A->diagpos,
-                                                A->val, pc->idiag, pc->mdiag);
-    GP_CHECK_LAUNCH();
-  }
-  return GP_OK;
+  return sor_refresh(pc, s);
 }
 
 static int perms(Pc* pc, std::vector<int>& r, std::vector<int>& ic) {
@@ -1058,22 +1043,14 @@ int pc_update_values(Pc* pc, cudaStream_t s) {
       return GP_OK;
     case PC_ILU:
     case PC_ICC: return pc_factor_numeric(pc, s);
-    case PC_SOR:
-      // recomputed from the values by the next apply
-      GP_CUDA(cudaMemsetAsync(pc->sor_stale, 1, sizeof(int), s));
-      pc->sor_vver = A->vver;
-      return GP_OK;
+    case PC_SOR: return sor_refresh(pc, s);
     default: return GP_OK;  // none
   }
 }
 
 int pc_values_sync(Pc* pc, cudaStream_t s) {
-  if (pc->opt.type != PC_SOR || !pc->ready || !pc->A || !pc->sor_stale) return GP_OK;
-  if (pc->A->vver != pc->sor_vver) {
-    GP_CUDA(cudaMemsetAsync(pc->sor_stale, 1, sizeof(int), s));
-    pc->sor_vver = pc->A->vver;
-  }
-  return GP_OK;
+  if (pc->opt.type != PC_SOR || !pc->ready || !pc->A || pc->A->vver == pc->sor_vver) return GP_OK;
+  return sor_refresh(pc, s);
 }
 
 int pc_setup(Pc* pc, Csr* A, cudaStream_t s) {
@@ -1156,37 +1133,18 @@ int pc_apply(Pc* pc, DRef x, DRef y, cudaStream_t s, const int* gate, int want) 
       const Csr* A = pc->A;
       const int flag = pc->opt.sor_flag;
       const bool fw = flag & kSorForward, bw = flag & kSorBackward;
-      // The reference runs MatInvertDiagonalForSOR_SeqAIJ on every apply, from
-      // the current values (src/ported.mojo:610-633).  The inverted diagonal
-      // and the sweeps' coefficients are functions of the values alone, so
-      // they are recomputed only while the device word sor_stale is set: by
-      // set-up, and before a launch when A's values changed since
-      // (pc_values_sync; a captured solve calls it before every launch).
       if (!stream_capturing(s)) GP_TRY(pc_values_sync(pc, s));
-      k_sor_diag<<<(n + 255) / 256, 256, 0, s>>>(n, pc->opt.omega, pc->opt.fshift, A->diagpos,
-                                                  A->val, pc->idiag, pc->mdiag, gate, want,
-                                                  pc->sor_stale);
       if (pc->ef.brick) {
-        GP_TRY(brick_refresh(pc->ef, A->val, pc->idiag, gate, want, pc->sor_stale, s));
-        GP_TRY(brick_refresh(pc->eb, A->val, pc->idiag, gate, want, pc->sor_stale, s));
-        k_clear_word<<<1, 1, 0, s>>>(gate, want, pc->sor_stale);
         if (fw)
           GP_TRY(brick_sweep(ELL_SOR_F, pc->ef, gate, want, x, y, nullptr, nullptr, pc->yf, pc->t,
                              pc->opt.omega, bw ? 0 : 1, tk0, pc->err, s));
         if (bw)
-          GP_TRY(brick_sweep(fw ? ELL_SOR_B : ELL_SOR_B0, pc->eb, gate, want, x, y, pc->yf, pc->t, nullptr, nullptr,
-                             pc->opt.omega, 1, tk1, pc->err, s));
+          GP_TRY(brick_sweep(fw ? ELL_SOR_B : ELL_SOR_B0, pc->eb, gate, want, x, y, pc->yf, pc->t,
+                             nullptr, nullptr, pc->opt.omega, 1, tk1, pc->err, s));
         break;
       }
       k_fill_pending<<<g, 256, 0, s>>>(gate, want, n, pc->yf, pc->yb);
       if (pc->ef.ok && pc->eb.ok) {
-        if (!pc->ef.tiled)
-          k_ell_refresh_g<<<g, 256, 0, s>>>(gate, want, pc->ef.n, pc->ef.cnt, pc->ef.cslot,
-                                            A->val, pc->ef.coef, pc->sor_stale);
-        if (!pc->eb.tiled)
-          k_ell_refresh_g<<<g, 256, 0, s>>>(gate, want, pc->eb.n, pc->eb.cnt, pc->eb.cslot,
-                                            A->val, pc->eb.coef, pc->sor_stale);
-        k_clear_word<<<1, 1, 0, s>>>(gate, want, pc->sor_stale);
         if (fw)
           GP_TRY(ell_sweep(ELL_SOR_F, pc->ef, gate, want, x, y, pc->yf, nullptr, pc->t, nullptr,
                            pc->idiag, pc->opt.omega, 0, bw ? 0 : 1, tk0, pc->err, A->val, s));
@@ -1195,7 +1153,6 @@ int pc_apply(Pc* pc, DRef x, DRef y, cudaStream_t s, const int* gate, int want) 
                            pc->idiag, pc->opt.omega, fw ? 1 : 0, 1, tk1, pc->err, A->val, s));
         break;
       }
-      k_clear_word<<<1, 1, 0, s>>>(gate, want, pc->sor_stale);
       if (fw)
         k_sor_fwd<<<sg, kSweepBlock, 0, s>>>(gate, want, n, pc->fwd.order, tk0, A->rowptr,
                                              A->colind, A->val, A->diagpos, pc->idiag, x, pc->t,

@@ -97,9 +97,8 @@ int brick_build(EllSweep& ef, EllSweep& eb, int mode_f, int mode_b, int n,
                 const std::vector<int>& dslot, const std::vector<int>& perm, int nlevels,
                 bool chosen_form, bool* built);
 // Coefficients (and diagonal: from src, or diag by row) of a brick sweep from
-// the current values; with `stale`, only while that word is set.
-int brick_refresh(EllSweep& e, const double* src, const double* diag, const int* gate, int want,
-                  const int* stale, cudaStream_t s);
+// the current values.
+int brick_refresh(EllSweep& e, const double* src, const double* diag, cudaStream_t s);
 int brick_reset(EllSweep& e, cudaStream_t s);
 // One brick sweep.  First sweeps read `in` and leave their values (tout) and
 // SOR's checkpoint (tout2) by row, where second sweeps read them (tin, tin2).
@@ -160,10 +159,8 @@ struct Pc {
   // SOR (uses A's arrays and diagpos)
   double* idiag = nullptr;
   double* mdiag = nullptr;
-  // SOR: nonzero while the inverted diagonal and the sweeps' coefficients
-  // must be recomputed from A's values (device word, read by the apply's
-  // kernels); sor_vver is the A->vver they were last marked for
-  int* sor_stale = nullptr;
+  // SOR: the A->vver that the inverted diagonal and the sweeps' coefficients
+  // were last computed for
   unsigned long long sor_vver = 0;
 
   // factor (ILU / IC), reference layout on the device
@@ -233,9 +230,9 @@ int pc_factor_numeric(Pc* pc, cudaStream_t s);
 // Same operator pattern, new values: redo only the numeric phase (factor
 // values, Jacobi diagonals) in the arrays of the last set-up.
 int pc_update_values(Pc* pc, cudaStream_t s);
-// Mark SOR's value-derived arrays for recomputation when the operator's values
-// changed since they were last marked (outside stream capture; a captured
-// solve graph calls it before every launch).
+// Recompute SOR's value-derived arrays when the operator's values changed since
+// (outside stream capture; a captured solve graph's owner calls it before every
+// launch).
 int pc_values_sync(Pc* pc, cudaStream_t s);
 int pc_import_factor(Pc* pc, int type, const FactorPattern& pat, const std::vector<int>& perm_c,
                      const double* ba_host, Csr* A, cudaStream_t s);

@@ -1055,7 +1055,7 @@ int sweep_wait_probe(int budget, int set, cudaStream_t s) {
 
 int ell_refresh(EllSweep& e, const double* src, cudaStream_t s) {
   if (!e.ok || e.tiled || e.n == 0) return GP_OK;  // the tiled form gathers at each sweep
-  if (e.brick) return brick_refresh(e, src, nullptr, nullptr, 0, nullptr, s);
+  if (e.brick) return brick_refresh(e, src, nullptr, s);
   k_ell_refresh<<<std::max(1, std::min((e.n + 255) / 256, num_sms() * 8)), 256, 0, s>>>(
       e.n, e.W, e.cnt, e.cslot, src, e.coef, e.dslot, e.dval);
   GP_CHECK_LAUNCH();
