@@ -37,10 +37,10 @@ namespace gp {
 
 constexpr int kMixBlock = 256;
 constexpr int kMixMaxM = 64;
+constexpr int kMixTickets = (kMixMaxM + 7) / 8;  // a ticket per eight dots
 
 // ------------------------------------------------------------------ kernels
-// CTAs of the multi-dot kernels: four per SM (more loads in flight; the last
-// CTA's fold stays short)
+// CTAs of the host form's dots: four per SM (the last CTA's fold stays short)
 static int mdot_grid(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 4));
 }
@@ -144,11 +144,11 @@ __device__ __forceinline__ void fold_partials(const double* partials, int kk, do
   }
 }
 
-// Dots of w against basis rows 0..k-1 (rows of V, leading dimension n), or
+// Dots of w against basis rows 0..k-1 (rows of V, leading dimension ld), or
 // ||w||^2 when V is null: FP32 per thread and per CTA, per-CTA partials in
 // FP64; the last CTA folds them (FP64) into out[0..k-1].
-__global__ void __launch_bounds__(kMixBlock) k_mdot32(int n, const float* __restrict__ V,
-                                                      int k, const float* __restrict__ w,
+__global__ void __launch_bounds__(kMixBlock) k_mdot32(int n, size_t ld,
+                                                      const float* __restrict__ V, int k, const float* __restrict__ w,
                                                       double* __restrict__ partials,
                                                       unsigned* ticket, double* out) {
   __shared__ float sh[kMixBlock / 32][kMixMaxM + 1];
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kMixBlock) k_mdot32(int n, const float* __rest
       const float wi = w[i];
 #pragma unroll
       for (int q = 0; q < 8; q++)
-        if (j0 + q < kk) acc[q] = __fmaf_rn(V ? V[(size_t)(j0 + q) * n + i] : wi, wi, acc[q]);
+        if (j0 + q < kk) acc[q] = __fmaf_rn(V ? V[(j0 + q) * ld + i] : wi, wi, acc[q]);
     }
 #pragma unroll
     for (int q = 0; q < 8; q++) {
@@ -189,14 +189,14 @@ __global__ void __launch_bounds__(kMixBlock) k_mdot32(int n, const float* __rest
 }
 
 // w -= sum_{j<k} h_j V_j   (h in FP64 on the device, applied in FP32)
-__global__ void k_maxpy32(int n, const float* __restrict__ V, int k, const double* __restrict__ h,
-                          float* __restrict__ w) {
+__global__ void k_maxpy32(int n, size_t ld, const float* __restrict__ V, int k,
+                          const double* __restrict__ h, float* __restrict__ w) {
   __shared__ float hs[kMixMaxM + 1];
   for (int j = threadIdx.x; j < k; j += blockDim.x) hs[j] = (float)h[j];
   __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float v = w[i];
-    for (int j = 0; j < k; j++) v = __fmaf_rn(-hs[j], V[(size_t)j * n + i], v);
+    for (int j = 0; j < k; j++) v = __fmaf_rn(-hs[j], V[j * ld + i], v);
     w[i] = v;
   }
 }
@@ -418,8 +418,15 @@ static void bt_free(BlockTri& b) {
   b = BlockTri();
 }
 
+// The column offsets of a matrix whose entries lie on W <= 8 diagonals, slot e
+// of every row being column i + d[e] (ascending).
+struct DiaOffsets {
+  int d[8];
+};
+
 struct Mixed {
   int n = 0, m = 0, device = -1;
+  size_t ld = 0;  // leading dimension of V: n up to a multiple of 4 (16-byte rows)
   BlockTri bl, bu;       // block layouts of L and U (tri_block != 0)
   int bt_rows = 0;       // their block length (0: not built)
   unsigned long long bt_generation = 0;
@@ -438,6 +445,16 @@ struct Mixed {
   int lW = 0, uW = 0;
   int *lell_ci = nullptr, *lell_slot = nullptr, *uell_ci = nullptr, *uell_slot = nullptr;
   float *lell_val = nullptr, *uell_val = nullptr;
+  // both triangles by diagonals: slot e of every row is column i + off.d[e]
+  // (the ELL slots and values are then in that order, and there are no columns)
+  bool tri_dia = false;
+  DiaOffsets loff{}, uoff{};
+  // A's FP32 values by diagonals ([e * n + i]; aW 0: not of that form)
+  int aW = 0;
+  DiaOffsets aoff{};
+  float* adia = nullptr;
+  int* a_scan = nullptr;
+  unsigned long long adia_uid = 0, adia_vver = 0;
   // work
   float *V = nullptr, *Z = nullptr, *w = nullptr, *t0 = nullptr, *t1 = nullptr, *t2 = nullptr;
   float *t3 = nullptr, *t4 = nullptr;
@@ -465,7 +482,7 @@ static void mixed_free(Mixed* M) {
                   M->uval, M->udinv, M->lell_ci, M->lell_slot, M->uell_ci, M->uell_slot,
                   M->lell_val, M->uell_val, M->V, M->Z, M->w, M->t0, M->t1, M->t2, M->t3, M->t4,
                   M->r, M->y,
-                  M->d64, M->h_dev, M->partials, M->x64tmp, M->ticket};
+                  M->d64, M->h_dev, M->partials, M->x64tmp, M->ticket, M->adia, M->a_scan};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (M->h_pinned) cudaFreeHost(M->h_pinned);
@@ -503,17 +520,23 @@ static int mixed_factors(Mixed* M, cudaStream_t s) {
       }
     std::vector<int> lrp(n + 1, 0), lci, lsl, urp(n + 1, 0), uci, usl, dsl(n);
     for (int i = 0; i < n; i++) {
-      for (int j = P.bi[i]; j < P.bi[i + 1]; j++) {
-        lci.push_back(P.bj[j]);
-        lsl.push_back(j);
-      }
-      lrp[i + 1] = (int)lci.size();
-      for (int j = P.bdiag[i + 1] + 1; j < P.bdiag[i]; j++) {
-        uci.push_back(P.bj[j]);
-        usl.push_back(j);
-      }
-      urp[i + 1] = (int)uci.size();
+      lrp[i + 1] = lrp[i] + P.bi[i + 1] - P.bi[i];
+      urp[i + 1] = urp[i] + P.bdiag[i] - P.bdiag[i + 1] - 1;
       dsl[i] = P.bdiag[i];
+    }
+    lci.resize(lrp[n]);
+    lsl.resize(lrp[n]);
+    uci.resize(urp[n]);
+    usl.resize(urp[n]);
+    for (int i = 0; i < n; i++) {
+      for (int j = lrp[i], q = P.bi[i]; j < lrp[i + 1]; j++, q++) {
+        lci[j] = P.bj[q];
+        lsl[j] = q;
+      }
+      for (int j = urp[i], q = P.bdiag[i + 1] + 1; j < urp[i + 1]; j++, q++) {
+        uci[j] = P.bj[q];
+        usl[j] = q;
+      }
     }
     M->lnnz = (int64_t)lci.size();
     M->unnz = (int64_t)uci.size();
@@ -527,7 +550,52 @@ static int mixed_factors(Mixed* M, cudaStream_t s) {
     GP_CUDA(cudaMalloc(&M->lval, std::max<int64_t>(M->lnnz, 1) * sizeof(float)));
     GP_CUDA(cudaMalloc(&M->uval, std::max<int64_t>(M->unnz, 1) * sizeof(float)));
     GP_CUDA(cudaMalloc(&M->udinv, std::max(n, 1) * sizeof(float)));
-    // ELL copies
+    // identity permutations (natural ordering) are skipped by the passes
+    std::vector<int> pr(n), pcv(n);
+    if (n) {
+      GP_CUDA(cudaMemcpy(pr.data(), pc->perm_r, n * sizeof(int), cudaMemcpyDeviceToHost));
+      GP_CUDA(cudaMemcpy(pcv.data(), pc->perm_c, n * sizeof(int), cudaMemcpyDeviceToHost));
+    }
+    M->ident_r = M->ident_c = true;
+    for (int i = 0; i < n; i++) {
+      M->ident_r = M->ident_r && pr[i] == i;
+      M->ident_c = M->ident_c && pcv[i] == i;
+    }
+    // by diagonals where both triangles are of that form in the operator's own
+    // order (a stencil's factor), else ELL copies
+    auto diagonals = [&](const std::vector<int>& rp, const std::vector<int>& ci, DiaOffsets& off,
+                         int& W) {
+      W = 0;
+      for (int i = 0; i < n; i++)
+        for (int j = rp[i], e = 0; j < rp[i + 1]; j++, e++) {
+          const int o = ci[j] - i;
+          if (j > rp[i] && ci[j] <= ci[j - 1]) return false;
+          while (e < W && off.d[e] < o) e++;
+          if (e < W && off.d[e] == o) continue;
+          if (W == 8) return false;
+          for (int q = W++; q > e; q--) off.d[q] = off.d[q - 1];
+          off.d[e] = o;
+        }
+      return W > 0;
+    };
+    M->tri_dia = M->ident_r && M->ident_c && diagonals(lrp, lci, M->loff, M->lW) &&
+                 diagonals(urp, uci, M->uoff, M->uW);
+    auto dia = [&](const std::vector<int>& rp, const std::vector<int>& ci,
+                   const std::vector<int>& sl, int W, const DiaOffsets& off, int** esl,
+                   float** eval) -> int {
+      std::vector<int> t((size_t)W * n);
+      for (int i = 0; i < n; i++) {
+        int j = rp[i];
+        for (int e = 0; e < W; e++) {
+          const bool here = j < rp[i + 1] && ci[j] - i == off.d[e];
+          t[(size_t)e * n + i] = here ? sl[j] : -1;
+          j += here;
+        }
+      }
+      GP_TRY(up_mixed(esl, t));
+      GP_CUDA(cudaMalloc(eval, (size_t)W * n * sizeof(float)));
+      return GP_OK;
+    };
     auto ell = [&](const std::vector<int>& rp, const std::vector<int>& ci,
                    const std::vector<int>& sl, int& W, int** eci, int** esl,
                    float** eval) -> int {
@@ -549,18 +617,12 @@ static int mixed_factors(Mixed* M, cudaStream_t s) {
       GP_CUDA(cudaMalloc(eval, (size_t)W * n * sizeof(float)));
       return GP_OK;
     };
-    GP_TRY(ell(lrp, lci, lsl, M->lW, &M->lell_ci, &M->lell_slot, &M->lell_val));
-    GP_TRY(ell(urp, uci, usl, M->uW, &M->uell_ci, &M->uell_slot, &M->uell_val));
-    // identity permutations (natural ordering) are skipped by the passes
-    std::vector<int> pr(n), pcv(n);
-    if (n) {
-      GP_CUDA(cudaMemcpy(pr.data(), pc->perm_r, n * sizeof(int), cudaMemcpyDeviceToHost));
-      GP_CUDA(cudaMemcpy(pcv.data(), pc->perm_c, n * sizeof(int), cudaMemcpyDeviceToHost));
-    }
-    M->ident_r = M->ident_c = true;
-    for (int i = 0; i < n; i++) {
-      M->ident_r = M->ident_r && pr[i] == i;
-      M->ident_c = M->ident_c && pcv[i] == i;
+    if (M->tri_dia) {
+      GP_TRY(dia(lrp, lci, lsl, M->lW, M->loff, &M->lell_slot, &M->lell_val));
+      GP_TRY(dia(urp, uci, usl, M->uW, M->uoff, &M->uell_slot, &M->uell_val));
+    } else {
+      GP_TRY(ell(lrp, lci, lsl, M->lW, &M->lell_ci, &M->lell_slot, &M->lell_val));
+      GP_TRY(ell(urp, uci, usl, M->uW, &M->uell_ci, &M->uell_slot, &M->uell_val));
     }
     M->pc_generation = pc->generation;
     M->pc_epoch = -1;
@@ -576,6 +638,97 @@ static int mixed_factors(Mixed* M, cudaStream_t s) {
       k_ell32_refresh<<<g, 256, 0, s>>>((int64_t)M->uW * n, M->uell_slot, pc->ba, M->uell_val);
     GP_CHECK_LAUNCH();
     M->pc_epoch = pc->epoch;
+  }
+  return GP_OK;
+}
+
+// A by diagonals, found on the device (the operator may have no host pattern):
+// scan = {bad, W, d[8], packed widest row}.
+__global__ void k_dia_widest(int n, const int* __restrict__ rp, unsigned long long* widest) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned len = i < n ? (unsigned)(rp[i + 1] - rp[i]) : 0u;
+  const unsigned wmax = __reduce_max_sync(0xffffffffu, len);
+  const unsigned who = __ballot_sync(0xffffffffu, len == wmax);
+  if ((int)(threadIdx.x & 31) == __ffs(who) - 1 && i < n)
+    atomicMax(widest, ((unsigned long long)wmax << 32) | (unsigned)i);
+}
+
+__global__ void k_dia_offsets(const int* __restrict__ rp, const int* __restrict__ ci, int* scan,
+                              const unsigned long long* widest) {
+  const int len = (int)(*widest >> 32), i = (int)(*widest & 0xffffffffu);
+  scan[0] = len < 1 || len > 8;
+  scan[1] = len;
+  for (int e = 0; e < len && e < 8; e++) scan[2 + e] = ci[rp[i] + e] - i;
+}
+
+// every row's entries on those diagonals, in their order
+__global__ void k_dia_check(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                            int* scan) {
+  if (*(volatile int*)scan) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int W = scan[1];
+  int e = 0;
+  for (int j = rp[i]; j < rp[i + 1]; j++) {
+    while (e < W && scan[2 + e] != ci[j] - i) e++;
+    if (e++ >= W) {
+      *(volatile int*)scan = 1;
+      return;
+    }
+  }
+}
+
+__global__ void k_dia_fill(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                           const float* __restrict__ val, int W, DiaOffsets off,
+                           float* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int j = rp[i];
+  const int je = rp[i + 1];
+  for (int e = 0; e < W; e++) {
+    const bool here = j < je && ci[j] - i == off.d[e];
+    out[(size_t)e * n + i] = here ? val[j] : 0.f;
+    j += here;
+  }
+}
+
+// (Re)build A's diagonals from its FP32 values, when its entries lie on at most
+// eight of them and some row has them all (no work for a denser matrix beyond
+// the scan, once per operator).
+static int mixed_operator(Mixed* M, const Csr* A, cudaStream_t s) {
+  const int n = A->n, gr = (n + 255) / 256;
+  if (M->adia_uid != A->uid) {
+    if (M->adia) GP_CUDA(cudaFree(M->adia));
+    M->adia = nullptr;
+    M->aW = 0;
+    if (!M->a_scan) GP_CUDA(cudaMalloc(&M->a_scan, 12 * sizeof(int)));
+    int h[10] = {1};
+    if (A->n == A->ncols && A->nnz) {
+      auto* widest = reinterpret_cast<unsigned long long*>(M->a_scan + 10);
+      GP_CUDA(cudaMemsetAsync(widest, 0, sizeof(*widest), s));
+      k_dia_widest<<<gr, 256, 0, s>>>(n, A->rowptr, widest);
+      k_dia_offsets<<<1, 1, 0, s>>>(A->rowptr, A->colind, M->a_scan, widest);
+      k_dia_check<<<gr, 256, 0, s>>>(n, A->rowptr, A->colind, M->a_scan);
+      GP_CUDA(cudaMemcpyAsync(h, M->a_scan, sizeof(h), cudaMemcpyDeviceToHost, s));
+      GP_CUDA(cudaStreamSynchronize(s));
+    }
+    // without the memory for the copy the passes read the CSR values
+    if (!h[0] && cudaMalloc(&M->adia, (size_t)h[1] * n * sizeof(float)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      M->adia = nullptr;
+      h[0] = 1;
+    }
+    if (!h[0]) {
+      M->aW = h[1];
+      std::copy(h + 2, h + 2 + h[1], M->aoff.d);
+    }
+    M->adia_uid = A->uid;
+    M->adia_vver = A->vver - 1;
+  }
+  if (M->aW && M->adia_vver != A->vver) {
+    k_dia_fill<<<gr, 256, 0, s>>>(n, A->rowptr, A->colind, A->val32, M->aW, M->aoff, M->adia);
+    GP_CHECK_LAUNCH();
+    M->adia_vver = A->vver;
   }
   return GP_OK;
 }
@@ -696,17 +849,23 @@ static int mixed_blocks(Mixed* M, int want, cudaStream_t s) {
   if (M->bt_rows != rows || M->bt_generation != pc->generation || !M->bl.cstart) {
     std::vector<int> lrp(n + 1, 0), lci, lsl, urp(n + 1, 0), uci, usl, dsl(n);
     for (int i = 0; i < n; i++) {
-      for (int j = P.bi[i]; j < P.bi[i + 1]; j++) {
-        lci.push_back(P.bj[j]);
-        lsl.push_back(j);
-      }
-      lrp[i + 1] = (int)lci.size();
-      for (int j = P.bdiag[i + 1] + 1; j < P.bdiag[i]; j++) {
-        uci.push_back(P.bj[j]);
-        usl.push_back(j);
-      }
-      urp[i + 1] = (int)uci.size();
+      lrp[i + 1] = lrp[i] + P.bi[i + 1] - P.bi[i];
+      urp[i + 1] = urp[i] + P.bdiag[i] - P.bdiag[i + 1] - 1;
       dsl[i] = P.bdiag[i];
+    }
+    lci.resize(lrp[n]);
+    lsl.resize(lrp[n]);
+    uci.resize(urp[n]);
+    usl.resize(urp[n]);
+    for (int i = 0; i < n; i++) {
+      for (int j = lrp[i], q = P.bi[i]; j < lrp[i + 1]; j++, q++) {
+        lci[j] = P.bj[q];
+        lsl[j] = q;
+      }
+      for (int j = urp[i], q = P.bdiag[i + 1] + 1; j < urp[i + 1]; j++, q++) {
+        uci[j] = P.bj[q];
+        usl[j] = q;
+      }
     }
     GP_TRY(bt_build(M->bl, n, true, lrp, lci, lsl, nullptr, &P.r, rows));
     GP_TRY(bt_build(M->bu, n, false, urp, uci, usl, &dsl, nullptr, rows));
@@ -761,7 +920,8 @@ static int mixed_buffers(Mixed* M, int n, int m) {
   if (M->h_pinned) cudaFreeHost(M->h_pinned);
   M->h_pinned = nullptr;
   const size_t nn = std::max(n, 1);
-  GP_CUDA(cudaMalloc(&M->V, (size_t)(m + 1) * nn * sizeof(float)));
+  M->ld = (nn + 3) & ~(size_t)3;
+  GP_CUDA(cudaMalloc(&M->V, (size_t)(m + 1) * M->ld * sizeof(float)));
   GP_CUDA(cudaMalloc(&M->Z, (size_t)m * nn * sizeof(float)));
   for (float** p : {&M->w, &M->t0, &M->t1, &M->t2, &M->t3, &M->t4})
     GP_CUDA(cudaMalloc(p, nn * sizeof(float)));
@@ -769,8 +929,8 @@ static int mixed_buffers(Mixed* M, int n, int m) {
   GP_CUDA(cudaMalloc(&M->y, nn * sizeof(double)));
   GP_CUDA(cudaMalloc(&M->h_dev, (m + 2) * sizeof(double)));
   GP_CUDA(cudaMalloc(&M->partials, (size_t)(m + 2) * mix_grid(n) * sizeof(double)));
-  GP_CUDA(cudaMalloc(&M->ticket, sizeof(unsigned)));
-  GP_CUDA(cudaMemset(M->ticket, 0, sizeof(unsigned)));
+  GP_CUDA(cudaMalloc(&M->ticket, kMixTickets * sizeof(unsigned)));
+  GP_CUDA(cudaMemset(M->ticket, 0, kMixTickets * sizeof(unsigned)));
   GP_CUDA(cudaMallocHost(&M->h_pinned, (m + 2) * sizeof(double)));
   M->n = n;
   M->m = m;
@@ -780,7 +940,7 @@ static int mixed_buffers(Mixed* M, int n, int m) {
 // k dots of w against V's first k rows (or ||w||^2 with V null) into host h
 static int mdot_host(Mixed* M, const float* V, int k, const float* w, double* h, cudaStream_t s) {
   const int n = M->n, g = mix_grid(n);
-  k_mdot32<<<mdot_grid(n), kMixBlock, 0, s>>>(n, V, k, w, M->partials, M->ticket, M->h_dev);
+  k_mdot32<<<mdot_grid(n), kMixBlock, 0, s>>>(n, M->ld, V, k, w, M->partials, M->ticket, M->h_dev);
   GP_CHECK_LAUNCH();
   const int kk = V ? k : 1;
   GP_CUDA(cudaMemcpyAsync(M->h_pinned, M->h_dev, kk * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -896,7 +1056,7 @@ int mixed_solve(Mixed* M, Csr* A, Pc* pc, const double* b, double* x, const Mixe
     gv[0] = beta;
     int kdim = 0;
     for (int j = 0; j < m; j++) {
-      float* vj = M->V + (size_t)j * n;
+      float* vj = M->V + (size_t)j * M->ld;
       float* zj = M->Z + (size_t)j * n;
       GP_TRY(mixed_pc(M, o.tri_sweeps, vj, zj, s));
       if (A->coff16)
@@ -905,7 +1065,7 @@ int mixed_solve(Mixed* M, Csr* A, Pc* pc, const double* b, double* x, const Mixe
         k_spmv32<int><<<gr, kMixBlock, 0, s>>>(n, A->rowptr, A->colind, A->val32, zj, M->w);
       // classical Gram-Schmidt against v_0..v_j
       GP_TRY(mdot_host(M, M->V, j + 1, M->w, h.data(), s));
-      k_maxpy32<<<g, kMixBlock, 0, s>>>(n, M->V, j + 1, M->h_dev, M->w);
+      k_maxpy32<<<g, kMixBlock, 0, s>>>(n, M->ld, M->V, j + 1, M->h_dev, M->w);
       double hn2 = 0.0;
       GP_TRY(mdot_host(M, nullptr, 1, M->w, &hn2, s));
       const double hn = std::sqrt(hn2);
@@ -927,7 +1087,7 @@ int mixed_solve(Mixed* M, Csr* A, Pc* pc, const double* b, double* x, const Mixe
       kdim = j + 1;
       if (!(hn > 0.0) || std::fabs(gv[j + 1]) <= o.inner_rtol * beta) break;
       if (j + 1 < m)
-        k_scale32<<<g, kMixBlock, 0, s>>>(n, M->w, (float)(1.0 / hn), M->V + (size_t)(j + 1) * n);
+        k_scale32<<<g, kMixBlock, 0, s>>>(n, M->w, (float)(1.0 / hn), M->V + (size_t)(j + 1) * M->ld);
     }
     // y = H^-1 g (upper triangular), d = Z y, x += ||r|| d
     for (int i = kdim - 1; i >= 0; i--) {
@@ -954,7 +1114,7 @@ int mixed_solve(Mixed* M, Csr* A, Pc* pc, const double* b, double* x, const Mixe
 // correction.  The host launches passes and reads one status word per pass.
 struct MixDev {
   int pass_on, active, kdim, its, passes, pad_;
-  double rn, rtol_bnorm, beta2, beta, tol, inner_rtol, hn2;
+  double rn, rtol_bnorm, beta2, beta, tol, inner_rtol, hjj;
   // reciprocals computed once by the one thread that has the norm (a divide
   // in every thread of a streaming kernel costs more than the stream)
   double inv_rn;
@@ -1128,6 +1288,129 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_tri_ell(
   }
 }
 
+// A load of constant data that stays where it is written: before the wait on the
+// previous kernel (the compiler sinks a plain one to its use, past the wait).
+__device__ __forceinline__ float ld_here(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+// The same pass over a triangle stored by diagonals: no columns to load (a third
+// of the bytes at three slots), and all of a thread's eight rows' loads -- its
+// coefficients before the wait, right-hand sides and gathers after it -- are in
+// flight together, where the ELL form's gathers wait on its columns and go out
+// a row at a time (its conditional permutation and scale keep them apart).  A
+// row past the end loads the last one's values and stores nothing; an entry a
+// row does not have has a zero coefficient and is left out of the sum.  Bound by
+// the L2 (25 MB of it at 96^3 in 3.4 us; 1, 2 and 4 rows a thread: 9.7, 6.1 and
+// 4.3 us), with consecutive tiles of a block no worse than grid-wide strides.
+//
+// What lies between the passes is done here too.  sc: rhs and in are the
+// unscaled new basis vector, *sc its factor, and the scaled one goes to vout
+// (the first L pass; a launch and 7 MB less).  out2 = out * scale2 (the last L
+// pass leaves D^-1 y for the first U pass, which then gathers one array, not two).
+template <int W>
+__global__ void __launch_bounds__(kMixBlock) k_mx_tri_dia(
+    const int* gate, int n, DiaOffsets off, const float* __restrict__ val,
+    const float* __restrict__ dinv, const float* __restrict__ rhs, const float* __restrict__ in,
+    const float* sc, float* __restrict__ vout, float* __restrict__ out,
+    const float* __restrict__ scale2, float* __restrict__ out2) {
+  constexpr int R = kTriRows;
+  const int i0 = blockIdx.x * (R * kMixBlock) + threadIdx.x;
+  float a[R][W], x[R][W], acc[R], dv[R];
+  auto coefs = [&]() {
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+      const int i = min(i0 + q * kMixBlock, n - 1);
+#pragma unroll
+      for (int e = 0; e < W; e++) a[q][e] = ld_here(val + (size_t)e * n + i);
+    }
+    if (dinv) {
+#pragma unroll
+      for (int q = 0; q < R; q++) dv[q] = ld_here(dinv + min(i0 + q * kMixBlock, n - 1));
+    } else {
+#pragma unroll
+      for (int q = 0; q < R; q++) dv[q] = 1.f;
+    }
+  };
+  // constant during a solve; the gate read before the wait only decides when
+  const bool early = !gated_off(gate, 1);
+  if (early) coefs();
+  pdl_wait();
+  pdl_trigger();
+  if (gated_off(gate, 1)) return;
+  if (!early) coefs();
+  const float f = sc ? *sc : 1.f;
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int i = min(i0 + q * kMixBlock, n - 1);
+    acc[q] = rhs[i];
+#pragma unroll
+    for (int e = 0; e < W; e++) x[q][e] = in[min(max(i + off.d[e], 0), n - 1)];
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int i = i0 + q * kMixBlock;
+    float r = acc[q] * f;
+    if (vout && i < n) vout[i] = r;
+#pragma unroll
+    for (int e = 0; e < W; e++) {
+      const float t = __fmaf_rn(-a[q][e], x[q][e] * f, r);
+      r = a[q][e] != 0.f ? t : r;
+    }
+    r *= dv[q];
+    if (i < n) out[i] = r;
+    if (out2 && i < n) out2[i] = r * scale2[i];
+  }
+}
+
+// y = A x over A's diagonals: coalesced loads only, a row's gathers waiting on
+// nothing (4.1 us at 96^3; a row a thread over CSR reads each of a warp's value
+// slots from seven cache lines: 14 us).  Two rows a thread (1: 4.4 us, 4: 4.9).
+constexpr int kMxSpmvRows = 2;
+
+template <int W>
+__global__ void __launch_bounds__(kMixBlock) k_mx_spmv_dia(const int* gate, int n, DiaOffsets off,
+                                                           const float* __restrict__ val,
+                                                           const float* __restrict__ x,
+                                                           float* __restrict__ y) {
+  constexpr int R = kMxSpmvRows;
+  const int i0 = blockIdx.x * (R * kMixBlock) + threadIdx.x;
+  float a[R][W], t[R][W];
+  auto coefs = [&]() {
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+      const int i = min(i0 + q * kMixBlock, n - 1);
+#pragma unroll
+      for (int e = 0; e < W; e++) a[q][e] = ld_here(val + (size_t)e * n + i);
+    }
+  };
+  const bool early = !gated_off(gate, 1);
+  if (early) coefs();
+  pdl_wait();
+  pdl_trigger();
+  if (gated_off(gate, 1)) return;
+  if (!early) coefs();
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int i = min(i0 + q * kMixBlock, n - 1);
+#pragma unroll
+    for (int e = 0; e < W; e++) t[q][e] = x[min(max(i + off.d[e], 0), n - 1)];
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int i = i0 + q * kMixBlock;
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < W; e++) {
+      const float v = __fmaf_rn(a[q][e], t[q][e], acc);
+      acc = a[q][e] != 0.f ? v : acc;
+    }
+    if (i < n) y[i] = acc;
+  }
+}
+
 template <typename CT>
 __global__ void __launch_bounds__(kMixBlock) k_mx_spmv32(const int* gate, int n,
                                                          const int* __restrict__ rp,
@@ -1147,145 +1430,203 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_spmv32(const int* gate, int n,
   y[row] = acc;
 }
 
-// w -= V h and ||w||^2 in one pass (the orthogonalised vector's norm is
-// folded while it is written): FP32 per thread and per CTA, per-CTA partials
-// in FP64, the last CTA folds them into *out.  Gated on `*gate == 1`.
-__global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_norm(const int* gate, int n,
+// The earlier rotations of Hessenberg column j (FP64, one warp): a chain, t_{i+1}
+// = c_i h_{i+1} - s_i t_i, of which only the one fused multiply-add a rotation
+// (64 cycles) runs in order; the products before it and the entries c_i t_i +
+// s_i h_{i+1} after it go a rotation a lane.  Its end is the column's last entry.
+__device__ void mx_rotate(MixDev* st, const double* __restrict__ h, int j, int m) {
+  __shared__ double cs[kMixMaxM], sn[kMixMaxM], ch[kMixMaxM], sh[kMixMaxM], tv[kMixMaxM];
+  const int lane = threadIdx.x & 31;
+  for (int i = lane; i < j; i += 32) {
+    const double c = st->cs[i], sv = st->sn[i], h1 = h[i + 1];
+    cs[i] = c;
+    sn[i] = sv;
+    ch[i] = __dmul_rn(c, h1);
+    sh[i] = __dmul_rn(sv, h1);
+  }
+  double t = h[0];
+  __syncwarp();
+  for (int i = 0; i < j; i++) {
+    if (lane == 0) tv[i] = t;
+    t = __fma_rn(-sn[i], t, ch[i]);
+  }
+  __syncwarp();
+  for (int i = lane; i < j; i += 32) st->H[i * m + j] = __fma_rn(cs[i], tv[i], sh[i]);
+  if (lane == 0) st->hjj = t;
+}
+
+// The new rotation and the residual estimate, by one warp (two lanes take a
+// reciprocal each).
+__device__ void mx_givens(MixDev* st, double hn2, int j, int m) {
+  const int lane = threadIdx.x & 31;
+  const double t = __ldcg(&st->hjj), gj = __ldcg(&st->g[j]), tol = __ldcg(&st->tol);
+  const double hn = sqrt(hn2);
+  // one square root and one reciprocal (FP64 divide, square root and hypot
+  // are long dependent sequences on this part; the operands are far from
+  // overflow: a normalised basis keeps them O(||A||))
+  const double den = sqrt(__fma_rn(t, t, hn2));
+  const double v = lane == 0 ? den : hn;
+  const double r = v > 0.0 ? 1.0 / v : 0.0;
+  const double rden = __shfl_sync(0xffffffffu, r, 0), rhn = __shfl_sync(0xffffffffu, r, 1);
+  if (lane) return;
+  st->inv_hn = (float)rhn;
+  const double cj = den > 0.0 ? t * rden : 1.0;
+  const double sj = den > 0.0 ? hn * rden : 0.0;
+  st->H[j * m + j] = den;
+  st->cs[j] = cj;
+  st->sn[j] = sj;
+  const double gn = -sj * gj;
+  st->g[j + 1] = gn;
+  st->g[j] = cj * gj;
+  st->kdim = j + 1;
+  st->its += 1;
+  if (!(hn > 0.0) || fabs(gn) <= tol || j + 1 == m) st->active = 0;
+}
+
+__device__ __forceinline__ void fma4(float4& v, float c, const float4& t) {
+  v.x = __fmaf_rn(c, t.x, v.x);
+  v.y = __fmaf_rn(c, t.y, v.y);
+  v.z = __fmaf_rn(c, t.z, v.z);
+  v.w = __fmaf_rn(c, t.w, v.w);
+}
+
+// The sum of nb CTAs' FP32 partials in FP64 by one warp, sixteen loads a lane in
+// flight (a round trip to the L2 each sixteen, not each load).
+__device__ __forceinline__ double fold_row(const float* partials, int nb) {
+  const int lane = threadIdx.x & 31;
+  double t = 0.0;
+  for (int b = lane; b < nb; b += 16 * 32) {
+    float v[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = b + q * 32 < nb ? __ldcg(partials + b + q * 32) : 0.f;
+#pragma unroll
+    for (int q = 0; q < 16; q++) t += (double)v[q];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// w -= V h, ||w||^2 and the step's control in one pass: the orthogonalised
+// vector's norm is folded while it is written (FP32 per thread and per CTA, the
+// CTAs' sums in FP64 by the last one, which then makes the new rotation); CTA 0
+// meanwhile applies the earlier rotations to the column, which need no norm.
+// Gated on `active`.  A streaming read of V's k rows: 16-byte loads, eight rows
+// of V in flight a thread (with 4-byte loads the addresses take the registers
+// that the loads need), from the last row of the vectors down, so that what the
+// dots read last, which the L2 still holds, is read first.
+__global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_step(int n, size_t ld,
                                                              const float* __restrict__ V, int k,
                                                              const double* __restrict__ h,
                                                              float* __restrict__ w,
-                                                             double* __restrict__ partials,
-                                                             unsigned* ticket, double* out) {
+                                                             float* __restrict__ partials,
+                                                             unsigned* ticket, MixDev* st, int m) {
   pdl_wait();
   pdl_trigger();
-  if (gated_off(gate, 1)) return;
+  if (gated_off(&st->active, 1)) return;
   __shared__ float hs[kMixMaxM + 1];
   __shared__ float sh[kMixBlock / 32];
+  __shared__ double shd[kMixBlock / 32];
   __shared__ bool last;
-  for (int j = threadIdx.x; j < k; j += blockDim.x) hs[j] = (float)h[j];
-  __syncthreads();
-  float acc = 0.f;
-  // two rows a thread per step, eight basis loads of each in flight before
-  // their (ordered) multiply-adds
-  const int stride = gridDim.x * blockDim.x;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + stride < n; i += 2 * stride) {
-    float v0 = w[i], v1 = w[i + stride];
-    int j = 0;
-    for (; j + 8 <= k; j += 8) {
-      float t0[8], t1[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        t0[q] = V[(size_t)(j + q) * n + i];
-        t1[q] = V[(size_t)(j + q) * n + i + stride];
-      }
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        v0 = __fmaf_rn(-hs[j + q], t0[q], v0);
-        v1 = __fmaf_rn(-hs[j + q], t1[q], v1);
-      }
-    }
-    for (; j < k; j++) {
-      v0 = __fmaf_rn(-hs[j], V[(size_t)j * n + i], v0);
-      v1 = __fmaf_rn(-hs[j], V[(size_t)j * n + i + stride], v1);
-    }
-    w[i] = v0;
-    w[i + stride] = v1;
-    acc = __fmaf_rn(v0, v0, acc);
-    acc = __fmaf_rn(v1, v1, acc);
-  }
-  for (; i < n; i += stride) {
-    float v = w[i];
-    for (int j = 0; j < k; j++) v = __fmaf_rn(-hs[j], V[(size_t)j * n + i], v);
-    w[i] = v;
-    acc = __fmaf_rn(v, v, acc);
-  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nb = gridDim.x - 1;  // CTAs that stream
+  float acc = 0.f;
+  if (blockIdx.x == 0) {
+    if (wid == 0) mx_rotate(st, h, k - 1, m);
+    if (wid == 1 && lane < (n & 3)) {  // and the rows beyond the last four
+      const int i = (n & ~3) + lane;
+      float v = w[i];
+      for (int j = 0; j < k; j++) v = __fmaf_rn(-(float)h[j], V[j * ld + i], v);
+      w[i] = v;
+      acc = __fmaf_rn(v, v, acc);
+    }
+  } else {
+    for (int j = threadIdx.x; j < k; j += blockDim.x) hs[j] = (float)h[j];
+    __syncthreads();
+    const int n4 = n >> 2;
+    float4* w4 = reinterpret_cast<float4*>(w);
+    for (int i = n4 - 1 - (int)((blockIdx.x - 1) * kMixBlock + threadIdx.x); i >= 0;
+         i -= nb * kMixBlock) {
+      float4 v = w4[i];
+      for (int j = 0; j < k; j += 8) {
+        float4 t[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if (j + q < k) t[q] = reinterpret_cast<const float4*>(V + (j + q) * ld)[i];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if (j + q < k) fma4(v, -hs[j + q], t[q]);
+      }
+      w4[i] = v;
+      acc = __fmaf_rn(v.x, v.x, acc);
+      acc = __fmaf_rn(v.y, v.y, acc);
+      acc = __fmaf_rn(v.z, v.z, acc);
+      acc = __fmaf_rn(v.w, v.w, acc);
+    }
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if (lane == 0) sh[wid] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     float t = 0.f;
-    for (int ww = 0; ww < (int)(blockDim.x >> 5); ww++) t += sh[ww];
-    partials[blockIdx.x] = (double)t;
+    for (int ww = 0; ww < kMixBlock / 32; ww++) t += sh[ww];
+    partials[blockIdx.x] = t;
     last = atomic_add_acq_rel(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
-  fold_partials(partials, 1, out);
+  double t = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 8 * kMixBlock) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      v[q] = b + q * kMixBlock < (int)gridDim.x ? __ldcg(partials + b + q * kMixBlock) : 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) t += (double)v[q];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if (lane == 0) shd[wid] = t;
   __syncthreads();
-  if (threadIdx.x == 0) *ticket = 0u;
+  if (wid) return;
+  double hn2 = lane < kMixBlock / 32 ? shd[lane] : 0.0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) hn2 += __shfl_down_sync(0xffffffffu, hn2, o);
+  hn2 = __shfl_sync(0xffffffffu, hn2, 0);
+  if (lane == 0) *ticket = 0u;
+  mx_givens(st, hn2, k - 1, m);
 }
 
-// Hessenberg column j, rotations and the residual estimate (one thread, FP64)
-// One warp: the lanes stage the new column and the earlier rotations in
-// shared memory (independent loads), then lane 0 runs the rotations out of
-// shared memory -- the chain is the FP64 arithmetic, not a memory round trip
-// per rotation.
-__global__ void k_mx_givens(MixDev* st, const double* __restrict__ h, int j, int m) {
-  pdl_wait();
-  pdl_trigger();
-  if (!st->active) return;
-  __shared__ double col[kMixMaxM + 1], cs[kMixMaxM], sn[kMixMaxM];
-  for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-    col[i] = h[i];
-    if (i < j) {
-      cs[i] = st->cs[i];
-      sn[i] = st->sn[i];
-    }
-  }
-  __syncwarp();
-  if (threadIdx.x != 0) return;
-  double* H = st->H;
-  const double hn = sqrt(st->hn2);
-  st->inv_hn = hn > 0.0 ? (float)(1.0 / hn) : 0.f;
-  for (int i = 0; i < j; i++) {
-    const double a = col[i], c = col[i + 1];
-    col[i] = cs[i] * a + sn[i] * c;
-    col[i + 1] = -sn[i] * a + cs[i] * c;
-  }
-  const double hjj = col[j];
-  // one square root and one reciprocal (FP64 divide, square root and hypot
-  // are long dependent sequences on this part; the operands are far from
-  // overflow: a normalised basis keeps them O(||A||))
-  const double den = sqrt(hjj * hjj + hn * hn);
-  const double rden = den > 0.0 ? 1.0 / den : 0.0;
-  const double cj = den > 0.0 ? hjj * rden : 1.0;
-  const double sj = den > 0.0 ? hn * rden : 0.0;
-  col[j] = den;
-  for (int i = 0; i <= j; i++) H[i * m + j] = col[i];
-  st->cs[j] = cj;
-  st->sn[j] = sj;
-  const double gj = st->g[j];
-  st->g[j + 1] = -sj * gj;
-  st->g[j] = cj * gj;
-  st->kdim = j + 1;
-  st->its += 1;
-  if (!(hn > 0.0) || fabs(-sj * gj) <= st->tol || j + 1 == m) st->active = 0;
-}
-
-// Back-substitution of the least-squares system: the warp stages the upper
-// triangle of H and g in shared memory, lane 0 solves out of it.
+// Back-substitution of the least-squares system by one warp, by columns: the
+// lanes hold the rows (two each), the reciprocals of the diagonal are taken a
+// lane each beforehand, and an unknown costs one multiply, its broadcast and one
+// multiply-add (row by row in one thread, with a divide and a chain of sums for
+// each, it took 45 us for 30).
 __global__ void k_mx_backsub(MixDev* st, int m) {
   if (!st->pass_on) return;
-  __shared__ double Hs[kMixMaxM * kMixMaxM], gs[kMixMaxM], ys[kMixMaxM];
-  const int k = st->kdim;
-  for (int q = threadIdx.x; q < k * k; q += blockDim.x) {
+  __shared__ double Hs[kMixMaxM * kMixMaxM];
+  const int k = st->kdim, lane = threadIdx.x;
+  for (int q = lane; q < k * k; q += 32) {
     const int i = q / k, c = q % k;
     if (c >= i) Hs[i * k + c] = st->H[i * m + c];
   }
-  for (int i = threadIdx.x; i < k; i += blockDim.x) gs[i] = st->g[i];
   __syncwarp();
-  if (threadIdx.x == 0) {
-    for (int i = k - 1; i >= 0; i--) {
-      double t = gs[i];
-      for (int c = i + 1; c < k; c++) t -= Hs[i * k + c] * ys[c];
-      ys[i] = Hs[i * k + i] != 0.0 ? t / Hs[i * k + i] : 0.0;
-    }
+  double t[2], rd[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int i = lane + 32 * u;
+    t[u] = i < k ? st->g[i] : 0.0;
+    const double d = i < k ? Hs[i * k + i] : 0.0;
+    rd[u] = d != 0.0 ? 1.0 / d : 0.0;
   }
-  __syncwarp();
-  for (int i = threadIdx.x; i < k; i += blockDim.x) st->y[i] = ys[i];
+  for (int c = k - 1; c >= 0; c--) {
+    const int u = c >> 5;
+    const double y = __shfl_sync(0xffffffffu, u ? t[1] * rd[1] : t[0] * rd[0], c & 31);
+    if (lane == (c & 31)) st->y[c] = y;
+    if (lane < c) t[0] = __fma_rn(-Hs[lane * k + c], y, t[0]);
+    if (lane + 32 < c) t[1] = __fma_rn(-Hs[(lane + 32) * k + c], y, t[1]);
+  }
 }
 
 // x += rn * sum_{j < kdim} y_j Z_j
@@ -1312,70 +1653,83 @@ __global__ void k_mx_correct(int n, const float* __restrict__ Z, const MixDev* s
   }
 }
 
-// the mdot of the host-driven form, gated on `*gate == 1`
-__global__ void __launch_bounds__(kMixBlock) k_mx_mdot(const int* gate, int n,
-                                                       const float* __restrict__ V, int k,
-                                                       const float* __restrict__ w,
-                                                       double* __restrict__ partials,
-                                                       unsigned* ticket, double* out) {
+// Dots of w against V's rows 8 blockIdx.y .. + 7 (of k), gated on `*gate == 1`:
+// FP32 per thread and per CTA, the CTAs' sums in FP64 by the last CTA of each
+// eight.  16-byte loads, the eight rows of V in flight together; a CTA of 128
+// threads takes one such load a thread up to 96^3 (k = 16 in 6.1 us there, with
+// CTAs of 256 7.5, with the eights in turn inside a CTA 7.2; four rows a thread
+// with 4-byte loads and the eights in turn took 28 for 12).
+constexpr int kMdotBlock = 128;
+
+static dim3 mx_mdot_grid(int64_t n, int k) {
+  const int64_t b = (n / 4 + kMdotBlock - 1) / kMdotBlock;
+  return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)num_sms() * 3)),
+              (unsigned)((k + 7) / 8));
+}
+
+__global__ void __launch_bounds__(kMdotBlock) k_mx_mdot(const int* gate, int n, size_t ld,
+                                                        const float* __restrict__ V, int k,
+                                                        const float* __restrict__ w,
+                                                        float* __restrict__ partials,
+                                                        unsigned* ticket, double* out) {
   pdl_wait();
   pdl_trigger();
   if (gated_off(gate, 1)) return;
-  __shared__ float sh[kMixBlock / 32][kMixMaxM + 1];
+  constexpr int nw = kMdotBlock / 32;
+  __shared__ float sh[nw][8];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int kk = V ? k : 1;
-  for (int j0 = 0; j0 < kk; j0 += 8) {
-    float acc[8];
+  const int j0 = blockIdx.y * 8, kk = min(8, k - j0), n4 = n >> 2;
+  V += j0 * ld;
+  float acc[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) acc[q] = 0.f;
-    // two rows a thread per step, all their loads issued before the
-    // multiply-adds (accumulation order per thread unchanged: row by row)
-    const int stride = gridDim.x * blockDim.x;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    for (; i + stride < n; i += 2 * stride) {
-      const float w0 = w[i], w1 = w[i + stride];
-      float v0[8], v1[8];
+  for (int q = 0; q < 8; q++) acc[q] = 0.f;
+  for (int i = blockIdx.x * kMdotBlock + threadIdx.x; i < n4; i += gridDim.x * kMdotBlock) {
+    float4 t[8];
+    const float4 ww = reinterpret_cast<const float4*>(w)[i];
 #pragma unroll
-      for (int q = 0; q < 8; q++)
-        if (j0 + q < kk) {
-          v0[q] = V ? V[(size_t)(j0 + q) * n + i] : w0;
-          v1[q] = V ? V[(size_t)(j0 + q) * n + i + stride] : w1;
-        }
+    for (int q = 0; q < 8; q++)
+      if (q < kk) t[q] = reinterpret_cast<const float4*>(V + q * ld)[i];
 #pragma unroll
-      for (int q = 0; q < 8; q++)
-        if (j0 + q < kk) {
-          acc[q] = __fmaf_rn(v0[q], w0, acc[q]);
-          acc[q] = __fmaf_rn(v1[q], w1, acc[q]);
-        }
-    }
-    for (; i < n; i += stride) {
-      const float wi = w[i];
+    for (int q = 0; q < 8; q++)
+      if (q < kk) {
+        acc[q] = __fmaf_rn(t[q].x, ww.x, acc[q]);
+        acc[q] = __fmaf_rn(t[q].y, ww.y, acc[q]);
+        acc[q] = __fmaf_rn(t[q].z, ww.z, acc[q]);
+        acc[q] = __fmaf_rn(t[q].w, ww.w, acc[q]);
+      }
+  }
+  if (blockIdx.x == 0 && (int)threadIdx.x < (n & 3)) {
+    const int i = (n4 << 2) + threadIdx.x;
 #pragma unroll
-      for (int q = 0; q < 8; q++)
-        if (j0 + q < kk) acc[q] = __fmaf_rn(V ? V[(size_t)(j0 + q) * n + i] : wi, wi, acc[q]);
-    }
+    for (int q = 0; q < 8; q++)
+      if (q < kk) acc[q] = __fmaf_rn(V[q * ld + i], w[i], acc[q]);
+  }
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
+  for (int q = 0; q < 8; q++) {
+    if (q < kk) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
-      if (lane == 0 && j0 + q < kk) sh[wid][j0 + q] = acc[q];
+      if (lane == 0) sh[wid][q] = acc[q];
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < kk; j++) {
-      float t = 0.f;
-      for (int ww = 0; ww < (int)(blockDim.x >> 5); ww++) t += sh[ww][j];
-      partials[(size_t)j * gridDim.x + blockIdx.x] = (double)t;
-    }
-    last = atomic_add_acq_rel(ticket, 1u) == gridDim.x - 1;
+  // a thread a value; the ticket's release covers the CTA's stores, which the
+  // barrier orders before it
+  if ((int)threadIdx.x < kk) {
+    float t = 0.f;
+    for (int ww = 0; ww < nw; ww++) t += sh[ww][threadIdx.x];
+    partials[(size_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
   }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomic_add_acq_rel(ticket + blockIdx.y, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
-  fold_partials(partials, kk, out);
-  __syncthreads();
-  if (threadIdx.x == 0) *ticket = 0u;
+  for (int q = wid; q < kk; q += nw) {
+    const double t = fold_row(partials + (size_t)(j0 + q) * gridDim.x, gridDim.x);
+    if (lane == 0) out[j0 + q] = t;
+  }
+  if (threadIdx.x == 0) ticket[blockIdx.y] = 0u;
 }
 
 __global__ void k_mx_cast64(const int* gate, int n, const float* __restrict__ a,
@@ -1390,6 +1744,49 @@ __global__ void k_mx_cast32(const int* gate, int n, const double* __restrict__ a
   if (gated_off(gate, 1)) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     b[i] = __double2float_rn(a[i]);
+}
+
+// One pass of a triangle stored by diagonals.
+static void tri_pass_dia(int W, const DiaOffsets& off, const float* val, const int* gate, int n,
+                         const float* dinv, const float* rhs, const float* in, const float* sc,
+                         float* vout, float* out, const float* scale2, float* out2,
+                         cudaStream_t s) {
+  const int gr = (n + kMixBlock * kTriRows - 1) / (kMixBlock * kTriRows);
+#define GP_TRI_DIA(WW)                                                                       \
+  case WW:                                                                                   \
+    (void)launch_pdl(k_mx_tri_dia<WW>, gr, kMixBlock, s, gate, n, off, val, dinv, rhs, in,   \
+                     sc, vout, out, scale2, out2);                                           \
+    return;
+  switch (W) {
+    GP_TRI_DIA(1)
+    GP_TRI_DIA(2)
+    GP_TRI_DIA(3)
+    GP_TRI_DIA(4)
+    GP_TRI_DIA(5)
+    GP_TRI_DIA(6)
+    GP_TRI_DIA(7)
+    GP_TRI_DIA(8)
+  }
+#undef GP_TRI_DIA
+}
+
+static void spmv_dia(const Mixed* M, const int* gate, const float* x, float* y, cudaStream_t s) {
+  const int n = M->n, gr = (n + kMixBlock * kMxSpmvRows - 1) / (kMixBlock * kMxSpmvRows);
+#define GP_SPMV_DIA(WW)                                                                      \
+  case WW:                                                                                   \
+    (void)launch_pdl(k_mx_spmv_dia<WW>, gr, kMixBlock, s, gate, n, M->aoff, M->adia, x, y);  \
+    return;
+  switch (M->aW) {
+    GP_SPMV_DIA(1)
+    GP_SPMV_DIA(2)
+    GP_SPMV_DIA(3)
+    GP_SPMV_DIA(4)
+    GP_SPMV_DIA(5)
+    GP_SPMV_DIA(6)
+    GP_SPMV_DIA(7)
+    GP_SPMV_DIA(8)
+  }
+#undef GP_SPMV_DIA
 }
 
 // One triangle pass: the ELL form when the triangle has at most 8 slots a row.
@@ -1424,6 +1821,9 @@ static void tri_pass(int W, const int* eci, const float* eval, const int* rp, co
 static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, double* x,
                        int tri_sweeps, int tri_block, cudaStream_t s) {
   const int n = M->n, m = M->m, g = mix_grid(n), gr = (n + kMixBlock - 1) / kMixBlock;
+  // CTAs of the 16-byte kernels, and who scales the new basis vector
+  const int g4 = mix_grid((n + 3) / 4);
+  const bool scaled_by_pass = tri_sweeps > 0 && tri_block == 0 && M->tri_dia;
   MixDev* st = M->st;
   const int* on = &st->pass_on;
   const int* act = &st->active;
@@ -1434,12 +1834,13 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
   GP_TRY(spmv(s, A, DRef::of(x), DRef::of(M->y)));
   k_mx_resid<<<red_grid(n), kRedBlock, 0, s>>>(n, b, M->y, M->r, slot, st);
   k_mx_v0<<<g, kMixBlock, 0, s>>>(n, M->r, st, M->V);
-  k_mx_mdot<<<mdot_grid(n), kMixBlock, 0, s>>>(on, n, nullptr, 1, M->V, M->partials, M->ticket,
-                                     &st->beta2);
+  float* parts = reinterpret_cast<float*>(M->partials);
+  k_mx_mdot<<<mx_mdot_grid(n, 1), kMdotBlock, 0, s>>>(on, n, M->ld, M->V, 1, M->V, parts,
+                                                      M->ticket, &st->beta2);
   k_mx_beta<<<1, 1, 0, s>>>(st, m);
   k_mx_scale<<<g, kMixBlock, 0, s>>>(n, M->V, M->V, st, 0);
   for (int j = 0; j < m; j++) {
-    float* vj = M->V + (size_t)j * n;
+    float* vj = M->V + (size_t)j * M->ld;
     float* zj = M->Z + (size_t)j * n;
     const int* perm_r = M->ident_r ? nullptr : pc->perm_r;
     const int* perm_c = M->ident_c ? nullptr : pc->perm_c;
@@ -1463,6 +1864,32 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
         launch_btri<true>(tu, M->bu.nblocks, M->bu.smem, act, yfin, xprev, lastp ? zj : xa,
                           lastp ? perm_c : nullptr, s);
         xprev = xa;
+        std::swap(xa, xb);
+      }
+    } else if (tri_sweeps > 0 && M->tri_dia) {
+      // as below, by diagonals; the basis vector is scaled by the first pass
+      // (the first vector already is) and D^-1 y written by the last L pass
+      const float* src = j ? M->w : vj;
+      const float* sc = j ? &st->inv_hn : nullptr;
+      float* ya = M->t1;
+      float* yb = M->t2;
+      const float* yin = src;
+      for (int k = 0; k < tri_sweeps; k++) {
+        const bool firstp = k == 0, lastp = k + 1 == tri_sweeps;
+        tri_pass_dia(M->lW, M->loff, M->lell_val, act, n, nullptr, firstp ? src : vj, yin,
+                     firstp ? sc : nullptr, firstp && j ? vj : nullptr, ya, M->udinv,
+                     lastp ? M->t4 : nullptr, s);
+        yin = ya;
+        std::swap(ya, yb);
+      }
+      float* xa = M->t3;
+      float* xb = M->t4;
+      const float* xin = M->t4;
+      for (int k = 0; k < tri_sweeps; k++) {
+        const bool lastp = k + 1 == tri_sweeps;
+        tri_pass_dia(M->uW, M->uoff, M->uell_val, act, n, M->udinv, yin, xin, nullptr, nullptr,
+                     lastp ? zj : xa, nullptr, nullptr, s);
+        xin = xa;
         std::swap(xa, xb);
       }
     } else if (tri_sweeps > 0) {
@@ -1498,19 +1925,21 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
     }
     // the step's kernels start while their predecessor drains (each waits
     // in pdl_wait() before reading it)
-    if (A->coff16)
+    if (M->aW)
+      spmv_dia(M, act, zj, M->w, s);
+    else if (A->coff16)
       GP_CUDA(launch_pdl(k_mx_spmv32<short>, gr, kMixBlock, s, act, n, A->rowptr,
                          (const short*)A->coff16, A->val32, zj, M->w));
     else
       GP_CUDA(launch_pdl(k_mx_spmv32<int>, gr, kMixBlock, s, act, n, A->rowptr,
                          (const int*)A->colind, A->val32, zj, M->w));
-    GP_CUDA(launch_pdl(k_mx_mdot, mdot_grid(n), kMixBlock, s, act, n, M->V, j + 1, M->w,
-                       M->partials, M->ticket, M->h_dev));
-    GP_CUDA(launch_pdl(k_mx_maxpy_norm, g, kMixBlock, s, act, n, M->V, j + 1, M->h_dev, M->w,
-                       M->partials, M->ticket, &st->hn2));
-    GP_CUDA(launch_pdl(k_mx_givens, 1, 32, s, st, M->h_dev, j, m));
-    if (j + 1 < m)
-      GP_CUDA(launch_pdl(k_mx_scale, g, kMixBlock, s, n, M->w, M->V + (size_t)(j + 1) * n, st, 1));
+    GP_CUDA(launch_pdl(k_mx_mdot, mx_mdot_grid(n, j + 1), kMdotBlock, s, act, n, M->ld, M->V,
+                       j + 1, M->w, parts, M->ticket, M->h_dev));
+    GP_CUDA(launch_pdl(k_mx_maxpy_step, g4 + 1, kMixBlock, s, n, M->ld, M->V, j + 1, M->h_dev, M->w,
+                       parts, M->ticket, st, m));
+    if (j + 1 < m && !scaled_by_pass)
+      GP_CUDA(launch_pdl(k_mx_scale, g, kMixBlock, s, n, M->w, M->V + (size_t)(j + 1) * M->ld, st,
+                         1));
   }
   k_mx_backsub<<<1, 32, 0, s>>>(st, m);
   k_mx_correct<<<g, kMixBlock, 0, s>>>(n, M->Z, st, x);
@@ -1537,6 +1966,7 @@ int mixed_solve_graph(Mixed* M, Csr* A, Pc* pc, const double* b, double* x,
   GP_CUDA(cudaStreamWaitEvent(s, ev, 0));
   GP_TRY(csr_make_val32(A, s));
   GP_TRY(mixed_factors(M, s));
+  GP_TRY(mixed_operator(M, A, s));
   if (o.tri_sweeps > 0 && o.tri_block != 0) GP_TRY(mixed_blocks(M, o.tri_block, s));
   double bb = 0.0;
   GP_TRY(vec_reduce(s, RED_NORM2SQ, n, b, nullptr, &bb));
