@@ -29,8 +29,14 @@
 //     signalling NaN marks "not yet"), indexed by the step;
 //   * a value on the face of a brick goes out to global memory, and the fetch
 //     warps of the neighbouring CTA poll it there, eight lanes a face line, a
-//     row each, and drop each into the reader's ring the moment it is in.  A brick that runs a hand-off behind its neighbour never waits on
-//     memory; on 128^3 the chain crosses 22 brick faces instead of 381 levels;
+//     row each, and drop each into the reader's ring the moment it is in.  A
+//     brick that runs a hand-off behind its neighbour never waits on memory; on
+//     128^3 the chain crosses 22 brick faces instead of 381 levels;
+//   * in 3-D up to 2 x 4 bricks are a thread-block cluster: a value on a face
+//     between two of them is stored straight into the reading tile's ring in the
+//     other CTA's shared memory (0.9 us a face where memory takes 2, under load);
+//     16 of those 22 faces are then of that kind.  A writer needs to know how far
+//     its reader is: a relay warp of the reader's CTA sends that on;
 //   * the faces have two copies, used in turn: a sweep reads and writes one
 //     and marks the other "not yet" for the next sweep, so nothing is cleared
 //     in between and the values of the rows themselves need no flags;
@@ -40,18 +46,18 @@
 //     by cp.async.  Loads into registers would not stay in flight over that
 //     many steps: a warp has six scoreboards, and a wait on one is a wait for
 //     every load that was put on it (a register ring measured 0.4 us a step);
-//   * bricks are handed out by a ticket in wavefront order (P + Q); a brick
-//     depends only on the bricks at P - 1 and Q - 1, which CTAs that are
+//   * bricks (clusters of them) are handed out by a ticket in wavefront order
+//     (P + Q); one depends only on those at P - 1 and Q - 1, which CTAs that are
 //     already running hold, so the sweep cannot deadlock whatever the number
 //     of resident CTAs.  Within a CTA a warp waits on lower steps only (for a
 //     value, or for a reader a whole ring behind), and every wait has a budget.
 //
-// What it measures (one sweep, GB300): 163-168 us on 128^3 (382 rows of chain;
-// 370 forward and 466 backward in the level-ordered form), 98 us on 256^2 (511
-// rows; 250 in the chunked form).  A step of a tile costs 0.15 us in 3-D forward
-// (three dependent FP64 operations are 0.093) and 0.2 with faces to read and
-// write; a brick face 1.3 us alone and up to 3 us with 128 CTAs at work, where
-// the latest of its 24 lines decides.
+// What it measures (one sweep, GB300): 122 us forward and 135 backward on 128^3
+// (382 rows of chain; 163-168 with every face through memory, 370 and 466 in the
+// level-ordered form), 92 and 100 on 96^3 (104 and 121), 92-98 on 256^2 (511 rows;
+// 250 in the chunked form).  Its time is 0.24 us a row of the chain in 3-D (three
+// dependent FP64 operations are 0.093, and a face's shuffle, poll and store lie
+// between), 0.9 us a face inside a cluster and 2 us one through memory.
 //
 // Every row is the reference's fold of its terms in ascending-column order,
 // with the same operations as k_ell_sweep: results are bit-identical to the
@@ -77,8 +83,8 @@ constexpr int kHalf = 8;             // steps between two looks at the neighbour
 constexpr int kStages = 2;           // groups in shared memory
 constexpr int kBrickPoll = 8;        // lanes that poll a face line, a row each (fewer for many lines)
 // threads: the tiles' warps and those that fetch
-constexpr int kBrickFetchMax = 8;
-constexpr int kBrickMaxThreads = 32 * (kBrickWarps + kBrickFetchMax);
+constexpr int kBrickFetchMax = 7;
+constexpr int kBrickMaxThreads = 32 * (kBrickWarps + kBrickFetchMax + 1);
 // Doubles of a ring step: Wq p-face lines, Wp q-face lines, a column that is
 // never empty and one that is never read (for lanes with no face)
 __host__ __device__ constexpr int brick_pitch(bool full, bool d3) {
@@ -98,6 +104,7 @@ struct BrickShape {
   int sw, sp, sq;
   int Wp, Wq, LW;    // lines of a tile; LW = Wp Wq of them stored, rounded up to even
   int CP, CQ;        // tiles of a brick
+  int XP, XQ;        // bricks of a cluster
   int ntP, ntQ, nbP, nbQ;
   int NS;            // steps stored a tile: nw + Wp + Wq - 2 and its phase, in whole groups
   int nwp;           // rows of a face line in memory
@@ -106,8 +113,8 @@ struct BrickShape {
 
 struct BrickArgs {
   BrickShape g;
-  int nbricks;
-  const int* border;      // [2 * nbricks]: (P, Q) of each brick in hand-out order
+  int nclusters;
+  const int* border;      // [2 * nclusters]: (P, Q) of each cluster in hand-out order
   const double* coef;     // [tile][step][columns by lane]: brick_store
   double* faces;          // [2][fsize]: the p faces, then the q faces
   long long fsize, qface;  // doubles of one copy; where its q faces start
@@ -119,6 +126,7 @@ struct BrickArgs {
   double om1;
   int write_out;
   int poll;               // fetching lanes a face line
+  int nf;                 // fetch warps
   unsigned* tickets;
   DevErr* err;
 };
@@ -231,11 +239,19 @@ __device__ __forceinline__ double ring_get(unsigned a) {
 __device__ __forceinline__ void ring_put(unsigned a, double v) {
   asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(a), "d"(v));
 }
+// CL: an address of cluster_addr, of this or another CTA of the cluster.
+template <bool CL>
 __device__ __forceinline__ void ring_put_if(bool p, unsigned a, double v) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
-      "@p st.volatile.shared.f64 [%0], %1;\n\t}" ::"r"(a),
-      "d"(v), "r"((unsigned)p));
+  if constexpr (CL)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+        "@p st.relaxed.cluster.shared::cluster.f64 [%0], %1;\n\t}" ::"r"(a),
+        "d"(v), "r"((unsigned)p));
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+        "@p st.volatile.shared.f64 [%0], %1;\n\t}" ::"r"(a),
+        "d"(v), "r"((unsigned)p));
 }
 // Whether a slot is still empty.  The high word decides: no double with the
 // flag's high word is ever computed (every one is a signalling NaN).
@@ -268,6 +284,55 @@ __device__ __forceinline__ void face_put_if(bool p, double* a, double v) {
       "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
       "@p st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(a),
       "d"(v), "r"((unsigned)p));
+}
+
+// ---- clusters
+__device__ __forceinline__ int cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile(
+      "barrier.cluster.arrive.release;\n\t"
+      "barrier.cluster.wait.acquire;" ::
+          : "memory");
+}
+// A shared-memory address in a CTA of the cluster.
+__device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+// The same shared-memory variable of another CTA of the cluster.
+template <typename T>
+__device__ __forceinline__ T* cluster_map(T* p, int rank) {
+  unsigned long long q;
+  asm volatile("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+  return reinterpret_cast<T*>(q);
+}
+
+// One lane of the relay warp: a tile's progress (prog) to the CTA that writes one
+// of its faces (dst, in that CTA), until the tile is at `end`.  The tile's own
+// warp publishes to its CTA only: a release that other SMs can see waits for the
+// warp's stores on their way to the L2, a thousand cycles every kHalf steps.
+__device__ void brick_relay(const int* prog, int* dst, int at, int end, bool on, DevErr* err) {
+  int spins = 0;
+  while (__any_sync(0xffffffffu, on)) {
+    if (on) {
+      int v;
+      asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(bk_smem(prog)) : "memory");
+      if (v != at) {
+        asm volatile("st.release.cluster.b32 [%0], %1;" ::"l"(dst), "r"(v) : "memory");
+        at = v;
+        spins = 0;
+        on = v < end;
+      } else if (++spins > kBrickSpin) {
+        if (atomicCAS(&err->code, 0, GP_ERR_TIMEOUT) == 0) err->where = 45;
+        on = false;
+      }
+    }
+  }
 }
 
 // One lane of a fetch warp: rows i, i + poll, ... of one face line into
@@ -319,7 +384,7 @@ __host__ __device__ __forceinline__ int brick_phase(const BrickShape& g, int P, 
 // place of a group, and no address within a group is computed.  The step's
 // instructions are what is left on the chain besides its FP64 operations, so
 // the loop is kept to about forty, nearly all without a branch.
-template <int MODE, bool FMA, bool FULL, bool D3>
+template <int MODE, bool FMA, bool FULL, bool D3, bool CL>
 __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* gate, int want,
                                                                      BrickArgs a, DRef inr,
                                                                      DRef outr) {
@@ -338,6 +403,8 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
   extern __shared__ __align__(16) double brick_smem[];
   __shared__ unsigned long long bars[kBrickWarps][kStages];
   __shared__ int prog[kBrickWarps];  // each tile's next step
+  // and of the tiles in the cluster's other CTAs that read its p and q faces
+  __shared__ int rprog[2][kBrickWarps];
   __shared__ int s_brick;
   const int nw = g.nw, Wp = g.Wp, Wq = g.Wq, LW = FULL ? 32 : g.LW, NS = g.NS;
   const int nt = g.CP * g.CQ, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -355,15 +422,43 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   const int tq = lane / Wp, tp = lane - tq * Wp;
   unsigned phases = 0;  // parity of each stage's next wait
+  const int XC = CL ? g.XP * g.XQ : 1, rank = CL ? cluster_rank() : 0;
+  const int xp = CL ? rank % g.XP : 0, xq = CL ? rank / g.XP : 0;
   for (;;) {
-    if (threadIdx.x == 0) s_brick = (int)atomicAdd(&a.tickets[0], 1u);
-    if (threadIdx.x < nt)
-      prog[threadIdx.x] = (threadIdx.x % g.CP * Wp + threadIdx.x / g.CP * Wq) / kHalf * kHalf;
-    __syncthreads();
+    // the last brick's reads and writes are over in the whole cluster
+    if constexpr (CL) cluster_sync();
+    if (threadIdx.x == 0 && rank == 0) {
+      const int b = (int)atomicAdd(&a.tickets[0], 1u);
+      s_brick = b;
+      for (int r = 1; r < XC; r++) *cluster_map(&s_brick, r) = b;
+    }
+    if (threadIdx.x < nt) {
+      const int cp = threadIdx.x % g.CP, cq = threadIdx.x / g.CP;
+      prog[threadIdx.x] = (cp * Wp + cq * Wq) / kHalf * kHalf;
+      if constexpr (CL) {
+        rprog[0][threadIdx.x] = cq * Wq / kHalf * kHalf;
+        rprog[1][threadIdx.x] = cp * Wp / kHalf * kHalf;
+      }
+    }
+    if constexpr (CL)
+      cluster_sync();
+    else
+      __syncthreads();
     const int b = s_brick;
-    if (b >= a.nbricks) break;
-    const int bP = a.border[2 * b], bQ = a.border[2 * b + 1];
-    if (warp >= nt) {
+    if (b >= a.nclusters) break;
+    const int bP = a.border[2 * b] * (CL ? g.XP : 1) + xp;
+    const int bQ = a.border[2 * b + 1] * (CL ? g.XQ : 1) + xq;
+    if (CL && warp >= nt + a.nf) {
+      // ---- relay: lane 2 w + d, tile w's progress to the writer of its p (d 0)
+      // or q face, where that is in the cluster
+      const int w = lane >> 1, d = lane & 1, cp = w % g.CP, cq = w / g.CP;
+      const bool on = w < nt && bP * g.CP + cp < g.ntP && bQ * g.CQ + cq < g.ntQ &&
+                      (d ? D3 && cq == 0 && xq > 0 : cp == 0 && xp > 0);
+      const int sb = (cp * Wp + cq * Wq) / kHalf * kHalf;
+      int* dst = cluster_map(&rprog[d][on ? (d ? (g.CQ - 1) * g.CP + cp : cq * g.CP + g.CP - 1) : 0],
+                             on ? rank - (d ? g.XP : 1) : rank);
+      brick_relay(&prog[on ? w : 0], dst, sb, sb + NS, on, a.err);
+    } else if (warp >= nt) {
       // ---- fetch: the brick's p faces (CQ Wq lines), then its q faces,
       // a.poll lanes a line
       const int np = g.CQ * Wq, lines = np + (D3 ? g.CP * Wp : 0);
@@ -377,7 +472,7 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
         w = cq * g.CP;
         t0 = c - 1;  // the step before row 0 of line (0, c)
         const int Q = bQ * g.CQ + cq, ql = Q * Wq + col;
-        act = bP > 0 && ql < g.nq;
+        act = bP > 0 && xp == 0 && bP < g.nbP && ql < g.nq;
         line = ((long long)bP * (g.ntQ * Wq) + ql) * g.nwp;
       } else if (c < lines) {
         const int cp = (c - np) / Wp, tl = c - np - cp * Wp;
@@ -385,7 +480,7 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
         t0 = c - np - 1;
         col = Wq + tl;
         const int P = bP * g.CP + cp, pl = P * Wp + tl;
-        act = bQ > 0 && pl < g.np;
+        act = bQ > 0 && xq == 0 && bQ < g.nbQ && pl < g.np;
         line = a.qface + ((long long)bQ * (g.ntP * Wp) + pl) * g.nwp;
       }
       brick_fetch<PITCH>(f_now + line, f_next + line, t % a.poll, a.poll,
@@ -446,17 +541,31 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
         const bool faces = __any_sync(full, fromp || fromq);
         const bool lastp = line && tp == Wp - 1 && P + 1 < g.ntP;
         const bool lastq = D3 && line && tq == Wq - 1 && Q + 1 < g.ntQ;
-        const bool outs = __any_sync(full, lastp || lastq);
         const bool ringp = cp + 1 < g.CP && P + 1 < g.ntP, ringq = cq + 1 < g.CQ && Q + 1 < g.ntQ;
-        const bool rings = ringp || ringq;
+        // faces that go into the ring of a tile in another CTA of the cluster
+        const bool clp = CL && !ringp && P + 1 < g.ntP && xp + 1 < g.XP;
+        const bool clq = CL && D3 && !ringq && Q + 1 < g.ntQ && xq + 1 < g.XQ;
+        const bool rings = ringp || ringq || clp || clq;
         // this lane's columns: read from, emptied, and the neighbouring tiles'
         const unsigned colp = ring + 8 * tq, colq = ring + 8 * (Wq + tp);
         const unsigned full_col = ring + 8 * (PITCH - 2), no_col = ring + 8 * (PITCH - 1);
         const unsigned rp = fromp ? colp : full_col, rq = fromq ? colq : full_col;
         const unsigned ep = fromp ? colp : no_col, eq = fromq ? colq : no_col;
-        const unsigned np = lastp && ringp ? colp + 8 * RING : no_col;
-        const unsigned nq = lastq && ringq ? colq + 8 * g.CP * RING : no_col;
-        const bool outp = lastp && !ringp, outq = lastq && !ringq;
+        // a neighbour in the cluster's next CTA is its tile (0, cq) or (cp, 0), and a
+        // brick's step t is step t - shp (shq) there, both multiples of kHalf
+        const int shp = CL && clp ? g.CP * Wp : 0, shq = CL && clq ? g.CQ * Wq : 0;
+        unsigned np = lastp && ringp ? colp + 8 * RING : no_col;
+        unsigned nq = lastq && ringq ? colq + 8 * g.CP * RING : no_col;
+        if constexpr (CL) {
+          np = cluster_addr(lastp && clp ? ring0 + 8 * (cq * g.CP * RING + tq) : np,
+                            lastp && clp ? rank + 1 : rank);
+          nq = cluster_addr(lastq && clq ? ring0 + 8 * (cp * RING + Wq + tp) : nq,
+                            lastq && clq ? rank + g.XP : rank);
+        }
+        // faces that go to memory, and the lanes that write them
+        const bool memp = P + 1 < g.ntP && !ringp && !clp;
+        const bool memq = D3 && Q + 1 < g.ntQ && !ringq && !clq;
+        const bool outp = lastp && memp, outq = lastq && memq;
         const int nwop = outp ? nw : 0, nwoq = outq ? nw : 0;
         // face lines this lane writes (row -off at the pointer)
         double* fop = f_now + ((long long)(bP + 1) * (g.ntQ * Wq) + ql) * g.nwp - (outp ? off : 0);
@@ -497,9 +606,15 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
             return r;
           };
           BrickRow r = take(0);
-          // with_faces: some lane reads face values; with_out: some lane's are read
-          auto steps = [&](auto with_faces, auto with_out) {
-            constexpr bool FACES = decltype(with_faces)::value, OUTS = decltype(with_out)::value;
+          // with_faces: some lane reads face values.  out: the last lines' values go
+          // to rings (1), to the faces in memory (2), or both.  In 3-D, where a
+          // tile may have one of each, all take the same code: four forms with
+          // one store a direction cost 25% on 128^3, a fetch of instructions for
+          // each of the SM's warps.  In 2-D the tiles of a row differ less, and
+          // one store saves 6% on 256^2 (210 to 198 us a pair of sweeps).
+          auto steps = [&](auto with_faces, auto out) {
+            constexpr bool FACES = decltype(with_faces)::value;
+            constexpr int OUT = decltype(out)::value;
             // unrolled over half a group: the code has to stay in the
             // instruction cache of the sub-partition that runs it
 #pragma unroll 1
@@ -510,12 +625,16 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
                   if (lane == 0) publish(&prog[warp], sb + s0 + u0);
                 }
               }
-              if constexpr (OUTS) {
+              if constexpr (OUT & 1) {
                 // room in the rings of the neighbouring tiles for the next values
                 if (rings) {
                   for (int spins = 0;; spins++) {
-                    const int at_p = ringp ? *(volatile int*)&prog[warp + 1] : INT_MAX / 2;
-                    const int at_q = ringq ? *(volatile int*)&prog[warp + g.CP] : INT_MAX / 2;
+                    const int at_p = ringp ? *(volatile int*)&prog[warp + 1]
+                                     : clp ? *(volatile int*)&rprog[0][warp] + shp
+                                           : INT_MAX / 2;
+                    const int at_q = ringq ? *(volatile int*)&prog[warp + g.CP]
+                                     : clq ? *(volatile int*)&rprog[1][warp] + shq
+                                           : INT_MAX / 2;
                     if (sb + s0 + u0 + kHalf < min(at_p, at_q) + kBrickRing) break;
                     if (spins > kBrickSpin || ((spins & 4095) == 4095 && brick_failed(a.err))) {
                       if (lane == 0 && atomicCAS(&a.err->code, 0, GP_ERR_TIMEOUT) == 0)
@@ -526,6 +645,10 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
                 }
               }
               const unsigned slot = 8 * (((sb + s0 + u0) & (kBrickRing - 1)) * PITCH);
+              const unsigned wp = np + (CL ? 8 * (((sb + s0 + u0 - shp) & (kBrickRing - 1)) * PITCH)
+                                           : slot);
+              const unsigned wq = nq + (CL ? 8 * (((sb + s0 + u0 - shq) & (kBrickRing - 1)) * PITCH)
+                                           : slot);
 #pragma unroll
               for (int h = 0; h < kHalf; h++) {
               const int u = u0 + h, w = s0 - off + u;
@@ -583,9 +706,11 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
                 y = sum;
               prev = act ? y : prev;
               // the values other tiles wait on go out first
-              if constexpr (OUTS) {
-                ring_put_if(act, np + slot + h * (8 * PITCH), y);
-                if constexpr (D3) ring_put_if(act, nq + slot + h * (8 * PITCH), y);
+              if constexpr (OUT & 1) {
+                ring_put_if<CL>(act, wp + h * (8 * PITCH), y);
+                if constexpr (D3) ring_put_if<CL>(act, wq + h * (8 * PITCH), y);
+              }
+              if constexpr (OUT & 2) {
                 face_put_if((unsigned)w < (unsigned)nwop, fop + h, y);
                 if constexpr (D3) face_put_if((unsigned)w < (unsigned)nwoq, foq + h, y);
               }
@@ -609,21 +734,30 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
               }
             }
           };
-          if (faces)
-            steps(std::true_type{}, std::true_type{});
-          else if (outs)
-            steps(std::false_type{}, std::true_type{});
-          else
-            steps(std::false_type{}, std::false_type{});
+          using std::integral_constant;
+          if constexpr (D3) {
+            steps(std::true_type{}, integral_constant<int, 3>{});
+          } else if (faces) {
+            if (memp)
+              steps(std::true_type{}, integral_constant<int, 2>{});
+            else
+              steps(std::true_type{}, integral_constant<int, 1>{});
+          } else if (memp) {
+            steps(std::false_type{}, integral_constant<int, 2>{});
+          } else if (rings) {
+            steps(std::false_type{}, integral_constant<int, 1>{});
+          } else {
+            steps(std::false_type{}, integral_constant<int, 0>{});
+          }
           __syncwarp();  // the stage is read, the ring's slots are free
           fill(s0 / kGroup + kStages, si);
           si = si + 1 == kStages ? 0 : si + 1;
-          if (faces && lane == 0) publish(&prog[warp], sb + s0 + kGroup);
+          if ((D3 || faces) && lane == 0) publish(&prog[warp], sb + s0 + kGroup);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
       }
     }
-    __syncthreads();
+    if constexpr (!CL) __syncthreads();
   }
   if (threadIdx.x == 0 && atomic_add_acq_rel(&a.tickets[1], 1u) == gridDim.x - 1) {
     a.tickets[0] = 0u;
@@ -762,16 +896,33 @@ static bool brick_detect(int n, bool forward, const std::vector<int>& dptr,
 }
 
 // Modelled duration of one brick sweep (us): the chain of nx + ny + nz - 2
-// rows at a step each plus a hand-off a brick face, or the bricks' steps over
-// the SMs, whichever is longer.  The other forms take at least 1.25 us a
-// dependency level in level order, or 0.4 us a level and the staging of a
-// chunk (their own model, gp_sweep.cu).
-constexpr double kBrickStep = 0.22, kBrickHandoff = 2.0, kBrickStart = 4.0;
+// rows at a step each plus a hand-off a brick face (less for one inside a
+// cluster), or the bricks' steps over the SMs, whichever is longer.  The other
+// forms take at least 1.25 us a dependency level in level order, or 0.4 us a
+// level and the staging of a chunk (their own model, gp_sweep.cu).
+constexpr double kBrickStep = 0.22, kBrickHandoff = 2.0, kBrickNear = 0.9, kBrickStart = 4.0;
 static double other_model_us(int nlevels) { return std::min(1.25 * nlevels, 20.0 + 0.4 * nlevels); }
 static double brick_model_us(const BrickShape& g) {
-  const double chain = (g.nw + g.np + g.nq - 2) * kBrickStep + (g.nbP + g.nbQ - 2) * kBrickHandoff;
+  const int ncP = (g.nbP + g.XP - 1) / g.XP, ncQ = (g.nbQ + g.XQ - 1) / g.XQ;
+  const int far = ncP + ncQ - 2, near = g.nbP + g.nbQ - 2 - far;
+  const double chain =
+      (g.nw + g.np + g.nq - 2) * kBrickStep + far * kBrickHandoff + near * kBrickNear;
   const double rounds = std::ceil((double)g.nbP * g.nbQ / std::max(1, num_sms()));
   return kBrickStart + std::max(chain, rounds * (g.NS * kBrickStep + kBrickStart));
+}
+
+// Bricks of a cluster: 2 x 4 of those of whole 3-D tiles (whose lines across are
+// multiples of kHalf, as the rings' shift between CTAs needs), eight being the
+// portable limit.  ILU applies, us: 128^3 286 (2 x 2: 308, 4 x 2: 291, none: 365),
+// 96^3 211 (221, 222, 235), 81^3 208 (210, 212, 223), 160^3, where the bricks take
+// two rounds, 408 (410, -, 436).  In 2-D a cluster saves one or two faces of 2 us
+// and its stores cost as much (256^2: 223 against 213).  The layout of the faces
+// depends on it, so it is a function of the shape alone.
+static void brick_cluster(BrickShape& g) {
+  g.XP = g.XQ = 1;
+  if (!g.d3 || g.Wp != 8 || g.Wq != 4 || g.CP != 2 || g.CQ != 2) return;
+  g.XP = std::min(2, g.nbP);
+  g.XQ = std::min(4, g.nbQ);
 }
 
 static BrickShape brick_shape(const int* dims, bool bwd, int lines) {
@@ -812,6 +963,7 @@ static BrickShape brick_shape(const int* dims, bool bwd, int lines) {
   g.ntQ = (g.nq + g.Wq - 1) / g.Wq;
   g.nbP = (g.ntP + g.CP - 1) / g.CP;
   g.nbQ = (g.ntQ + g.CQ - 1) / g.CQ;
+  brick_cluster(g);
   int phase = 0;  // the largest of any tile of a brick
   for (int cp = 0; cp < g.CP; cp++)
     for (int cq = 0; cq < g.CQ; cq++)
@@ -835,20 +987,38 @@ static void brick_launch(int grid, int threads, const int* gate, int want, const
   const bool full = g.LW == 32 && g.Wp + g.Wq <= (g.d3 ? 14 : 33);
   const size_t smem = (size_t)g.CP * g.CQ * 8 *
                       (brick_ring(full && f, g.d3) + kStages * kGroup * brick_cols(MODE, g.d3) * g.LW);
-  auto k = g.d3 ? (!f     ? k_brick_sweep<MODE, false, false, true>
-                   : full ? k_brick_sweep<MODE, true, true, true>
-                          : k_brick_sweep<MODE, true, false, true>)
-                : (!f     ? k_brick_sweep<MODE, false, false, false>
-                   : full ? k_brick_sweep<MODE, true, true, false>
-                          : k_brick_sweep<MODE, true, false, false>);
-  k<<<grid, threads, smem, s>>>(gate, want, a, in, out);
+  const bool cl = g.XP * g.XQ > 1;  // then the tiles are full ones (brick_cluster)
+  auto k = cl       ? (f ? k_brick_sweep<MODE, true, true, true, true>
+                         : k_brick_sweep<MODE, false, false, true, true>)
+           : g.d3 ? (!f     ? k_brick_sweep<MODE, false, false, true, false>
+                     : full ? k_brick_sweep<MODE, true, true, true, false>
+                            : k_brick_sweep<MODE, true, false, true, false>)
+                  : (!f     ? k_brick_sweep<MODE, false, false, false, false>
+                     : full ? k_brick_sweep<MODE, true, true, false, false>
+                            : k_brick_sweep<MODE, true, false, false, false>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = g.XP * g.XQ;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = g.XP * g.XQ > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, gate, want, a, in, out);
 }
 
 template <int MODE>
 static void brick_attrs() {
-  for (auto k : {k_brick_sweep<MODE, true, true, true>, k_brick_sweep<MODE, true, false, true>,
-                 k_brick_sweep<MODE, false, false, true>, k_brick_sweep<MODE, true, true, false>,
-                 k_brick_sweep<MODE, true, false, false>, k_brick_sweep<MODE, false, false, false>})
+  for (auto k :
+       {k_brick_sweep<MODE, true, true, true, true>, k_brick_sweep<MODE, false, false, true, true>,
+        k_brick_sweep<MODE, true, true, true, false>, k_brick_sweep<MODE, true, false, true, false>,
+        k_brick_sweep<MODE, false, false, true, false>,
+        k_brick_sweep<MODE, true, true, false, false>,
+        k_brick_sweep<MODE, true, false, false, false>,
+        k_brick_sweep<MODE, false, false, false, false>})
     cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kBrickSmemMax);
 }
@@ -889,11 +1059,12 @@ static int brick_layout(EllSweep& e, int mode, const int* dims, int lines,
   e.W = 3;
   e.bcols = brick_coefs(mode, g.d3);
   e.nbricks = g.nbP * g.nbQ;
-  // hand-out order: wavefronts P + Q, then Q
+  // hand-out order of the clusters: wavefronts P + Q, then Q
+  const int ncP = (g.nbP + g.XP - 1) / g.XP, ncQ = (g.nbQ + g.XQ - 1) / g.XQ;
   std::vector<int> border;
-  border.reserve(2 * (size_t)e.nbricks);
-  for (int w = 0; w <= g.nbP + g.nbQ - 2; w++)
-    for (int Q = std::max(0, w - (g.nbP - 1)); Q <= std::min(w, g.nbQ - 1); Q++) {
+  border.reserve(2 * (size_t)ncP * ncQ);
+  for (int w = 0; w <= ncP + ncQ - 2; w++)
+    for (int Q = std::max(0, w - (ncP - 1)); Q <= std::min(w, ncQ - 1); Q++) {
       border.push_back(w - Q);
       border.push_back(Q);
     }
@@ -977,7 +1148,8 @@ int brick_sweep(int mode, const EllSweep& e, const int* gate, int want, DRef in,
   if (e.n == 0) return GP_OK;
   BrickArgs a;
   a.g = shape_of(e);
-  a.nbricks = e.nbricks;
+  const int xc = a.g.XP * a.g.XQ;
+  a.nclusters = ((a.g.nbP + a.g.XP - 1) / a.g.XP) * ((a.g.nbQ + a.g.XQ - 1) / a.g.XQ);
   a.border = e.border;
   a.coef = e.coef;
   a.faces = e.faces;
@@ -997,10 +1169,11 @@ int brick_sweep(int mode, const EllSweep& e, const int* gate, int want, DRef in,
   const int cols = a.g.CQ * a.g.Wq + (a.g.d3 ? a.g.CP * a.g.Wp : 0);
   a.poll = kBrickPoll;
   while (a.poll > 1 && cols * a.poll > 32 * kBrickFetchMax) a.poll /= 2;
-  const int nf = e.nbricks > 1 ? (cols * a.poll + 31) / 32 : 0;
-  const int threads = 32 * (a.g.CP * a.g.CQ + nf);
-  int grid = std::min(e.nbricks, num_sms() * 2);
+  a.nf = a.nclusters > 1 ? (cols * a.poll + 31) / 32 : 0;
+  const int threads = 32 * (a.g.CP * a.g.CQ + a.nf + (xc > 1 ? 1 : 0));
+  int grid = std::min(a.nclusters * xc, num_sms() * 2);
   if (brick_tuning().max_ctas > 0) grid = std::min(grid, brick_tuning().max_ctas);
+  grid = std::max(grid / xc, 1) * xc;
 #define BRICK_LAUNCH(M) \
   case M: brick_launch<M>(grid, threads, gate, want, a, in, out, s); break;
   switch (mode) {

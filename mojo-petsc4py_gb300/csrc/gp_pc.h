@@ -78,7 +78,7 @@ struct EllSweep {
   bool brick = false, bwd = false;
   int gx = 0, gy = 0, gz = 0, BJ = 0, BK = 0, nbricks = 0, npos = 0, bcols = 0;
   int blines = 0;             // forced lines of a brick (0: chosen)
-  int* border = nullptr;      // [2 * nbricks]: place of each brick in hand-out order
+  int* border = nullptr;      // place (P, Q) of each cluster of bricks in hand-out order
   double* faces = nullptr;    // two copies of the bricks' face values, used in turn
   long long fsize = 0, qface = 0;
   int* parity = nullptr;      // which copy the next sweep uses (in faces' block)
