@@ -1483,6 +1483,18 @@ __device__ void mx_givens(MixDev* st, double hn2, int j, int m) {
   if (!(hn > 0.0) || fabs(gn) <= tol || j + 1 == m) st->active = 0;
 }
 
+// Four values of a basis row at their last use in a step: evicted from the L2
+// before the factor and the operator, which every step reads again (with this the
+// solve at 96^3 takes 10.1 ms, without 10.7; with the dots' reads so, too, 10.4:
+// this second reading then misses more).
+__device__ __forceinline__ float4 ld_basis(const float* p, int i, uint64_t pol) {
+  float4 v;
+  asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p + 4 * (size_t)i), "l"(pol));
+  return v;
+}
+
 __device__ __forceinline__ void fma4(float4& v, float c, const float4& t) {
   v.x = __fmaf_rn(c, t.x, v.x);
   v.y = __fmaf_rn(c, t.y, v.y);
@@ -1545,6 +1557,7 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_step(int n, size_t ld,
     __syncthreads();
     const int n4 = n >> 2;
     float4* w4 = reinterpret_cast<float4*>(w);
+    const uint64_t pol = l2_evict_first();
     for (int i = n4 - 1 - (int)((blockIdx.x - 1) * kMixBlock + threadIdx.x); i >= 0;
          i -= nb * kMixBlock) {
       float4 v = w4[i];
@@ -1552,7 +1565,7 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_step(int n, size_t ld,
         float4 t[8];
 #pragma unroll
         for (int q = 0; q < 8; q++)
-          if (j + q < k) t[q] = reinterpret_cast<const float4*>(V + (j + q) * ld)[i];
+          if (j + q < k) t[q] = ld_basis(V + (j + q) * ld, i, pol);
 #pragma unroll
         for (int q = 0; q < 8; q++)
           if (j + q < k) fma4(v, -hs[j + q], t[q]);
