@@ -54,7 +54,7 @@
 //
 // What it measures (one sweep, GB300): 122 us forward and 135 backward on 128^3
 // (382 rows of chain; 163-168 with every face through memory, 370 and 466 in the
-// level-ordered form), 92 and 100 on 96^3 (104 and 121), 92-98 on 256^2 (511 rows;
+// level-ordered form), 92 and 100 on 96^3 (110 and 121), 83 and 94 on 256^2 (511 rows;
 // 250 in the chunked form).  Its time is 0.24 us a row of the chain in 3-D (three
 // dependent FP64 operations are 0.093, and a face's shuffle, poll and store lie
 // between), 0.9 us a face inside a cluster and 2 us one through memory.
