@@ -278,6 +278,24 @@ __device__ __forceinline__ void stage_get2(unsigned a, double& x, double& y) {
 __device__ __forceinline__ void publish(int* p, int step) {
   asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(bk_smem(p)), "r"(step) : "memory");
 }
+// A tile's progress, read by a writer of its ring: an acquire, paired with the
+// release of the publishing warp (or of the relay, for a tile in another CTA of
+// the cluster), so that the slots' emptying comes before the values that the
+// writer stores into them next.  A plain read and the branch on it would promise
+// no such order.
+__device__ __forceinline__ int progress(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(bk_smem(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ int progress_cluster(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cluster.shared::cta.b32 %0, [%1];"
+               : "=r"(v)
+               : "r"(bk_smem(p))
+               : "memory");
+  return v;
+}
 // A face value to the other bricks.
 __device__ __forceinline__ void face_put_if(bool p, double* a, double v) {
   asm volatile(
@@ -320,8 +338,7 @@ __device__ void brick_relay(const int* prog, int* dst, int at, int end, bool on,
   int spins = 0;
   while (__any_sync(0xffffffffu, on)) {
     if (on) {
-      int v;
-      asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(bk_smem(prog)) : "memory");
+      const int v = progress(prog);
       if (v != at) {
         asm volatile("st.release.cluster.b32 [%0], %1;" ::"l"(dst), "r"(v) : "memory");
         at = v;
@@ -341,13 +358,13 @@ __device__ void brick_relay(const int* prog, int* dst, int at, int end, bool on,
 // line's other copy is emptied for the next sweep.
 template <int PITCH>
 __device__ void brick_fetch(const double* line, double* next, int i, int poll, int nw, unsigned ring,
-                            int t0, volatile const int* prog, bool act, DevErr* err) {
+                            int t0, const int* prog, bool act, DevErr* err) {
   int spins = 0;
   if (!act) i = nw;
   while (__any_sync(0xffffffffu, i < nw)) {
     if (i < nw) {
       unsigned long long v = kPending;
-      const bool room = i + t0 < *prog + kBrickRing - 1;
+      const bool room = i + t0 < progress(prog) + kBrickRing - 1;
       if (room) v = ld_relaxed_bits(line + i);
       if (++spins > kBrickSpin || ((spins & 1023) == 1023 && brick_failed(err))) {
         // never arrived (or the reader never moved): record it and hand on a
@@ -629,11 +646,11 @@ __global__ void __launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep(const int* 
                 // room in the rings of the neighbouring tiles for the next values
                 if (rings) {
                   for (int spins = 0;; spins++) {
-                    const int at_p = ringp ? *(volatile int*)&prog[warp + 1]
-                                     : clp ? *(volatile int*)&rprog[0][warp] + shp
+                    const int at_p = ringp ? progress(&prog[warp + 1])
+                                     : clp ? progress_cluster(&rprog[0][warp]) + shp
                                            : INT_MAX / 2;
-                    const int at_q = ringq ? *(volatile int*)&prog[warp + g.CP]
-                                     : clq ? *(volatile int*)&rprog[1][warp] + shq
+                    const int at_q = ringq ? progress(&prog[warp + g.CP])
+                                     : clq ? progress_cluster(&rprog[1][warp]) + shq
                                            : INT_MAX / 2;
                     if (sb + s0 + u0 + kHalf < min(at_p, at_q) + kBrickRing) break;
                     if (spins > kBrickSpin || ((spins & 4095) == 4095 && brick_failed(a.err))) {

@@ -1,0 +1,27 @@
+"""Rules of the native sources whose breach no run shows reliably: read from the
+source files (no GPU)."""
+import pathlib
+import re
+
+CSRC = pathlib.Path(__file__).resolve().parents[1] / "mojo-petsc4py_gb300" / "csrc"
+
+
+def _code(name):
+    """A source file without its comments."""
+    return re.sub(r"/\*.*?\*/|//[^\n]*", "", (CSRC / name).read_text(), flags=re.S)
+
+
+def test_ring_writers_read_progress_by_acquire():
+    """k_brick_sweep: a writer stores into slots of another tile's ring once that
+    tile has published that it emptied them, so it reads the progress words
+    (prog, rprog) by acquire, never by a plain or volatile load."""
+    code = _code("gp_brick.cu")
+    assert not re.search(r"volatile[^;{]*\bprog\b|volatile[^;{]*\brprog\b", code)
+    body = code[code.index("__launch_bounds__(kBrickMaxThreads, 1) k_brick_sweep"):]
+    body = body[:body.index("__global__")]
+    for word, scope in (("prog", "progress"), ("rprog", "progress_cluster")):
+        uses = re.findall(r"(\w*)\(?&" + word + r"\[", body)
+        assert uses and set(uses) <= {scope, "publish", "cluster_map", "brick_relay", ""}
+        assert scope in uses
+    assert re.search(r"ld\.acquire\.cta\.shared\.b32", code)
+    assert re.search(r"ld\.acquire\.cluster\.shared::cta\.b32", code)
