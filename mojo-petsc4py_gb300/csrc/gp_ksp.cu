@@ -1577,6 +1577,9 @@ static int ensure(Ksp* k, int n, bool* moved) {
   return GP_OK;
 }
 
+// Vector `i` of the workspace: its offset can pass 2^31 elements.
+static double* work_vec(const Ksp* k, int i) { return k->work + (size_t)i * k->n; }
+
 namespace {
 
 // launch helpers bound to one solve
@@ -1697,7 +1700,7 @@ static int cg_body(const Run& r, double* x) {
   const int n = r.n;
   double* R = k->work;
   double* Z = k->work + n;
-  double* P = k->work + 2 * n;
+  double* P = work_vec(k, 2);
   double* W = Z;  // the reference's W = Z aliasing
   KspState* st = k->st;
   const int* on = r.G(G_ON);
@@ -1774,7 +1777,7 @@ static int cg_body_fused(const Run& r, double* x) {
   const int n = r.n;
   double* R = k->work;
   double* Z = k->work + n;
-  double* P = k->work + 2 * n;
+  double* P = work_vec(k, 2);
   double* W = Z;  // the reference's W = Z aliasing
   const Csr* A = r.A;
   GP_CUDA(launch_pdl(arith_mode() == kFma ? k_cgf_p<true> : k_cgf_p<false>, r.grid(), 256, r.s,
@@ -1825,9 +1828,8 @@ static int bcgs_prologue(const Run& r, const double* b, double* x) {
   Ksp* k = r.k;
   const KspOptions& o = k->opt;
   const int n = r.n;
-  double* w = k->work;
-  DRef R = DRef::of(w), RP = DRef::of(w + n), V = DRef::of(w + 2 * n), T = DRef::of(w + 3 * n);
-  DRef P = DRef::of(w + 5 * n), GUESS = DRef::of(w + 6 * n);
+  auto vec = [&](int i) { return DRef::of(work_vec(k, i)); };
+  DRef R = vec(0), RP = vec(1), V = vec(2), T = vec(3), P = vec(5), GUESS = vec(6);
   GP_TRY(r.initial_residual(o.pc_side, o.guess_zero, DRef::of(x), V, T, R, DRef::of(b)));
   if (o.pc_side == 1 && !o.guess_zero) {
     GP_TRY(r.copy(nullptr, DRef::of(x), GUESS));
@@ -1852,9 +1854,8 @@ static int bcgs_prologue(const Run& r, const double* b, double* x) {
 static int bcgs_body_fused(const Run& r, double* x) {
   Ksp* k = r.k;
   const int n = r.n, side = k->opt.pc_side;
-  double* w = k->work;
-  double *R = w, *RP = w + n, *V = w + 2 * (size_t)n, *T = w + 3 * (size_t)n,
-         *S = w + 4 * (size_t)n, *P = w + 5 * (size_t)n;
+  double *R = work_vec(k, 0), *RP = work_vec(k, 1), *V = work_vec(k, 2), *T = work_vec(k, 3),
+         *S = work_vec(k, 4), *P = work_vec(k, 5);
   KspState* st = k->st;
   const int* on = r.G(G_ON);
   const bool f = arith_mode() == kFma;
@@ -1881,9 +1882,8 @@ static int bcgs_body_fused(const Run& r, double* x) {
 static int bcgs_body(const Run& r, double* x) {
   Ksp* k = r.k;
   const int n = r.n, side = k->opt.pc_side;
-  double* w = k->work;
-  DRef R = DRef::of(w), RP = DRef::of(w + n), V = DRef::of(w + 2 * n), T = DRef::of(w + 3 * n);
-  DRef S = DRef::of(w + 4 * n), P = DRef::of(w + 5 * n), X = DRef::of(x);
+  auto vec = [&](int i) { return DRef::of(work_vec(k, i)); };
+  DRef R = vec(0), RP = vec(1), V = vec(2), T = vec(3), S = vec(4), P = vec(5), X = DRef::of(x);
   KspState* st = k->st;
   const int* on = r.G(G_ON);
   GP_TRY(r.red<D_DOT>(on, R, RP, r.S(&KspState::rho), nullptr));
@@ -1918,8 +1918,7 @@ static int bcgs_epilogue(const Run& r, double* x) {
   Ksp* k = r.k;
   const KspOptions& o = k->opt;
   const int n = r.n;
-  double* w = k->work;
-  DRef T = DRef::of(w + 3 * n), GUESS = DRef::of(w + 6 * n), X = DRef::of(x);
+  DRef T = DRef::of(work_vec(k, 3)), GUESS = DRef::of(work_vec(k, 6)), X = DRef::of(x);
   // KSPUnwindPreconditioner (src/ksp.mojo:211-218)
   if (o.pc_side == 1) {
     GP_TRY(r.pcapply(nullptr, X, T));

@@ -25,3 +25,13 @@ def test_ring_writers_read_progress_by_acquire():
         assert scope in uses
     assert re.search(r"ld\.acquire\.cta\.shared\.b32", code)
     assert re.search(r"ld\.acquire\.cluster\.shared::cta\.b32", code)
+
+
+def test_workspace_offsets_are_64_bit():
+    """A solver's workspace is up to seven vectors of n < 2^31 doubles: an offset
+    of several vectors is never a product of 32-bit integers."""
+    for path in sorted(CSRC.glob("gp_*.cu")):
+        code = _code(path.name)
+        assert not re.findall(r"[+]\s*\(?[0-9]\s*\*\s*n\b", code), path.name
+    code = _code("gp_ksp.cu")
+    assert "return k->work + (size_t)i * k->n;" in code
