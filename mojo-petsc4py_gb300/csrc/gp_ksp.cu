@@ -1593,6 +1593,7 @@ struct Run {
   // 0 none, 1 host-driven trip bookkeeping, 2 also the graph condition
   int loop = 0;
   cudaGraphConditionalHandle cond = 0;
+  int steps = 1;  // Arnoldi steps a trip: gm_steps in the graph, one from the host
   const int* G(int idx) const { return &k->st->g[idx]; }
   double* S(double KspState::*f) const { return &(k->st->*f); }
   int grid() const { return vgrid(n); }
@@ -1827,7 +1828,6 @@ static bool bcgs_fused_ok() { return arith_mode() != kOrdered; }
 static int bcgs_prologue(const Run& r, const double* b, double* x) {
   Ksp* k = r.k;
   const KspOptions& o = k->opt;
-  const int n = r.n;
   auto vec = [&](int i) { return DRef::of(work_vec(k, i)); };
   DRef R = vec(0), RP = vec(1), V = vec(2), T = vec(3), P = vec(5), GUESS = vec(6);
   GP_TRY(r.initial_residual(o.pc_side, o.guess_zero, DRef::of(x), V, T, R, DRef::of(b)));
@@ -1975,7 +1975,7 @@ static bool gm_fused(const Run& r) {
   return arith_mode() != kOrdered && !r.k->opt.orthog && r.k->opt.cgstype == 0;
 }
 
-// Arnoldi steps per loop trip.  The trip's other kernels (a restart before the
+// Arnoldi steps per trip of the graph's loop.  The trip's other kernels (a restart before the
 // steps and the solution update after them, gated off in most trips) and the
 // loop's own node cost about 30 us a trip at any size, an unused step about 10;
 // as many as divide the restart, up to 10.  The modified Gram-Schmidt's steps
@@ -2060,7 +2060,7 @@ static int gmres_body(const Run& r, const double* b, double* x) {
   GP_CHECK_LAUNCH();
   // ---- Arnoldi steps
   DRef vit = DRef::at(&st->vv_it), vit1 = DRef::at(&st->vv_it1);
-  for (int step = gm_steps(r); step > 0; step--) {
+  for (int step = r.steps; step > 0; step--) {
     GP_TRY(r.apply_ba(r.G(1), side, vit, vit1, TMATOP));
     if (gm_fused(r)) {
       GP_TRY(cgs_dots(r, 1));
@@ -2133,7 +2133,7 @@ static int fgmres_body(const Run& r, const double* b, double* x) {
   GP_CHECK_LAUNCH();
   // ---- flexible Arnoldi steps
   DRef vit = DRef::at(&st->vv_it), vit1 = DRef::at(&st->vv_it1), pit = DRef::at(&st->pv_it);
-  for (int step = gm_steps(r); step > 0; step--) {
+  for (int step = r.steps; step > 0; step--) {
     GP_TRY(r.pcapply(r.G(1), vit, pit));
     GP_TRY(r.matmult(r.G(1), pit, vit1));
     if (gm_fused(r)) {
@@ -2226,6 +2226,8 @@ static int body_unroll(const Run& r) {
 
 // GPETSC_KSP_GRAPH=0: drive the loop from the host (same kernels, launched on
 // the stream, convergence polled every kEagerPoll trips) instead of one graph.
+// One Arnoldi step a trip: a launch from the host costs as much idle as not
+// (GMRES+Jacobi on 32^2, one step: 690 us; 1980 with the graph's ten a trip).
 static bool eager_mode() {
   static bool v = [] {
     const char* e = std::getenv("GPETSC_KSP_GRAPH");
@@ -2295,6 +2297,7 @@ static int capture(const Run& r, const double* b, double* x) {
     } else {
       Run rb = r;
       rb.s = k->stream2;
+      rb.steps = gm_steps(r);
       const bool own = body_ends_trip(r);
       // several gated copies of the body per conditional trip amortise the
       // conditional node's re-launch; copies after convergence are no-ops

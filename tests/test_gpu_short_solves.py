@@ -1,0 +1,48 @@
+"""Solves that end after a few iterations run few idle kernels: the steps and loop
+copies that a trip holds for longer solves are not launched, or not all, once a
+solve has ended.  Counted from the launch accounting; the host-driven form, which
+has none, by its time against a long solve's."""
+import time
+
+import numpy as np
+import pytest
+
+from mojopetsc4py import PETSc, _lib, gallery
+
+pytestmark = [pytest.mark.gpu, pytest.mark.fma]
+
+
+def _solver(kt, pt, its, form="graph"):
+    ip, ix, v = gallery.laplacian_2d(32)
+    n = len(ip) - 1
+    A = PETSc.Mat().createSeqAIJ((n, n))
+    A.setValuesCSR(ip, ix, v)
+    A.assemble()
+    ksp = PETSc.KSP().create()
+    pc = PETSc.PC().create()
+    pc.setType(pt)
+    ksp.setPC(pc)
+    ksp.setType(kt)
+    ksp.setOperators(A)
+    ksp.setTolerances(rtol=1e-14, atol=1e-50, divtol=1e30, max_it=its)
+    ksp.setLaunchForm(form)
+    b = PETSc.Vec().createWithArray(np.random.default_rng(0).uniform(-1.0, 1.0, n))
+    x = PETSc.Vec().createSeq(n)
+    ksp.solve(b, x)
+    return ksp, b, x
+
+
+@pytest.mark.parametrize("kt", ["gmres", "fgmres"])
+def test_host_form_launches_the_steps_it_needs(kt):
+    def best(its):
+        ksp, b, x = _solver(kt, "jacobi", its, "host")
+        times = []
+        for _ in range(20):
+            t = time.perf_counter()
+            ksp.solve(b, x)
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    # 8 trips against 72 (polled every eight), of one step each; with the graph's ten
+    # steps a trip both launch 80
+    assert best(1) < 0.5 * best(70)
