@@ -378,7 +378,8 @@ int gp_ksp_set_launch_form(gp_ksp ksp, int form);
 
 /* Kernel-launch accounting of the last solve: loop trips, kernels outside the
  * loop (prologue, epilogue) and kernels per trip.  Kernels launched =
- * top_kernels + trips * body_kernels. */
+ * top_kernels + trips * body_kernels; top_kernels includes those that only some
+ * of the trips ran. */
 int gp_ksp_stats(gp_ksp ksp, int64_t *trips, int64_t *top_kernels, int64_t *body_kernels);
 
 

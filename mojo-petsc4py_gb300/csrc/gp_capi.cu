@@ -464,7 +464,8 @@ int gp_ksp_set_launch_form(gp_ksp ksp, int form) {
 int gp_ksp_stats(gp_ksp ksp, int64_t* trips, int64_t* top_kernels, int64_t* body_kernels) {
   if (!ksp) return bad("gp_ksp_stats: null argument");
   if (trips) *trips = ksp->k->last_trips;
-  if (top_kernels) *top_kernels = ksp->k->top_kernels;
+  if (top_kernels)
+    *top_kernels = ksp->k->top_kernels + ksp->k->last_more * ksp->k->more_kernels;
   if (body_kernels) *body_kernels = ksp->k->body_kernels;
   return GP_OK;
 }

@@ -1516,6 +1516,7 @@ int ksp_destroy(Ksp* k) {
   if (k->h_st) cudaFreeHost(k->h_st);
   if (k->stream) cudaStreamDestroy(k->stream);
   if (k->stream2) cudaStreamDestroy(k->stream2);
+  if (k->stream3) cudaStreamDestroy(k->stream3);
   delete k;
   return GP_OK;
 }
@@ -1574,6 +1575,21 @@ static int ensure(Ksp* k, int n, bool* moved) {
   if (r != GP_OK && r != 1000) return r;
   *moved |= r == 1000;
   k->hist_cap = (int)hc;
+  return GP_OK;
+}
+
+static int count_kernels(cudaGraph_t g, int64_t* out) {
+  size_t cnt = 0;
+  GP_CUDA(cudaGraphGetNodes(g, nullptr, &cnt));
+  std::vector<cudaGraphNode_t> nodes(cnt);
+  if (cnt) GP_CUDA(cudaGraphGetNodes(g, nodes.data(), &cnt));
+  int64_t k = 0;
+  for (auto nd : nodes) {
+    cudaGraphNodeType t;
+    GP_CUDA(cudaGraphNodeGetType(nd, &t));
+    if (t == cudaGraphNodeTypeKernel) k++;
+  }
+  *out = k;
   return GP_OK;
 }
 
@@ -2033,6 +2049,66 @@ static int gmres_prologue(const Run& r) {
   return GP_OK;
 }
 
+// Whether another Arnoldi step follows, for the IF node of a trip's later steps.
+__global__ void k_more_steps(cudaGraphConditionalHandle h, KspState* st) {
+  const bool more = st->g[1] != 0;
+  st->more += more;
+  cudaGraphSetConditional(h, more ? 1u : 0u);
+}
+
+// `count` more steps of a captured trip, in an IF node that is taken while a step
+// is to come.
+template <typename F>
+static int capture_more(const Run& r, int count, F step) {
+  Ksp* k = r.k;
+  if (!k->stream3) GP_CUDA(cudaStreamCreateWithFlags(&k->stream3, cudaStreamNonBlocking));
+  cudaStreamCaptureStatus cs;
+  cudaGraph_t graph = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  cudaGraphConditionalHandle h = 0;
+  GP_CUDA(cudaStreamGetCaptureInfo(r.s, &cs, nullptr, &graph, &deps, nullptr, &ndeps));
+  GP_CUDA(cudaGraphConditionalHandleCreate(&h, graph, 0, 0));
+  k_more_steps<<<1, 1, 0, r.s>>>(h, k->st);
+  GP_CHECK_LAUNCH();
+  GP_CUDA(cudaStreamGetCaptureInfo(r.s, &cs, nullptr, &graph, &deps, nullptr, &ndeps));
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = h;
+  cp.conditional.type = cudaGraphCondTypeIf;
+  cp.conditional.size = 1;
+  cudaGraphNode_t node = nullptr;
+  GP_CUDA(cudaGraphAddNode(&node, graph, deps, nullptr, ndeps, &cp));
+  GP_CUDA(cudaStreamUpdateCaptureDependencies(r.s, &node, nullptr, 1,
+                                              cudaStreamSetCaptureDependencies));
+  GP_CUDA(cudaStreamBeginCaptureToGraph(k->stream3, cp.conditional.phGraph_out[0], nullptr, nullptr,
+                                        0, cudaStreamCaptureModeRelaxed));
+  Run rr = r;
+  rr.s = k->stream3;
+  int status = GP_OK;
+  for (int i = 0; i < count && status == GP_OK; i++) status = step(rr);
+  cudaGraph_t out = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(k->stream3, &out);
+  GP_TRY(status);
+  GP_CUDA(e);
+  return count_kernels(out, &k->more_kernels);
+}
+
+// A trip's steps.  Those after the first three are left out together once no step
+// is to come: a solve of up to three steps (an almost exact preconditioner, a warm
+// start) then has no idle ones after it, five launches or more of up to 3 us each
+// a step (GMRES+Jacobi, one step: 110 us on 32^2 and 172 on 64^3, 131 and 269
+// without the node, 122 and 206 with one step a trip); the node costs a long solve
+// 8 us a trip.
+constexpr int kFirstSteps = 3;
+
+template <typename F>
+static int trip_steps(const Run& r, F step) {
+  const int first = r.steps > kFirstSteps + 1 ? kFirstSteps : r.steps;
+  for (int i = 0; i < first; i++) GP_TRY(step(r));
+  return r.steps > first ? capture_more(r, r.steps - first, step) : GP_OK;
+}
+
 // A trip: a restart where a cycle begins, steps, and the solution update where
 // they ended the cycle (so the trip that converges is the last one).
 static int gmres_body(const Run& r, const double* b, double* x) {
@@ -2060,7 +2136,7 @@ static int gmres_body(const Run& r, const double* b, double* x) {
   GP_CHECK_LAUNCH();
   // ---- Arnoldi steps
   DRef vit = DRef::at(&st->vv_it), vit1 = DRef::at(&st->vv_it1);
-  for (int step = r.steps; step > 0; step--) {
+  auto step = [&](const Run& r) -> int {
     GP_TRY(r.apply_ba(r.G(1), side, vit, vit1, TMATOP));
     if (gm_fused(r)) {
       GP_TRY(cgs_dots(r, 1));
@@ -2079,7 +2155,9 @@ static int gmres_body(const Run& r, const double* b, double* x) {
       k_gm_step_ctrl<<<1, 32, 0, r.s>>>(st, k->hs, k->hist, k->vv, n);
     }
     GP_CHECK_LAUNCH();
-  }
+    return GP_OK;
+  };
+  GP_TRY(trip_steps(r, step));
   // ---- build the solution at the end of a cycle (KSPGMRESBuildSoln)
   k_gm_backsub<<<1, 1, 0, r.s>>>(st, k->hs);
   const int m = k->opt.restart;
@@ -2133,7 +2211,7 @@ static int fgmres_body(const Run& r, const double* b, double* x) {
   GP_CHECK_LAUNCH();
   // ---- flexible Arnoldi steps
   DRef vit = DRef::at(&st->vv_it), vit1 = DRef::at(&st->vv_it1), pit = DRef::at(&st->pv_it);
-  for (int step = r.steps; step > 0; step--) {
+  auto step = [&](const Run& r) -> int {
     GP_TRY(r.pcapply(r.G(1), vit, pit));
     GP_TRY(r.matmult(r.G(1), pit, vit1));
     if (gm_fused(r)) {
@@ -2153,7 +2231,9 @@ static int fgmres_body(const Run& r, const double* b, double* x) {
                                                 r.S(&KspState::inv));
     GP_TRY(r.zero(r.G(12), TEMP));
     GP_CHECK_LAUNCH();
-  }
+    return GP_OK;
+  };
+  GP_TRY(trip_steps(r, step));
   // ---- build (KSPFGMRESBuildSoln)
   k_fg_backsub<<<1, 1, 0, r.s>>>(st, k->hs);
   FL(k_maxpy_dyn, r.grid(), 256, r.s, r.G(8), 1, n, TEMP, k->prevec, rs, &st->kcount, 1);
@@ -2164,23 +2244,6 @@ static int fgmres_body(const Run& r, const double* b, double* x) {
 }
 
 // ------------------------------------------------------------------ solve
-
-// The whole solve as one graph: prologue kernels, a WHILE node whose body is
-// one iteration, the epilogue, and the read-back of the state block.
-static int count_kernels(cudaGraph_t g, int64_t* out) {
-  size_t cnt = 0;
-  GP_CUDA(cudaGraphGetNodes(g, nullptr, &cnt));
-  std::vector<cudaGraphNode_t> nodes(cnt);
-  if (cnt) GP_CUDA(cudaGraphGetNodes(g, nodes.data(), &cnt));
-  int64_t k = 0;
-  for (auto nd : nodes) {
-    cudaGraphNodeType t;
-    GP_CUDA(cudaGraphNodeGetType(nd, &t));
-    if (t == cudaGraphNodeTypeKernel) k++;
-  }
-  *out = k;
-  return GP_OK;
-}
 
 static int run_prologue(const Run& r, const double* b, double* x) {
   switch (r.k->opt.type) {
@@ -2257,12 +2320,16 @@ static int run_eager(const Run& r, const double* b, double* x) {
   GP_CUDA(cudaMemcpyAsync(k->h_st, k->st, sizeof(KspState), cudaMemcpyDeviceToHost, r.s));
   k->top_kernels = -1;
   k->body_kernels = -1;
+  k->more_kernels = 0;
   return GP_OK;
 }
 
+// The whole solve as one graph: prologue kernels, a WHILE node whose body is a
+// trip of the loop, the epilogue, and the read-back of the state block.
 static int capture(const Run& r, const double* b, double* x) {
   Ksp* k = r.k;
   drop_graph(k);
+  k->more_kernels = 0;
   if (!k->stream2) GP_CUDA(cudaStreamCreateWithFlags(&k->stream2, cudaStreamNonBlocking));
   GP_CUDA(cudaStreamBeginCapture(r.s, cudaStreamCaptureModeRelaxed));
   int st = run_prologue(r, b, x);
@@ -2448,6 +2515,7 @@ int ksp_solve(Ksp* k, Csr* A, Pc* pc, const double* b, double* x, KspResult* res
   res->reason = h.reason;
   res->rnorm = h.rnorm;
   k->last_trips = h.trips;
+  k->last_more = h.more;
   if (hist_out && hist_len > 0) {
     const int64_t cnt = std::min<int64_t>(hist_len, std::min<int64_t>(h.its + 1, k->hist_cap));
     GP_CUDA(cudaMemcpy(hist_out, k->hist, (size_t)cnt * sizeof(double), cudaMemcpyDeviceToHost));

@@ -42,6 +42,7 @@ struct KspState {
   int active;       // 1 while the solve runs (CG, BCGS)
   int phase;        // GMRES / FGMRES phase
   int trips;
+  int more;         // trips whose later steps ran (GMRES / FGMRES)
   int g[16];        // per-driver conditional gates
   // CG
   double beta, betaold, dpi, dpiold, a, dp, bcoef;
@@ -89,9 +90,11 @@ struct Ksp {
   const void* cap_x = nullptr;
   int cap_key[13] = {0};
   cudaStream_t stream2 = nullptr;  // body capture stream
+  cudaStream_t stream3 = nullptr;  // and that of a trip's later steps
   int64_t top_kernels = 0;         // kernels outside the loop body
   int64_t body_kernels = 0;        // kernels per loop trip
-  int64_t last_trips = 0;
+  int64_t more_kernels = 0;        // kernels of a trip's later steps, where they run
+  int64_t last_trips = 0, last_more = 0;
   int launch_form = -1;  // -1 the environment's (GPETSC_KSP_GRAPH), 0 graph, 1 host loop
   int transpose = 0;     // solve A^T x = b (A^T multiply, transposed preconditioner)
 };

@@ -2,6 +2,7 @@
 copies that a trip holds for longer solves are not launched, or not all, once a
 solve has ended.  Counted from the launch accounting; the host-driven form, which
 has none, by its time against a long solve's."""
+import ctypes
 import time
 
 import numpy as np
@@ -46,3 +47,20 @@ def test_host_form_launches_the_steps_it_needs(kt):
     # 8 trips against 72 (polled every eight), of one step each; with the graph's ten
     # steps a trip both launch 80
     assert best(1) < 0.5 * best(70)
+
+
+def _launched(kt, pt, its):
+    """Kernels of a solve of `its` iterations."""
+    ksp, _, _ = _solver(kt, pt, its)
+    assert abs(ksp.getIterationNumber() - its) <= 1
+    c = [ctypes.c_int64() for _ in range(3)]
+    _lib.check(_lib.lib().gp_ksp_stats(ksp._gp, *(ctypes.byref(v) for v in c)))
+    trips, top, body = (v.value for v in c)
+    return top + trips * body
+
+
+@pytest.mark.parametrize("kt", ["gmres", "fgmres"])
+def test_a_trip_leaves_out_its_later_steps(kt):
+    # ten steps a trip: the start and end of a cycle are about four steps' worth
+    assert _launched(kt, "jacobi", 1) == _launched(kt, "jacobi", 3)
+    assert _launched(kt, "jacobi", 3) < 0.7 * _launched(kt, "jacobi", 10)
