@@ -64,3 +64,9 @@ def test_a_trip_leaves_out_its_later_steps(kt):
     # ten steps a trip: the start and end of a cycle are about four steps' worth
     assert _launched(kt, "jacobi", 1) == _launched(kt, "jacobi", 3)
     assert _launched(kt, "jacobi", 3) < 0.7 * _launched(kt, "jacobi", 10)
+
+
+@pytest.mark.parametrize("kt,pt", [("cg", "none"), ("cg", "icc"), ("bcgs", "jacobi")])
+def test_one_iteration_has_no_idle_copies(kt, pt):
+    one, two, three, four = (_launched(kt, pt, its) for its in (1, 2, 3, 4))
+    assert one < two == three < four
