@@ -35,8 +35,8 @@ def _solver(kt, pt, its, form="graph"):
 
 @pytest.mark.parametrize("kt", ["gmres", "fgmres"])
 def test_host_form_launches_the_steps_it_needs(kt):
-    def best(its):
-        ksp, b, x = _solver(kt, "jacobi", its, "host")
+    def best(kt):
+        ksp, b, x = _solver(kt, "jacobi", 1, "host")
         times = []
         for _ in range(20):
             t = time.perf_counter()
@@ -44,9 +44,10 @@ def test_host_form_launches_the_steps_it_needs(kt):
             times.append(time.perf_counter() - t)
         return min(times)
 
-    # 8 trips against 72 (polled every eight), of one step each; with the graph's ten
-    # steps a trip both launch 80
-    assert best(1) < 0.5 * best(70)
+    # One iteration is eight trips (the convergence is polled then) of about 25
+    # launches, of which five are the step, or of BiCGStab's 15; with the graph's ten
+    # steps a trip they were about 75.  Between the ratios 1.7 and 5: 3
+    assert best(kt) < 3.0 * best("bcgs")
 
 
 def _launched(kt, pt, its):
