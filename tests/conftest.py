@@ -43,6 +43,17 @@ def _arithmetic(request):
     _lib.set_arithmetic(before)
 
 
+@pytest.fixture(scope="module", autouse=True)
+def _default_sweep_forms():
+    """Every test file begins with the sweep forms that a user gets, whatever the
+    files before it set and "restored" (the settings are process-wide)."""
+    lib = sys.modules.get("mojopetsc4py._lib")
+    if lib is not None:
+        lib.set_sweep_form(True, 0)
+        lib.set_sweep_bricks(1, 0, 0, 0)
+    yield
+
+
 def has_gpu() -> bool:
     try:
         from mojopetsc4py import _lib
