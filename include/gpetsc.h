@@ -293,7 +293,10 @@ int gp_pc_sweep_form(gp_pc pc, int32_t which, int32_t *tiled, int32_t *rows_per_
  *   lines_j in 1..128 forces bricks of that many neighbouring lines (in equal
  *   tiles, so rounded up where they do not divide evenly); 0 lets the set-up
  *   choose.  lines_k must be 0 or 1.  max_ctas > 0 caps the persistent grid
- *   (each CTA then walks several bricks); 0 sizes it to the device.
+ *   (each CTA then walks several bricks), at one cluster of bricks at the
+ *   least; 0 sizes it to the device.
+ * In 3-D the bricks form thread-block clusters where the device can hold them
+ * (GPETSC_BRICK_CLUSTERS=0: without).
  * Bit-identical to the other forms.  Defaults from GPETSC_SWEEP_BRICKS and
  * GPETSC_BRICK_LINES.  No counterpart in the reference. */
 int gp_set_sweep_bricks(int32_t mode, int32_t lines_j, int32_t lines_k, int32_t max_ctas);

@@ -934,15 +934,16 @@ static double brick_model_us(const BrickShape& g) {
 // 96^3 211 (221, 222, 235), 81^3 208 (210, 212, 223), 160^3, where the bricks take
 // two rounds, 408 (410, -, 436).  In 2-D a cluster saves one or two faces of 2 us
 // and its stores cost as much (256^2: 223 against 213).  The layout of the faces
-// depends on it, so it is a function of the shape alone.
-static void brick_cluster(BrickShape& g) {
+// depends on it, so it is settled at set-up: by the shape, and by whether the
+// device can hold such a cluster (brick_cluster_fits).
+static void brick_cluster(BrickShape& g, bool clusters) {
   g.XP = g.XQ = 1;
-  if (!g.d3 || g.Wp != 8 || g.Wq != 4 || g.CP != 2 || g.CQ != 2) return;
+  if (!clusters || !g.d3 || g.Wp != 8 || g.Wq != 4 || g.CP != 2 || g.CQ != 2) return;
   g.XP = std::min(2, g.nbP);
   g.XQ = std::min(4, g.nbQ);
 }
 
-static BrickShape brick_shape(const int* dims, bool bwd, int lines) {
+static BrickShape brick_shape(const int* dims, bool bwd, int lines, bool clusters) {
   BrickShape g{};
   const int nx = dims[0], ny = dims[1], nz = dims[2];
   g.n = nx * ny * nz;
@@ -980,7 +981,7 @@ static BrickShape brick_shape(const int* dims, bool bwd, int lines) {
   g.ntQ = (g.nq + g.Wq - 1) / g.Wq;
   g.nbP = (g.ntP + g.CP - 1) / g.CP;
   g.nbQ = (g.ntQ + g.CQ - 1) / g.CQ;
-  brick_cluster(g);
+  brick_cluster(g, clusters);
   int phase = 0;  // the largest of any tile of a brick
   for (int cp = 0; cp < g.CP; cp++)
     for (int cq = 0; cq < g.CQ; cq++)
@@ -992,40 +993,56 @@ static BrickShape brick_shape(const int* dims, bool bwd, int lines) {
 
 static BrickShape shape_of(const EllSweep& e) {
   const int dims[3] = {e.gx, e.gy, e.gz};
-  return brick_shape(dims, e.bwd, e.blines);
+  return brick_shape(dims, e.bwd, e.blines, e.clusters);
 }
 
-template <int MODE>
-static void brick_launch(int grid, int threads, const int* gate, int want, const BrickArgs& a,
-                         DRef in, DRef out, cudaStream_t s) {
-  const BrickShape& g = a.g;
-  // the other arithmetics, and tiles of other shapes, take the general addresses
-  const bool f = arith_mode() == kFma;
-  const bool full = g.LW == 32 && g.Wp + g.Wq <= (g.d3 ? 14 : 33);
-  const size_t smem = (size_t)g.CP * g.CQ * 8 *
-                      (brick_ring(full && f, g.d3) + kStages * kGroup * brick_cols(MODE, g.d3) * g.LW);
-  const bool cl = g.XP * g.XQ > 1;  // then the tiles are full ones (brick_cluster)
-  auto k = cl       ? (f ? k_brick_sweep<MODE, true, true, true, true>
-                         : k_brick_sweep<MODE, false, false, true, true>)
-           : g.d3 ? (!f     ? k_brick_sweep<MODE, false, false, true, false>
-                     : full ? k_brick_sweep<MODE, true, true, true, false>
-                            : k_brick_sweep<MODE, true, false, true, false>)
-                  : (!f     ? k_brick_sweep<MODE, false, false, false, false>
-                     : full ? k_brick_sweep<MODE, true, true, false, false>
-                            : k_brick_sweep<MODE, true, false, false, false>);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = g.XP * g.XQ;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = g.XP * g.XQ > 1 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k, gate, want, a, in, out);
+// Fetching lanes a face line (a.poll) and fetch warps: kBrickPoll lanes for every
+// face line of a brick; none where one brick is the grid.
+static void brick_fetchers(const BrickShape& g, int& poll, int& nf) {
+  const int cols = g.CQ * g.Wq + (g.d3 ? g.CP * g.Wp : 0);
+  poll = kBrickPoll;
+  while (poll > 1 && cols * poll > 32 * kBrickFetchMax) poll /= 2;
+  nf = g.nbP > g.XP || g.nbQ > g.XQ ? (cols * poll + 31) / 32 : 0;
 }
+
+static int brick_threads(const BrickShape& g) {
+  int poll, nf;
+  brick_fetchers(g, poll, nf);
+  return 32 * (g.CP * g.CQ + nf + (g.XP * g.XQ > 1 ? 1 : 0));
+}
+
+// A sweep's kernel and its launch.
+template <int MODE>
+struct BrickLaunch {
+  void (*kernel)(const int*, int, BrickArgs, DRef, DRef);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+
+  BrickLaunch(const BrickShape& g, int grid, cudaStream_t s, bool f) {
+    // the other arithmetics, and tiles of other shapes, take the general addresses
+    const bool full = g.LW == 32 && g.Wp + g.Wq <= (g.d3 ? 14 : 33);
+    const bool cl = g.XP * g.XQ > 1;  // then the tiles are full ones (brick_cluster)
+    kernel = cl       ? (f ? k_brick_sweep<MODE, true, true, true, true>
+                           : k_brick_sweep<MODE, false, false, true, true>)
+             : g.d3 ? (!f     ? k_brick_sweep<MODE, false, false, true, false>
+                       : full ? k_brick_sweep<MODE, true, true, true, false>
+                              : k_brick_sweep<MODE, true, false, true, false>)
+                    : (!f     ? k_brick_sweep<MODE, false, false, false, false>
+                       : full ? k_brick_sweep<MODE, true, true, false, false>
+                              : k_brick_sweep<MODE, true, false, false, false>);
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(brick_threads(g));
+    cfg.dynamicSmemBytes =
+        (size_t)g.CP * g.CQ * 8 *
+        (brick_ring(full && f, g.d3) + kStages * kGroup * brick_cols(MODE, g.d3) * g.LW);
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = g.XP * g.XQ;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cl ? 1 : 0;
+  }
+};
 
 template <int MODE>
 static void brick_attrs() {
@@ -1040,29 +1057,60 @@ static void brick_attrs() {
                          kBrickSmemMax);
 }
 
+// The modes as template arguments: M in X.
+#define BRICK_MODES(X) \
+  X(ELL_ILU_F) X(ELL_ILU_B) X(ELL_ILUT_F) X(ELL_ILUT_B) X(ELL_ICC_F) X(ELL_ICC_B) \
+  X(ELL_SOR_F) X(ELL_SOR_B) X(ELL_SOR_B0)
+
 // The kernels' shared-memory limit, once a device (at set-up: not capturable).
 static void brick_set_attrs() {
   static std::atomic<unsigned long long> done{0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && (done.load() >> dev & 1ull)) return;
-  brick_attrs<ELL_ILU_F>();
-  brick_attrs<ELL_ILU_B>();
-  brick_attrs<ELL_ILUT_F>();
-  brick_attrs<ELL_ILUT_B>();
-  brick_attrs<ELL_ICC_F>();
-  brick_attrs<ELL_ICC_B>();
-  brick_attrs<ELL_SOR_F>();
-  brick_attrs<ELL_SOR_B>();
-  brick_attrs<ELL_SOR_B0>();
+#define BRICK_ATTRS(M) brick_attrs<M>();
+  BRICK_MODES(BRICK_ATTRS)
+#undef BRICK_ATTRS
   if (dev < 64) done |= 1ull << dev;
 }
 
-static int brick_layout(EllSweep& e, int mode, const int* dims, int lines,
+// Whether the device can hold a cluster of this sweep's bricks at all, in either
+// arithmetic: eight SMs of one GPC with a CTA's shared memory each, which a
+// partition or a restricted set of SMs may not have.  GPETSC_BRICK_CLUSTERS=0
+// answers no.
+template <int MODE>
+static bool brick_cluster_fits(const BrickShape& g) {
+  static const char* env = std::getenv("GPETSC_BRICK_CLUSTERS");
+  if (env && std::string(env) == "0") return false;
+  for (bool f : {true, false}) {
+    BrickLaunch<MODE> l(g, g.XP * g.XQ, nullptr, f);
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, (const void*)l.kernel, &l.cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      fit = 0;
+    }
+    if (fit < 1) return false;
+  }
+  return true;
+}
+
+static bool brick_clusters(int mode, const int* dims, int lines) {
+  const BrickShape g = brick_shape(dims, brick_bwd(mode), lines, true);
+  if (g.XP * g.XQ == 1) return false;
+  brick_set_attrs();
+#define BRICK_FITS(M) \
+  case M: return brick_cluster_fits<M>(g);
+  switch (mode) { BRICK_MODES(BRICK_FITS) }
+#undef BRICK_FITS
+  return false;
+}
+
+static int brick_layout(EllSweep& e, int mode, const int* dims, int lines, bool clusters,
                         const std::vector<int>& slot, const std::vector<int>& dslot) {
   ell_free(e);
   brick_set_attrs();
-  const BrickShape g = brick_shape(dims, brick_bwd(mode), lines);
+  const BrickShape g = brick_shape(dims, brick_bwd(mode), lines, clusters);
+  e.clusters = clusters;
   e.brick = true;
   e.bwd = brick_bwd(mode);
   e.blines = lines;
@@ -1127,8 +1175,10 @@ int brick_build(EllSweep& ef, EllSweep& eb, int mode_f, int mode_b, int n,
   if (df[0] != db[0] || df[1] != db[1] || df[2] != db[2]) return GP_OK;
   const int lines = std::max(0, tu.BJ);
   double est = 0.0;
+  bool clusters[2];
   for (bool bwd : {false, true}) {
-    const BrickShape g = brick_shape(df, bwd, lines);
+    clusters[bwd] = brick_clusters(bwd ? mode_b : mode_f, df, lines);
+    const BrickShape g = brick_shape(df, bwd, lines, clusters[bwd]);
     // positions (steps x lanes, idle ones included) are int32, and few lanes
     // idle: a grid of very short lines keeps the other forms
     const long long pos = (long long)g.ntP * g.ntQ * g.NS * g.LW;
@@ -1139,13 +1189,16 @@ int brick_build(EllSweep& ef, EllSweep& eb, int mode_f, int mode_b, int n,
       return GP_OK;
     est += us;
   }
-  GP_TRY(brick_layout(ef, mode_f, df, lines, sf, dslot));
-  GP_TRY(brick_layout(eb, mode_b, df, lines, sb, dslot));
-  if (std::getenv("GPETSC_SWEEP_VERBOSE"))
+  GP_TRY(brick_layout(ef, mode_f, df, lines, clusters[0], sf, dslot));
+  GP_TRY(brick_layout(eb, mode_b, df, lines, clusters[1], sb, dslot));
+  if (std::getenv("GPETSC_SWEEP_VERBOSE")) {
+    const BrickShape gf = shape_of(ef), gb = shape_of(eb);
     std::fprintf(stderr,
                  "gpetsc sweep: n=%d grid %dx%dx%d bricks of %dx%d (forward) and %dx%d lines: "
-                 "%d and %d, est=%.0fus\n",
-                 n, df[0], df[1], df[2], ef.BJ, ef.BK, eb.BJ, eb.BK, ef.nbricks, eb.nbricks, est);
+                 "%d and %d, clusters of %dx%d and %dx%d, est=%.0fus\n",
+                 n, df[0], df[1], df[2], ef.BJ, ef.BK, eb.BJ, eb.BK, ef.nbricks, eb.nbricks, gf.XP,
+                 gf.XQ, gb.XP, gb.XQ, est);
+  }
   *built = true;
   return GP_OK;
 }
@@ -1181,29 +1234,17 @@ int brick_sweep(int mode, const EllSweep& e, const int* gate, int want, DRef in,
   a.write_out = write_out;
   a.tickets = tickets;
   a.err = err;
-  // kBrickPoll lanes for every face line of a brick; none where one brick is
-  // the grid
-  const int cols = a.g.CQ * a.g.Wq + (a.g.d3 ? a.g.CP * a.g.Wp : 0);
-  a.poll = kBrickPoll;
-  while (a.poll > 1 && cols * a.poll > 32 * kBrickFetchMax) a.poll /= 2;
-  a.nf = a.nclusters > 1 ? (cols * a.poll + 31) / 32 : 0;
-  const int threads = 32 * (a.g.CP * a.g.CQ + a.nf + (xc > 1 ? 1 : 0));
+  brick_fetchers(a.g, a.poll, a.nf);
   int grid = std::min(a.nclusters * xc, num_sms() * 2);
   if (brick_tuning().max_ctas > 0) grid = std::min(grid, brick_tuning().max_ctas);
   grid = std::max(grid / xc, 1) * xc;
-#define BRICK_LAUNCH(M) \
-  case M: brick_launch<M>(grid, threads, gate, want, a, in, out, s); break;
-  switch (mode) {
-    BRICK_LAUNCH(ELL_ILU_F)
-    BRICK_LAUNCH(ELL_ILU_B)
-    BRICK_LAUNCH(ELL_ILUT_F)
-    BRICK_LAUNCH(ELL_ILUT_B)
-    BRICK_LAUNCH(ELL_ICC_F)
-    BRICK_LAUNCH(ELL_ICC_B)
-    BRICK_LAUNCH(ELL_SOR_F)
-    BRICK_LAUNCH(ELL_SOR_B)
-    BRICK_LAUNCH(ELL_SOR_B0)
+#define BRICK_LAUNCH(M)                                                                \
+  case M: {                                                                            \
+    const BrickLaunch<M> l(a.g, grid, s, arith_mode() == kFma);                        \
+    GP_CUDA(cudaLaunchKernelEx(&l.cfg, l.kernel, gate, want, a, in, out));             \
+    break;                                                                             \
   }
+  switch (mode) { BRICK_MODES(BRICK_LAUNCH) }
 #undef BRICK_LAUNCH
   GP_CHECK_LAUNCH();
   return GP_OK;

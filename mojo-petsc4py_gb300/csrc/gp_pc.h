@@ -76,6 +76,7 @@ struct EllSweep {
   // [tile][step][bcols][lane] (npos steps x lanes, idle ones included).  The
   // two sweeps of a PC have it together.
   bool brick = false, bwd = false;
+  bool clusters = false;      // bricks in thread-block clusters where the shape has them
   int gx = 0, gy = 0, gz = 0, BJ = 0, BK = 0, nbricks = 0, npos = 0, bcols = 0;
   int blines = 0;             // forced lines of a brick (0: chosen)
   int* border = nullptr;      // place (P, Q) of each cluster of bricks in hand-out order
