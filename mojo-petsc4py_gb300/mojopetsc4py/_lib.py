@@ -203,11 +203,11 @@ def set_sweep_form(tiles: bool = True, tile_rows: int = 0) -> None:
     check(lib().gp_set_sweep_form(1 if tiles else 0, int(tile_rows)))
 
 
-def set_sweep_bricks(mode: int = 0, lines_j: int = 0, lines_k: int = 0,
+def set_sweep_bricks(mode: int = 1, lines_j: int = 0, lines_k: int = 0,
                      max_ctas: int = 0) -> None:
     """Brick form of the triangular sweeps of later PC set-ups (grid-structured
-    sweeps only): mode 0 never, 1 where modelled faster (a set-up's own
-    default), 2 whenever the structure allows; `lines_j` (1-128) forces bricks
+    sweeps only): mode 0 never, 1 where modelled faster (the default, here and
+    of a set-up), 2 whenever the structure allows; `lines_j` (1-128) forces bricks
     of that many neighbouring grid lines (`lines_k` 0 or 1); `max_ctas` caps the
     persistent grid.  Bit-identical to the other forms."""
     check(lib().gp_set_sweep_bricks(int(mode), int(lines_j), int(lines_k), int(max_ctas)))

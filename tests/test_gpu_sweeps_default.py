@@ -24,6 +24,13 @@ def test_a_grid_gets_bricks(pt):
     assert _bricks(_pc(pt, _mat(*gallery.laplacian_2d(40)), {}))
 
 
+def test_settings_without_arguments_are_the_default():
+    _lib.set_sweep_bricks(0)
+    assert not _bricks(_pc("ilu", _mat(*gallery.laplacian_3d(20)), {}))
+    _lib.set_sweep_bricks()
+    assert _bricks(_pc("ilu", _mat(*gallery.laplacian_3d(20)), {}))
+
+
 def test_transposed_solve():
     ip, ix, v = gallery.convection_diffusion_3d(20)
     n = len(ip) - 1
