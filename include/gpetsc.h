@@ -420,6 +420,11 @@ int gp_mixed_create(gp_mixed *out);
 int gp_mixed_destroy(gp_mixed m);
 int gp_mixed_solve(gp_mixed m, gp_mat A, gp_pc pc, const gp_mixed_options *o, const double *b,
                    double *x, gp_mixed_result *result, void *stream);
+/* Which matrices of the last solve were read by diagonals: diagonals[3] = the
+ * number of them of the operator, of L and of U, 0 for one read as sparse rows
+ * (more than eight diagonals, a reordered factor, no row with all of them).
+ * No counterpart in the reference. */
+int gp_mixed_form(gp_mixed m, int32_t *diagonals);
 
 /* ------------------------------------------------------------ batched CG
  * Many independent SPD systems with nrhs right-hand sides each, solved

@@ -1759,17 +1759,22 @@ __global__ void k_mx_cast32(const int* gate, int n, const double* __restrict__ a
     b[i] = __double2float_rn(a[i]);
 }
 
+static int bad_diagonals(int W) {
+  set_error("mixed solve: a kernel for " + std::to_string(W) + " diagonals was asked for");
+  return GP_ERR_INTERNAL;
+}
+
 // One pass of a triangle stored by diagonals.
-static void tri_pass_dia(int W, const DiaOffsets& off, const float* val, const int* gate, int n,
-                         const float* dinv, const float* rhs, const float* in, const float* sc,
-                         float* vout, float* out, const float* scale2, float* out2,
-                         cudaStream_t s) {
+static int tri_pass_dia(int W, const DiaOffsets& off, const float* val, const int* gate, int n,
+                        const float* dinv, const float* rhs, const float* in, const float* sc,
+                        float* vout, float* out, const float* scale2, float* out2,
+                        cudaStream_t s) {
   const int gr = (n + kMixBlock * kTriRows - 1) / (kMixBlock * kTriRows);
 #define GP_TRI_DIA(WW)                                                                       \
   case WW:                                                                                   \
-    (void)launch_pdl(k_mx_tri_dia<WW>, gr, kMixBlock, s, gate, n, off, val, dinv, rhs, in,   \
-                     sc, vout, out, scale2, out2);                                           \
-    return;
+    GP_CUDA(launch_pdl(k_mx_tri_dia<WW>, gr, kMixBlock, s, gate, n, off, val, dinv, rhs, in, \
+                       sc, vout, out, scale2, out2));                                        \
+    return GP_OK;
   switch (W) {
     GP_TRI_DIA(1)
     GP_TRI_DIA(2)
@@ -1781,14 +1786,16 @@ static void tri_pass_dia(int W, const DiaOffsets& off, const float* val, const i
     GP_TRI_DIA(8)
   }
 #undef GP_TRI_DIA
+  return bad_diagonals(W);
 }
 
-static void spmv_dia(const Mixed* M, const int* gate, const float* x, float* y, cudaStream_t s) {
+static int spmv_dia(const Mixed* M, const int* gate, const float* x, float* y, cudaStream_t s) {
   const int n = M->n, gr = (n + kMixBlock * kMxSpmvRows - 1) / (kMixBlock * kMxSpmvRows);
 #define GP_SPMV_DIA(WW)                                                                      \
   case WW:                                                                                   \
-    (void)launch_pdl(k_mx_spmv_dia<WW>, gr, kMixBlock, s, gate, n, M->aoff, M->adia, x, y);  \
-    return;
+    GP_CUDA(launch_pdl(k_mx_spmv_dia<WW>, gr, kMixBlock, s, gate, n, M->aoff, M->adia, x,    \
+                       y));                                                                  \
+    return GP_OK;
   switch (M->aW) {
     GP_SPMV_DIA(1)
     GP_SPMV_DIA(2)
@@ -1800,19 +1807,20 @@ static void spmv_dia(const Mixed* M, const int* gate, const float* x, float* y, 
     GP_SPMV_DIA(8)
   }
 #undef GP_SPMV_DIA
+  return bad_diagonals(M->aW);
 }
 
 // One triangle pass: the ELL form when the triangle has at most 8 slots a row.
-static void tri_pass(int W, const int* eci, const float* eval, const int* rp, const int* ci,
-                     const float* val, const int* gate, int n, const float* dinv,
-                     const float* rhs, const int* rhs_perm, const float* in, const int* in_perm,
-                     const float* in_scale, float* out, const int* out_perm, cudaStream_t s) {
+static int tri_pass(int W, const int* eci, const float* eval, const int* rp, const int* ci,
+                    const float* val, const int* gate, int n, const float* dinv,
+                    const float* rhs, const int* rhs_perm, const float* in, const int* in_perm,
+                    const float* in_scale, float* out, const int* out_perm, cudaStream_t s) {
   const int gr = (n + kMixBlock * kTriRows - 1) / (kMixBlock * kTriRows);
-#define GP_TRI_ELL(WW)                                                                     \
-  case WW:                                                                                 \
-    (void)launch_pdl(k_mx_tri_ell<WW>, gr, kMixBlock, s, gate, n, eci, eval, dinv, rhs,   \
-                     rhs_perm, in, in_perm, in_scale, out, out_perm);                      \
-    return;
+#define GP_TRI_ELL(WW)                                                                   \
+  case WW:                                                                               \
+    GP_CUDA(launch_pdl(k_mx_tri_ell<WW>, gr, kMixBlock, s, gate, n, eci, eval, dinv, rhs, \
+                       rhs_perm, in, in_perm, in_scale, out, out_perm));                 \
+    return GP_OK;
   switch (W) {
     GP_TRI_ELL(1)
     GP_TRI_ELL(2)
@@ -1826,8 +1834,9 @@ static void tri_pass(int W, const int* eci, const float* eval, const int* rp, co
       break;
   }
 #undef GP_TRI_ELL
-  (void)launch_pdl(k_mx_tri, (n + kMixBlock - 1) / kMixBlock, kMixBlock, s, gate, n, rp, ci, val,
-                   dinv, rhs, rhs_perm, in, in_perm, in_scale, out, out_perm);
+  GP_CUDA(launch_pdl(k_mx_tri, (n + kMixBlock - 1) / kMixBlock, kMixBlock, s, gate, n, rp, ci, val,
+                     dinv, rhs, rhs_perm, in, in_perm, in_scale, out, out_perm));
+  return GP_OK;
 }
 
 // Record one refinement pass into the current capture on stream s.
@@ -1889,9 +1898,9 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
       const float* yin = src;
       for (int k = 0; k < tri_sweeps; k++) {
         const bool firstp = k == 0, lastp = k + 1 == tri_sweeps;
-        tri_pass_dia(M->lW, M->loff, M->lell_val, act, n, nullptr, firstp ? src : vj, yin,
-                     firstp ? sc : nullptr, firstp && j ? vj : nullptr, ya, M->udinv,
-                     lastp ? M->t4 : nullptr, s);
+        GP_TRY(tri_pass_dia(M->lW, M->loff, M->lell_val, act, n, nullptr, firstp ? src : vj,
+                            yin, firstp ? sc : nullptr, firstp && j ? vj : nullptr, ya, M->udinv,
+                            lastp ? M->t4 : nullptr, s));
         yin = ya;
         std::swap(ya, yb);
       }
@@ -1900,8 +1909,8 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
       const float* xin = M->t4;
       for (int k = 0; k < tri_sweeps; k++) {
         const bool lastp = k + 1 == tri_sweeps;
-        tri_pass_dia(M->uW, M->uoff, M->uell_val, act, n, M->udinv, yin, xin, nullptr, nullptr,
-                     lastp ? zj : xa, nullptr, nullptr, s);
+        GP_TRY(tri_pass_dia(M->uW, M->uoff, M->uell_val, act, n, M->udinv, yin, xin, nullptr,
+                            nullptr, lastp ? zj : xa, nullptr, nullptr, s));
         xin = xa;
         std::swap(xa, xb);
       }
@@ -1912,8 +1921,8 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
       const float* yin = vj;
       const int* yperm = perm_r;
       for (int k = 0; k < tri_sweeps; k++) {
-        tri_pass(M->lW, M->lell_ci, M->lell_val, M->lrp, M->lci, M->lval, act, n, nullptr, vj,
-                 perm_r, yin, yperm, nullptr, ya, nullptr, s);
+        GP_TRY(tri_pass(M->lW, M->lell_ci, M->lell_val, M->lrp, M->lci, M->lval, act, n, nullptr,
+                        vj, perm_r, yin, yperm, nullptr, ya, nullptr, s));
         yin = ya;
         yperm = nullptr;
         std::swap(ya, yb);
@@ -1924,8 +1933,9 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
       const float* xscale = M->udinv;
       for (int k = 0; k < tri_sweeps; k++) {
         const bool lastp = k + 1 == tri_sweeps;
-        tri_pass(M->uW, M->uell_ci, M->uell_val, M->urp, M->uci, M->uval, act, n, M->udinv, yin,
-                 nullptr, xin, nullptr, xscale, lastp ? zj : xa, lastp ? perm_c : nullptr, s);
+        GP_TRY(tri_pass(M->uW, M->uell_ci, M->uell_val, M->urp, M->uci, M->uval, act, n,
+                        M->udinv, yin, nullptr, xin, nullptr, xscale, lastp ? zj : xa,
+                        lastp ? perm_c : nullptr, s));
         xin = xa;
         xscale = nullptr;
         std::swap(xa, xb);
@@ -1939,7 +1949,7 @@ static int record_pass(Mixed* M, const Csr* A, const Pc* pc, const double* b, do
     // the step's kernels start while their predecessor drains (each waits
     // in pdl_wait() before reading it)
     if (M->aW)
-      spmv_dia(M, act, zj, M->w, s);
+      GP_TRY(spmv_dia(M, act, zj, M->w, s));
     else if (A->coff16)
       GP_CUDA(launch_pdl(k_mx_spmv32<short>, gr, kMixBlock, s, act, n, A->rowptr,
                          (const short*)A->coff16, A->val32, zj, M->w));
@@ -2090,6 +2100,18 @@ int gp_mixed_destroy(gp_mixed m) {
   if (!m) return GP_OK;
   gp::mixed_destroy(m->M);
   delete m;
+  return GP_OK;
+}
+
+int gp_mixed_form(gp_mixed m, int32_t* diagonals) {
+  if (!m || !diagonals) {
+    gp::set_error("gp_mixed_form: null argument");
+    return GP_ERR_ARG;
+  }
+  const gp::Mixed* M = m->M;
+  diagonals[0] = M->aW;
+  diagonals[1] = M->tri_dia ? M->lW : 0;
+  diagonals[2] = M->tri_dia ? M->uW : 0;
   return GP_OK;
 }
 

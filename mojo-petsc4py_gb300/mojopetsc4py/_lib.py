@@ -80,6 +80,7 @@ GP_SIGNATURES = {
     "gp_mixed_options_default": ([P], None),
     "gp_mixed_create": ([PP], ctypes.c_int),
     "gp_mixed_destroy": ([P], ctypes.c_int),
+    "gp_mixed_form": ([P, P], ctypes.c_int),
     "gp_mixed_solve": ([P, P, P, P, P, P, P, P], ctypes.c_int),
     "gp_batch_create": ([PP, I64, P, P, P, P, ctypes.c_int32, P], ctypes.c_int),
     "gp_batch_destroy": ([P], ctypes.c_int),

@@ -35,3 +35,14 @@ def test_workspace_offsets_are_64_bit():
         assert not re.findall(r"[+]\s*\(?[0-9]\s*\*\s*n\b", code), path.name
     code = _code("gp_ksp.cu")
     assert "return k->work + (size_t)i * k->n;" in code
+
+
+def test_no_launch_status_is_dropped():
+    """A captured pass keeps no kernel whose launch was refused: the status of each
+    launch is looked at, in every source file."""
+    for path in sorted(CSRC.glob("gp_*.cu*")):
+        code = _code(path.name)
+        assert not re.search(r"\(void\)\s*launch_pdl", code), path.name
+        for call in re.finditer(r"(.{0,24})\blaunch_pdl\(", code, re.S):
+            before = call.group(1).rstrip()
+            assert before.endswith(("GP_CUDA(", "=", "cudaError_t")), (path.name, before)
