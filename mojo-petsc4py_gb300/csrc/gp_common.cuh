@@ -179,6 +179,25 @@ __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, 
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double div_(double a, double b) { return __ddiv_rn(a, b); }
 
+// x / d, correctly rounded, for many x and one d > 0: `r` is 1 / d rounded to
+// nearest.  Two corrections of the quotient x r by its exact remainder: the
+// first leaves it within an ulp of x / d, and from there the second rounds
+// correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Five FP64 instructions; a division by itself
+// costs about twice that, and FP64 instructions are what a normalisation is
+// bound by.  Outside the range where no step can round off or overflow
+// (plain_range) the division itself.
+__device__ __forceinline__ bool plain_range(double v) {
+  const unsigned e = (unsigned)__double2hiint(v) >> 20 & 0x7ffu;
+  return e - 523u < 1000u;  // 2^-500 <= |v| < 2^500
+}
+__device__ __forceinline__ double div_by(double x, double d, double r, bool d_plain) {
+  if (!d_plain || !plain_range(x)) return div_(x, d);
+  double q = mul(x, r);
+  q = __fma_rn(__fma_rn(-q, d, x), r, q);
+  return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
 // a * x + y in the selected arithmetic (see Arith)
 template <bool FMA>
 __device__ __forceinline__ double madd(double a, double x, double y) {

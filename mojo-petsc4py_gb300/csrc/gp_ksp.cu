@@ -172,25 +172,6 @@ __global__ void k_waxpy_d(const int* gate, int want, int n, DRef wr, const doubl
         xr.get(), yr.get());
 }
 
-// x / d, correctly rounded, for many x and one d > 0: `r` is 1 / d rounded to
-// nearest.  Two corrections of the quotient x r by its exact remainder: the
-// first leaves it within an ulp of x / d, and from there the second rounds
-// correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990).  Five FP64 instructions; a division by itself
-// costs about twice that, and FP64 instructions are what a normalisation is
-// bound by.  Outside the range where no step can round off or overflow
-// (plain_range) the division itself.
-__device__ __forceinline__ bool plain_range(double v) {
-  const unsigned e = (unsigned)__double2hiint(v) >> 20 & 0x7ffu;
-  return e - 523u < 1000u;  // 2^-500 <= |v| < 2^500
-}
-__device__ __forceinline__ double div_by(double x, double d, double r, bool d_plain) {
-  if (!d_plain || !plain_range(x)) return div_(x, d);
-  double q = mul(x, r);
-  q = __fma_rn(__fma_rn(-q, d, x), r, q);
-  return __fma_rn(__fma_rn(-q, d, x), r, q);
-}
-
 // x = x * (*a)   (VecScale)  or  x = x / (*a) when *a > 0 (VecNormalize)
 template <bool DIVIDE>
 __global__ void k_scale_d(const int* gate, int want, int n, DRef xr, const double* a) {

@@ -1613,9 +1613,9 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_step(int n, size_t ld,
 
 // Back-substitution of the least-squares system by one warp, by columns: the
 // lanes hold the rows (two each), the reciprocals of the diagonal are taken a
-// lane each beforehand, and an unknown costs one multiply, its broadcast and one
-// multiply-add (row by row in one thread, with a divide and a chain of sums for
-// each, it took 45 us for 30).
+// lane each beforehand, and an unknown costs a quotient by its reciprocal (five
+// operations, correctly rounded), its broadcast and one multiply-add (row by row in
+// one thread, with a divide and a chain of sums for each, it took 45 us for 30).
 __global__ void k_mx_backsub(MixDev* st, int m) {
   if (!st->pass_on) return;
   __shared__ double Hs[kMixMaxM * kMixMaxM];
@@ -1625,18 +1625,24 @@ __global__ void k_mx_backsub(MixDev* st, int m) {
     if (c >= i) Hs[i * k + c] = st->H[i * m + c];
   }
   __syncwarp();
-  double t[2], rd[2];
+  double t[2], d[2], rd[2];
 #pragma unroll
   for (int u = 0; u < 2; u++) {
     const int i = lane + 32 * u;
     t[u] = i < k ? st->g[i] : 0.0;
-    const double d = i < k ? Hs[i * k + i] : 0.0;
-    rd[u] = d != 0.0 ? 1.0 / d : 0.0;
+    d[u] = i < k ? Hs[i * k + i] : 0.0;
+    rd[u] = d[u] != 0.0 ? 1.0 / d[u] : 0.0;
   }
   for (int c = k - 1; c >= 0; c--) {
-    const int u = c >> 5;
-    const double y = __shfl_sync(0xffffffffu, u ? t[1] * rd[1] : t[0] * rd[0], c & 31);
-    if (lane == (c & 31)) st->y[c] = y;
+    const bool second = c >= 32;
+    double y = 0.0;
+    if (lane == (c & 31)) {
+      const double dc = second ? d[1] : d[0];
+      if (dc != 0.0)
+        y = div_by(second ? t[1] : t[0], dc, second ? rd[1] : rd[0], plain_range(dc));
+      st->y[c] = y;
+    }
+    y = __shfl_sync(0xffffffffu, y, c & 31);
     if (lane < c) t[0] = __fma_rn(-Hs[lane * k + c], y, t[0]);
     if (lane + 32 < c) t[1] = __fma_rn(-Hs[(lane + 32) * k + c], y, t[1]);
   }
