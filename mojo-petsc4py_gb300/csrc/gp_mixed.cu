@@ -1303,8 +1303,10 @@ __device__ __forceinline__ float ld_here(const float* p) {
 // a row at a time (its conditional permutation and scale keep them apart).  A
 // row past the end loads the last one's values and stores nothing; an entry a
 // row does not have has a zero coefficient and is left out of the sum.  Bound by
-// the L2 (25 MB of it at 96^3 in 3.4 us; 1, 2 and 4 rows a thread: 9.7, 6.1 and
-// 4.3 us), with consecutive tiles of a block no worse than grid-wide strides.
+// the L2 (25 MB of it at 96^3 in 3.4 us alone, back to back; 1, 2 and 4 rows a
+// thread: 9.7, 6.1 and 4.3 us), with consecutive tiles of a block no worse than
+// grid-wide strides.  In the solve's list of serialised launches, where the L2 holds
+// less of the factor and nothing overlaps, a pass takes 6.6 us (ELL 10.3).
 //
 // What lies between the passes is done here too.  sc: rhs and in are the
 // unscaled new basis vector, *sc its factor, and the scaled one goes to vout
@@ -1366,8 +1368,9 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_tri_dia(
 }
 
 // y = A x over A's diagonals: coalesced loads only, a row's gathers waiting on
-// nothing (4.1 us at 96^3; a row a thread over CSR reads each of a warp's value
-// slots from seven cache lines: 14 us).  Two rows a thread (1: 4.4 us, 4: 4.9).
+// nothing, where a row a thread over CSR reads each of a warp's value slots from
+// seven cache lines.  At 96^3 in the solve's list of serialised launches 11.5 us
+// (CSR 14); alone, back to back 4.1, with two rows a thread (1: 4.4, 4: 4.9).
 constexpr int kMxSpmvRows = 2;
 
 template <int W>
@@ -1558,6 +1561,7 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_step(int n, size_t ld,
     const int n4 = n >> 2;
     float4* w4 = reinterpret_cast<float4*>(w);
     const uint64_t pol = l2_evict_first();
+    float4 sq = make_float4(0.f, 0.f, 0.f, 0.f);  // a sum a value of a load, as k_mx_mdot
     for (int i = n4 - 1 - (int)((blockIdx.x - 1) * kMixBlock + threadIdx.x); i >= 0;
          i -= nb * kMixBlock) {
       float4 v = w4[i];
@@ -1571,21 +1575,25 @@ __global__ void __launch_bounds__(kMixBlock) k_mx_maxpy_step(int n, size_t ld,
           if (j + q < k) fma4(v, -hs[j + q], t[q]);
       }
       w4[i] = v;
-      acc = __fmaf_rn(v.x, v.x, acc);
-      acc = __fmaf_rn(v.y, v.y, acc);
-      acc = __fmaf_rn(v.z, v.z, acc);
-      acc = __fmaf_rn(v.w, v.w, acc);
+      sq.x = __fmaf_rn(v.x, v.x, sq.x);
+      sq.y = __fmaf_rn(v.y, v.y, sq.y);
+      sq.z = __fmaf_rn(v.z, v.z, sq.z);
+      sq.w = __fmaf_rn(v.w, v.w, sq.w);
     }
+    acc = (sq.x + sq.y) + (sq.z + sq.w);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if (lane == 0) sh[wid] = acc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int ww = 0; ww < kMixBlock / 32; ww++) t += sh[ww];
-    partials[blockIdx.x] = t;
-    last = atomic_add_acq_rel(ticket, 1u) == gridDim.x - 1;
+  if (wid == 0) {
+    float t = lane < kMixBlock / 32 ? sh[lane] : 0.f;
+#pragma unroll
+    for (int o = kMixBlock / 64; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) {
+      partials[blockIdx.x] = t;
+      last = atomic_add_acq_rel(ticket, 1u) == gridDim.x - 1;
+    }
   }
   __syncthreads();
   if (!last) return;
@@ -1674,10 +1682,14 @@ __global__ void k_mx_correct(int n, const float* __restrict__ Z, const MixDev* s
 
 // Dots of w against V's rows 8 blockIdx.y .. + 7 (of k), gated on `*gate == 1`:
 // FP32 per thread and per CTA, the CTAs' sums in FP64 by the last CTA of each
-// eight.  16-byte loads, the eight rows of V in flight together; a CTA of 128
-// threads takes one such load a thread up to 96^3 (k = 16 in 6.1 us there, with
-// CTAs of 256 7.5, with the eights in turn inside a CTA 7.2; four rows a thread
-// with 4-byte loads and the eights in turn took 28 for 12).
+// eight.  16-byte loads, the eight rows of V in flight together; up to three CTAs of
+// 128 threads an SM, one such load a thread to 61^3 and four at 96^3.  The four
+// values of a load have a sum each, so that no FP32 sum is longer than with a row a
+// thread on 155,648 threads (4 terms a thread at 96^3, joined in pairs; one sum for
+// all four had 15).  Alone, back to back at 96^3 with 16 rows: 6.1 us (CTAs of 256
+// threads 7.5, the eights in turn inside a CTA 7.2; four rows a thread with 4-byte
+// loads and the eights in turn took 28 for 12).  In the solve, where the L2 holds
+// less of V: 6.2 us + 0.64 a row (serialised launches).
 constexpr int kMdotBlock = 128;
 
 static dim3 mx_mdot_grid(int64_t n, int k) {
@@ -1700,9 +1712,9 @@ __global__ void __launch_bounds__(kMdotBlock) k_mx_mdot(const int* gate, int n, 
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int j0 = blockIdx.y * 8, kk = min(8, k - j0), n4 = n >> 2;
   V += j0 * ld;
-  float acc[8];
+  float4 sum[8];
 #pragma unroll
-  for (int q = 0; q < 8; q++) acc[q] = 0.f;
+  for (int q = 0; q < 8; q++) sum[q] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int i = blockIdx.x * kMdotBlock + threadIdx.x; i < n4; i += gridDim.x * kMdotBlock) {
     float4 t[8];
     const float4 ww = reinterpret_cast<const float4*>(w)[i];
@@ -1712,12 +1724,15 @@ __global__ void __launch_bounds__(kMdotBlock) k_mx_mdot(const int* gate, int n, 
 #pragma unroll
     for (int q = 0; q < 8; q++)
       if (q < kk) {
-        acc[q] = __fmaf_rn(t[q].x, ww.x, acc[q]);
-        acc[q] = __fmaf_rn(t[q].y, ww.y, acc[q]);
-        acc[q] = __fmaf_rn(t[q].z, ww.z, acc[q]);
-        acc[q] = __fmaf_rn(t[q].w, ww.w, acc[q]);
+        sum[q].x = __fmaf_rn(t[q].x, ww.x, sum[q].x);
+        sum[q].y = __fmaf_rn(t[q].y, ww.y, sum[q].y);
+        sum[q].z = __fmaf_rn(t[q].z, ww.z, sum[q].z);
+        sum[q].w = __fmaf_rn(t[q].w, ww.w, sum[q].w);
       }
   }
+  float acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) acc[q] = (sum[q].x + sum[q].y) + (sum[q].z + sum[q].w);
   if (blockIdx.x == 0 && (int)threadIdx.x < (n & 3)) {
     const int i = (n4 << 2) + threadIdx.x;
 #pragma unroll
