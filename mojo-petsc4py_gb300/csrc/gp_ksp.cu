@@ -2440,7 +2440,9 @@ int ksp_solve(Ksp* k, Csr* A, Pc* pc, const double* b, double* x, KspResult* res
   const int n = A->n;
   k->n = n;
   bool moved = false;
-  GP_TRY(ensure(k, n, &moved));
+  const int fit = ensure(k, n, &moved);
+  if (moved || fit != GP_OK) drop_graph(k);  // it holds the old buffers, now or after a failure
+  GP_TRY(fit);
   cudaStream_t s = k->stream;
   cudaEvent_t ev;
   GP_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

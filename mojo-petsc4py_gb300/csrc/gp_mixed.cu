@@ -503,12 +503,24 @@ static int up_mixed(V** d, const std::vector<V>& h) {
   return GP_OK;
 }
 
+// Device arrays that the captured pass reads are about to be freed: whatever fails
+// after that, the pass is not launched again, nor are half-built arrays taken for
+// whole ones (callers clear the mark of what they rebuild first).
+static void drop_pass(Mixed* M) {
+  if (M->exec) cudaGraphExecDestroy(M->exec);
+  if (M->graph) cudaGraphDestroy(M->graph);
+  M->exec = nullptr;
+  M->graph = nullptr;
+}
+
 // (Re)build the FP32 factor triangles from the PC's factor.
 static int mixed_factors(Mixed* M, cudaStream_t s) {
   const Pc* pc = M->pc;
   const FactorPattern& P = pc->pat;
   const int n = M->n;
   if (M->pc_generation != pc->generation) {
+    drop_pass(M);
+    M->pc_generation = 0;
     for (void** p : {(void**)&M->lrp, (void**)&M->lci, (void**)&M->lslot, (void**)&M->urp,
                      (void**)&M->uci, (void**)&M->uslot, (void**)&M->dslot, (void**)&M->lval,
                      (void**)&M->uval, (void**)&M->udinv, (void**)&M->lell_ci,
@@ -698,9 +710,11 @@ __global__ void k_dia_fill(int n, const int* __restrict__ rp, const int* __restr
 static int mixed_operator(Mixed* M, const Csr* A, cudaStream_t s) {
   const int n = A->n, gr = (n + 255) / 256;
   if (M->adia_uid != A->uid) {
-    if (M->adia) GP_CUDA(cudaFree(M->adia));
-    M->adia = nullptr;
+    drop_pass(M);
+    M->adia_uid = 0;
     M->aW = 0;
+    if (M->adia) cudaFree(M->adia);
+    M->adia = nullptr;
     if (!M->a_scan) GP_CUDA(cudaMalloc(&M->a_scan, 12 * sizeof(int)));
     int h[10] = {1};
     if (A->n == A->ncols && A->nnz) {
@@ -847,6 +861,8 @@ static int mixed_blocks(Mixed* M, int want, cudaStream_t s) {
   const int n = M->n;
   const int rows = bt_rows_for(P, n, want);
   if (M->bt_rows != rows || M->bt_generation != pc->generation || !M->bl.cstart) {
+    drop_pass(M);
+    M->bt_generation = 0;
     std::vector<int> lrp(n + 1, 0), lci, lsl, urp(n + 1, 0), uci, usl, dsl(n);
     for (int i = 0; i < n; i++) {
       lrp[i + 1] = lrp[i] + P.bi[i + 1] - P.bi[i];
@@ -910,6 +926,8 @@ static BtArgs bt_args(const BlockTri& b, int n) {
 
 static int mixed_buffers(Mixed* M, int n, int m) {
   if (M->n == n && M->m == m && M->V) return GP_OK;
+  drop_pass(M);
+  M->n = M->m = 0;
   for (void** p : {(void**)&M->V, (void**)&M->Z, (void**)&M->w, (void**)&M->t0, (void**)&M->t1,
                    (void**)&M->t2, (void**)&M->t3, (void**)&M->t4, (void**)&M->r, (void**)&M->y,
                    (void**)&M->h_dev, (void**)&M->partials, (void**)&M->ticket})
@@ -2031,10 +2049,7 @@ int mixed_solve_graph(Mixed* M, Csr* A, Pc* pc, const double* b, double* x,
                     std::equal(ikey, ikey + 5, M->cap_ikey) && M->cap_A_uid == A->uid &&
                     M->cap_pc_gen == pc->generation;
   if (!same) {
-    if (M->exec) cudaGraphExecDestroy(M->exec);
-    if (M->graph) cudaGraphDestroy(M->graph);
-    M->exec = nullptr;
-    M->graph = nullptr;
+    drop_pass(M);
     GP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
     int st = record_pass(M, A, pc, b, x, o.tri_sweeps, bt, s);
     cudaGraph_t gph = nullptr;

@@ -46,3 +46,25 @@ def test_no_launch_status_is_dropped():
         for call in re.finditer(r"(.{0,24})\blaunch_pdl\(", code, re.S):
             before = call.group(1).rstrip()
             assert before.endswith(("GP_CUDA(", "=", "cudaError_t")), (path.name, before)
+
+
+def _before(code, start, end):
+    code = code[code.index(start):]
+    return code[:code.index(end)]
+
+
+def test_captured_graphs_are_dropped_before_their_buffers():
+    """A workspace or layout that a captured graph reads is rebuilt only after the
+    graph is dropped and the mark of the old one cleared, so that an allocation that
+    fails half-way leaves neither a graph of freed memory nor a half-built one taken
+    for whole."""
+    code = _code("gp_mixed.cu")
+    for start, mark in (("static int mixed_buffers(", "M->n = M->m = 0;"),
+                        ("static int mixed_factors(", "M->pc_generation = 0;"),
+                        ("static int mixed_operator(", "M->adia_uid = 0;"),
+                        ("static int mixed_blocks(", "M->bt_generation = 0;")):
+        head = _before(code, start, "bt_build(" if "blocks" in start else "cudaFree(")
+        assert "drop_pass(M);" in head and mark in head, start
+    head = _before(_code("gp_ksp.cu"), "int ksp_solve(", "cudaGraphLaunch(")
+    assert re.search(r"fit = ensure\(k, n, &moved\);\s*if \(moved \|\| fit != GP_OK\) drop_graph\(k\);",
+                     head)
